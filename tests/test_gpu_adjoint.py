@@ -250,3 +250,24 @@ def test_window_rejects_rescaling_step_and_mixed(case):
         g.forward_window(5, PATCH[0], PATCH[1], 2)
     with pytest.raises(TblError):  # no window recorded
         g.backward_window(1.0)
+
+
+def test_first_window_of_a_handle_equals_the_next():
+    """A handle's first window allocates its tape; a 1 GB tape takes long
+    enough to clear for an unordered clear to wipe what the window writes."""
+    from turbulentbl_gb300.synth import small_workload, make_state
+    from turbulentbl_gb300.lib import TblGpu
+
+    wl = small_workload(nx=96, nz_span=48, ny_wall=48, kmax=30)
+    mesh, rp, st = make_state(wl, nproc=4)
+    rp.cum = 10 ** 6
+    g = TblGpu(mesh, rp)
+    got = []
+    for _ in range(2):
+        g.upload(st)
+        J, _ = g.forward_window(3, 2.0, 10.0, 1)
+        gc, _, _ = g.backward_window(1.0)
+        got.append((J, gc))
+    g.close()
+    assert got[0][0] == got[1][0]
+    assert np.array_equal(got[0][1], got[1][1])

@@ -834,7 +834,8 @@ int tape_alloc(tbl_handle* h, int W, int ck) {
     n += (size_t)g.nx * (g.ny - 2) + (size_t)g.nx * g.ny + 2 * pl + 4 * (size_t)g.nx + 8;
     n += 2 * (size_t)g.nx + 8;  // fin_diag
     TBL_CUDA_TRY(cudaMalloc((void**)&T->buf, n * sizeof(double)));
-    TBL_CUDA_TRY(cudaMemset(T->buf, 0, n * sizeof(double)));
+    // on the handle's stream: the legacy stream's memset is not ordered before the copies into the tape that follow
+    TBL_CUDA_TRY(cudaMemsetAsync(T->buf, 0, n * sizeof(double), h->stream));
     T->buf_n = n;
     T->W = W; T->ck = ck; T->nseg = nseg; T->vol = vol;
     double* p = T->buf;
@@ -948,7 +949,7 @@ int tbl_forward_window(tbl_handle* h, int32_t nsteps, const tbl_window_config* w
     if (bm == TBL_BRANCH_REPLAY && !T->bits_valid) return TBL_ERR_BAD_ARG;  // no record of this window
     if (bm != TBL_BRANCH_FREE && !T->bits) {
         TBL_CUDA_TRY(cudaMalloc((void**)&T->bits, (size_t)nsteps * vol));
-        TBL_CUDA_TRY(cudaMemset(T->bits, 0, (size_t)nsteps * vol));
+        TBL_CUDA_TRY(cudaMemsetAsync(T->bits, 0, (size_t)nsteps * vol, h->stream));
     }
     if (bm == TBL_BRANCH_RECORD) T->bits_valid = false;
     T->branch_mode = bm;

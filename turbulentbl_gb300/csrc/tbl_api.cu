@@ -289,6 +289,8 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
     TBL_CUDA_TRY(cudaMemcpy(h->sc, &s0, sizeof(s0), cudaMemcpyHostToDevice));
     TRY(build_sweep_ctas(h));
     TRY(check_cooperative(h));
+    // the zero fills and copies above ran on the legacy stream, which the handle's stream does not wait for
+    TBL_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     h->nstep = 0; h->cont = 0; h->nstat = 0; h->cnt2 = 0; h->time = 0.0;
     h->fluc_updated = false;
     h->replay_pos = 0;
