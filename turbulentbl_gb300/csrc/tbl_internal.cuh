@@ -75,6 +75,23 @@ struct RedWork {
 
 struct AdjTape;  // tbl_adjoint.cu
 
+// Points per lane and step of the wavefront sweeps (tbl_sweep.cu), the unit
+// of the streamwise SSOR blocks: 4 in FP64, 8 in FP32.
+constexpr int sweep_chunk(size_t value_bytes) { return value_bytes == 4 ? 8 : 4; }
+
+// How the line-scan sweeps (tbl_line.cu) split a grid; S = 0 where they do
+// not take it and the wavefront sweeps run.
+struct LineCta {
+    int slab, blk, kg;  // slab, span block, plane group
+};
+struct LineShape {
+    int S = 0, KP = 0, NC = 0;  // warps per line, planes per CTA, courier warps
+    int nblk = 0, rows = 0;     // span blocks per slab, rows per block
+    int ncta = 0;               // CTAs of a launch (one component)
+    size_t smem = 0;
+    LineCta* ctas = nullptr;    // [ncta]
+};
+
 template <typename T>
 struct Fields {
     T* U[3];
@@ -104,6 +121,11 @@ struct tbl_handle {
     float* gs_coef_f;   // 5 x nz: the update coefficients rounded to FP32 (+ the red-black U(k-1) one)
     double* lap_scale;  // nz: -w/Ap(k), the SSOR forward scaling folded into the matvec
     float* coef_f;      // 4 x nz FP32: Ab, At, Ap, -w/Ap (FP32 matvec)
+    double* ssor_scale;   // nz: the matvec's scale before an SSOR application: lap_scale, times the backward
+    float* ssor_scale_f;  // sweep's constant w (2-w)/w where the line-scan sweeps run (FP64 and FP32)
+    tbl::LineShape line[3];  // line-scan sweeps per mode (GS, forward, backward)
+    void* line_xch;          // their exchange between the CTAs of a column, empty words all ones
+    unsigned* line_ticket;   // their tickets [taken, finished]
     double* V;       // kmax+1 Krylov vectors, vol each
     double* uold1;   // U1 at i=1 before the inflow update, (ny, nz)
     // mixed precision (TBL_PREC_MIXED): FP32 fields and inner-GMRES vectors

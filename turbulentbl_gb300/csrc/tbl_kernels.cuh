@@ -33,6 +33,13 @@ int launch_ssor_fwd_f(tbl_handle* h, const float* Xf, const double* PCd, const d
 int launch_ssor_bwd_f(tbl_handle* h, float* out, const int* skip = nullptr);
 int selftest_bounded_wait(int* observed, double* seconds);
 
+// tbl_line.cu: line-scan sweeps, where h->line[mode].S > 0
+int line_create(tbl_handle* h);
+template <typename V>
+int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], V* halo_out, const int* comps, int ncomp);
+template <typename V>
+int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* skip);
+
 // tbl_lap.cu: R = scale(k) L7 X by TMA plane tiles (the Arnoldi matvec)
 template <typename T>
 int launch_lap_tma(tbl_handle* h, const T* X, T* R, T aw, T as, const T* Ab, const T* At, const T* Ap, const T* scale,

@@ -20,15 +20,17 @@
 //     mailbox in shared memory, one slot per row, whose value is its own flag
 //     (slots start as a NaN pattern that no result has), and is added after
 //     the scan, so that the chain between the warps of a line is one FMA;
-//   * the plane below is handed over row by row with st.async into a ring in
-//     the consumer's shared memory (its own CTA or the next CTA of the
-//     cluster), ordered by the ring slots' mbarriers;
-//   * slabs of more planes than a cluster holds continue in the next cluster
-//     through a global exchange buffer whose words are their own flags.
+//   * the plane below comes row by row: from another warp of the CTA straight
+//     into a ring in shared memory, from another CTA through a global exchange
+//     buffer whose words are their own flags too, which a courier warp polls
+//     and copies into the ring (the loads of a poll in flight would otherwise
+//     stall the sweeping warps); the row's operands are fetched into the same
+//     ring slot by a bulk copy, and one mbarrier per slot covers both.
 //
-// All waits are bounded; a wait that gives up sets the error word, and every
-// warp stays until the cluster's closing barrier, so no CTA leaves while
-// another may still reach its shared memory.
+// CTAs take their planes by ticket, the lowest planes of all slabs first, so
+// that a CTA only ever waits for CTAs that have started: the launch needs no
+// co-residency.  All waits are bounded; a wait that gives up sets the error
+// word and the warps that depend on it give up in turn.
 #include <algorithm>
 
 #include "tbl_internal.cuh"
@@ -37,21 +39,23 @@
 
 namespace tbl {
 
-constexpr int LINE_XR = 4;            // ring slots (rows) per warp
-constexpr int LINE_MAX_WARPS = 16;    // warps of a CTA at most
-constexpr int LINE_MAX_SLOTS = 8192;  // carry mailbox slots of a CTA at most (64 KB in FP64)
-constexpr int LINE_MAX_SMEM = 160 * 1024;  // above the largest CTA: 64 KB of rings, 64 KB of mailboxes, barriers
+constexpr int LINE_XR = 8;           // ring slots (rows) per warp, in two halves that are handed back whole
+constexpr int LINE_MAX_WARPS = 12;   // sweeping warps of a CTA at most
+constexpr int LINE_MAX_COURIERS = 4;
+constexpr int LINE_MAX_SMEM = 200 * 1024;
+constexpr int LINE_BARS = LINE_XR + 2;  // mbarriers per warp: a slot is full, a half is empty
 
 template <typename V>
 struct LineArgs {
     Geom g;
     const SlabDesc* slabs;
+    const LineCta* ctas;     // CTAs of one component, lowest planes first
+    unsigned* ticket;        // [taken, finished]
     int* err;
     const int* skip;
-    int S, KP;         // warps per line, planes per CTA
-    int nc, ngrp;      // CTAs per cluster, clusters per slab column
-    int nblk, rows;    // span blocks per slab, rows of a block (the last may have fewer)
-    int cb;            // SSOR streamwise blocks: chunks per block (0 = one block)
+    int S, KP, NC, nsets;  // warps per line, planes per CTA, couriers, components
+    int rows;              // rows of a span block (the last may have fewer)
+    int cb;                // SSOR streamwise blocks: chunks per block (0 = one block)
     const double *Ab, *At, *rAp;
     double aw, as, omega;
     const V* gsc;      // GS: [p0|p1|p2|p3] x nz of the handle's coefficient table
@@ -61,40 +65,83 @@ struct LineArgs {
     int comp[3];
     V* halo_out;       // GS: [comp][side][slab] planes of the next sweep's halo
     int P;
-    V* xch;            // [set][slab][block][cluster boundary][row][32 E S]
+    V* xch;            // [set][plane][span row][32 E S], empty words all ones
 };
 
 template <typename V> struct LineBits;
 template <> struct LineBits<double> {
-    using U = unsigned long long;
-    static __device__ __forceinline__ U of(double v) { return (U)__double_as_longlong(v); }
-    static __device__ __forceinline__ double from(U b) { return __longlong_as_double((long long)b); }
+    static __device__ __forceinline__ unsigned hi(double v) { return (unsigned)__double2hiint(v); }
+    static __device__ __forceinline__ double nan() { return __hiloint2double(0x7fffffff, -1); }
+    static __device__ __forceinline__ double empty() { return __hiloint2double(-1, -1); }
     static constexpr double tiny = 8.7e-19;  // 2^-60
 };
 template <> struct LineBits<float> {
-    using U = unsigned;
-    static __device__ __forceinline__ U of(float v) { return __float_as_uint(v); }
-    static __device__ __forceinline__ float from(U b) { return __uint_as_float(b); }
+    static __device__ __forceinline__ unsigned hi(float v) { return __float_as_uint(v); }
+    static __device__ __forceinline__ float nan() { return __uint_as_float(0x7fffffffu); }
+    static __device__ __forceinline__ float empty() { return __uint_as_float(0xffffffffu); }
     static constexpr float tiny = 2.3e-10f;  // 2^-32
 };
-// "not written yet": all bits set, a NaN that a result is never stored as
+// "Not written yet" is a NaN with its high word all ones; results with that
+// high word are stored as another NaN.
 template <typename V>
-__device__ __forceinline__ V line_flagged(V v) {
-    using B = LineBits<V>;
-    return B::of(v) == ~(typename B::U)0 ? B::from((~(typename B::U)0) >> 1) : v;
+__device__ __forceinline__ bool line_empty(V v) { return LineBits<V>::hi(v) == 0xffffffffu; }
+template <typename V>
+__device__ __forceinline__ V line_value(V v) { return line_empty(v) ? LineBits<V>::nan() : v; }
+
+// 16 bytes of the exchange buffer: each value is read and written whole.
+__device__ __forceinline__ void xch_ld(double* v, const double* p) {
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void xch_ld(float* v, const float* p) {
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void xch_st(double* p, const double* v) {
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v[0]), "d"(v[1]) : "memory");
+}
+__device__ __forceinline__ void xch_st(float* p, const float* v) {
+    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3])
+                 : "memory");
+}
+template <int E, typename V>
+__device__ __forceinline__ bool xch_row(V (&w)[E], const V* p) {
+    constexpr int W = 16 / sizeof(V);
+#pragma unroll
+    for (int b = 0; b < E / W; ++b) xch_ld(w + b * W, p + b * W);
+    bool have = true;
+#pragma unroll
+    for (int e = 0; e < E; ++e) have = have && !line_empty(w[e]);
+    return __all_sync(0xffffffffu, have);
+}
+template <int E, typename V>
+__device__ __forceinline__ void xch_put(V* p, const V (&w)[E]) {
+    constexpr int W = 16 / sizeof(V);
+#pragma unroll
+    for (int b = 0; b < E / W; ++b) xch_st(p + b * W, w + b * W);
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 
+// E values of shared memory, in sweep order.
 template <typename V, int E>
-__device__ __forceinline__ void line_load(V (&v)[E], const V* p, bool rev) {
+__device__ __forceinline__ void line_read(V (&v)[E], const V* p, bool rev) {
     constexpr int W = 16 / sizeof(V);
     V t[E];
 #pragma unroll
-    for (int b = 0; b < E / W; ++b) {
-        const int4 q = __ldcg(reinterpret_cast<const int4*>(p) + b);
-        *reinterpret_cast<int4*>(&t[b * W]) = q;
-    }
+    for (int b = 0; b < E / W; ++b)
+        *reinterpret_cast<int4*>(&t[b * W]) = *(reinterpret_cast<const int4*>(p) + b);
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = rev ? t[E - 1 - e] : t[e];
+}
+// `bytes` of global memory into this CTA's shared memory, counted by a barrier.
+__device__ __forceinline__ void line_fetch(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 template <typename V, int E>
 __device__ __forceinline__ void line_store(V* p, const V (&v)[E], bool rev) {
@@ -107,71 +154,111 @@ __device__ __forceinline__ void line_store(V* p, const V (&v)[E], bool rev) {
         *(reinterpret_cast<int4*>(p) + b) = *reinterpret_cast<const int4*>(&t[b * W]);
 }
 
-template <int MODE, typename V, int E, int D>
-__global__ void __launch_bounds__(32 * LINE_MAX_WARPS) k_line(const LineArgs<V> a) {
+template <int MODE, typename V, int E>
+__global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) k_line(const LineArgs<V> a) {
     if (a.skip && *a.skip) return;  // every CTA reads the same word, written by an earlier launch
     using B = LineBits<V>;
     constexpr bool GS = MODE == 0, BWD = MODE == 2;
-    constexpr unsigned XBYTES = 32 * E * sizeof(V);
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int XR = LINE_XR, H = XR / 2;
+    constexpr unsigned LBYTES = 32 * E * sizeof(V);  // a warp's segment of a row
     const Geom& g = a.g;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int S = a.S, KP = a.KP, NW = S * KP;
-    const int seg = wid % S, kp = wid / S;
-    const int set = blockIdx.y;
-    // grid.x: [slab][span block][cluster of the column][CTA of the cluster]
-    const int rank = blockIdx.x % a.nc, grp = (blockIdx.x / a.nc) % a.ngrp;
-    const int blk = (blockIdx.x / (a.nc * a.ngrp)) % a.nblk, slab = blockIdx.x / (a.nc * a.ngrp * a.nblk);
-    const SlabDesc sl = a.slabs[slab];
+
+    // shared memory: rings of the warps, a slot holding a row's operands and the
+    // row of the plane below | their barriers | carry mailboxes [warp][row]
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ unsigned s_ticket;
+    V* const rings = reinterpret_cast<V*>(s_dyn);
+    unsigned long long* const bars = reinterpret_cast<unsigned long long*>(s_dyn + (size_t)NW * XR * 2 * LBYTES);
+    V* const mail = reinterpret_cast<V*>(bars + NW * LINE_BARS);
+    if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
+    for (int q = threadIdx.x; q < NW * a.rows; q += blockDim.x) mail[q] = B::empty();
+    __syncthreads();
+    const int set = (int)(s_ticket % (unsigned)a.nsets);
+    const LineCta cta = a.ctas[s_ticket / (unsigned)a.nsets];
+    const SlabDesc sl = a.slabs[cta.slab];
     const int J = g.ny - 2, K = sl.K;
     const int comp = GS ? a.comp[set] : 0;
-    const int j0 = blk * a.rows, nrow = min(a.rows, J - j0);  // logical rows [j0, j0 + nrow)
-    const int kl = (grp * a.nc + rank) * KP + kp;             // logical plane
-    const bool live = kl < K;
+    const int j0 = cta.blk * a.rows, nrow = min(a.rows, J - j0);  // logical rows [j0, j0 + nrow)
+    const int jfirst = BWD ? J - 1 - j0 : j0;                     // logical row 0
+    const int seg = wid % S, kp = wid / S;
+    const int kl = cta.kg * KP + kp;  // logical plane
+    const bool sweeps = wid < NW && kl < K;
     const int kidx = BWD ? K - 1 - kl : kl;
-    const int k = sl.bn + (live ? kidx : 0);
-
-    // shared memory: rings of the warps | ring barriers (full, empty) | carry mailboxes
-    extern __shared__ __align__(16) unsigned char s_dyn[];
-    V* const ring = reinterpret_cast<V*>(s_dyn) + (size_t)wid * LINE_XR * 32 * E;
-    unsigned long long* const bars = reinterpret_cast<unsigned long long*>(s_dyn + (size_t)NW * LINE_XR * XBYTES);
-    unsigned long long* const full = bars + wid * 2 * LINE_XR;
-    unsigned long long* const empty = full + LINE_XR;
-    V* const mail = reinterpret_cast<V*>(bars + NW * 2 * LINE_XR);  // [warp][row]
-    for (int q = threadIdx.x; q < NW * a.rows; q += blockDim.x)
-        reinterpret_cast<typename B::U*>(mail)[q] = ~(typename B::U)0;
-    if (lane == 0) {
-        for (int q = 0; q < LINE_XR; ++q) {
-            mbar_init(&full[q], 1);
-            mbar_init(&empty[q], 1);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int q = 0; q < LINE_XR; ++q) mbar_arrive_expect_tx(&full[q], XBYTES);
-    }
+    const int k = sl.bn + (sweeps ? kidx : 0);
+    const bool below = kl > 0;  // a plane of the slab comes before this one
+    unsigned long long* const full = bars + (sweeps ? wid : 0) * LINE_BARS;
+    unsigned long long* const empty = full + XR;
+    if (sweeps && lane < LINE_BARS) mbar_init(&full[lane], lane < XR && below ? 2 : 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
-    cluster_sync_all();  // barriers initialised and armed in every CTA of the cluster
 
-    if (live) {
-        const bool first = kl == 0;
-        const bool last_of_grp = rank == a.nc - 1 && kp == KP - 1;
-        const bool from_ring = !first && !(rank == 0 && kp == 0);
-        const bool from_xch = !first && !from_ring;
+    const size_t xrow = (size_t)32 * E * S;
+    // exchange rows of physical plane kk, this lane's values of segment 0
+    auto xch_plane = [&](int kk) {
+        return a.xch + ((((size_t)set * g.nz + kk) * J + j0) * S * 32 + lane) * E;
+    };
+    if (wid >= NW) {
+        // Courier: the top plane of the CTA below, row by row, into the rings
+        // of this CTA's first plane; its words are emptied for the next launch.
+        if (cta.kg > 0 && cta.kg * KP < K) {
+            const int kb = BWD ? K - cta.kg * KP : cta.kg * KP - 1;
+            V* src = xch_plane(sl.bn + kb);
+            V none[E];
+#pragma unroll
+            for (int e = 0; e < E; ++e) none[e] = B::empty();
+            bool good = true;
+            for (int r = 0; r < nrow && good; ++r, src += xrow)
+                for (int sg = wid - NW; sg < S; sg += a.NC) {
+                    V w[E];
+                    long long spins = 0;
+                    while (!xch_row<E>(w, src + (size_t)sg * 32 * E))
+                        if (++spins > SPIN_LIMIT / 16) { good = false; break; }
+                    if (!good) break;
+                    xch_put<E>(src + (size_t)sg * 32 * E, none);
+                    const int u = r % XR;
+                    unsigned long long* fb = bars + sg * LINE_BARS;
+                    if (u % H == 0 && r >= XR &&
+                        !__all_sync(ALL, mbar_wait(&fb[XR + u / H], (unsigned)(r / XR - 1) & 1u))) {
+                        good = false;
+                        break;
+                    }
+                    V* dst = rings + (((size_t)sg * XR + u) * 64 + 32 + lane) * E;
+#pragma unroll
+                    for (int b = 0; b < E * (int)sizeof(V) / 16; ++b)
+                        reinterpret_cast<int4*>(dst)[b] = reinterpret_cast<const int4*>(w)[b];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&fb[u]);
+                }
+            if (!good && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
+        }
+    } else if (sweeps) {
+        V* const ring = rings + (size_t)wid * XR * 64 * E;
         const bool has_up = kl + 1 < K;
-        const bool to_ring = has_up && !last_of_grp, to_xch = has_up && last_of_grp;
-        const unsigned up_rank = kp < KP - 1 ? rank : rank + 1, dn_rank = kp > 0 ? rank : rank - 1;
-        const int up_wid = kp < KP - 1 ? wid + S : seg, dn_wid = kp > 0 ? wid - S : (KP - 1) * S + seg;
-        // shared-memory addresses in the neighbours' CTAs (the layout is the same in all)
-        V* const up_ring = reinterpret_cast<V*>(s_dyn) + (size_t)up_wid * LINE_XR * 32 * E;
-        const unsigned up_data = mapa_rank(smem_u32(up_ring + lane * E), to_ring ? up_rank : rank);
-        const unsigned up_full = mapa_rank(smem_u32(bars + up_wid * 2 * LINE_XR), to_ring ? up_rank : rank);
-        const unsigned dn_empty =
-            mapa_rank(smem_u32(bars + dn_wid * 2 * LINE_XR + LINE_XR), from_ring ? dn_rank : rank);
-        const size_t xrow = (size_t)32 * E * S;
-        const size_t xbase = (((size_t)set * a.P + slab) * a.nblk + blk) * (a.ngrp > 1 ? a.ngrp - 1 : 0);
-        V* const xin = from_xch ? a.xch + (xbase + grp - 1) * a.rows * xrow + (size_t)(seg * 32 + lane) * E : nullptr;
-        V* const xout = to_xch ? a.xch + (xbase + grp) * a.rows * xrow + (size_t)(seg * 32 + lane) * E : nullptr;
+        const bool to_ring = has_up && kp < KP - 1, to_xch = has_up && kp == KP - 1;
+        V* const up_ring = ring + (size_t)S * XR * 64 * E + (32 + lane) * E;
+        unsigned long long* const up_full = full + S * LINE_BARS;
+        V* xout = to_xch ? xch_plane(k) + (size_t)seg * 32 * E : nullptr;
+
+        // the row's segment in global memory: chunks [c0, ..) of the line, at
+        // chunk c0 - clo of the slot
+        const int C = (g.nx - 2) / E + 1;
+        const int clo = BWD ? C - 32 * (seg + 1) : 32 * seg, c0 = max(clo, 0);
+        const unsigned lbytes =
+            min((unsigned)(g.sx - E * c0), 32u * E - (unsigned)(E * (c0 - clo))) * (unsigned)sizeof(V);
+        const long long rstep = BWD ? -(long long)g.sx : (long long)g.sx;
+        const V* fsrc = a.in[comp] + (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * k) + E * c0;
+        const unsigned fdst = smem_u32(ring) + (unsigned)(c0 - clo) * E * (unsigned)sizeof(V), fbar = smem_u32(full);
+        if (lane == 0)
+            for (int q = 0; q < XR && q < nrow; ++q) {
+                mbar_arrive_expect_tx(&full[q], lbytes);
+                line_fetch(fdst + q * 2 * LBYTES, fsrc + q * rstep, lbytes, fbar + 8u * q);
+            }
+        fsrc += XR * rstep;
 
         // this lane's points: chunk ch of the line in sweep order, i = i0 .. i0 + E - 1
-        const int C = (g.nx - 2) / E + 1;
         const int ch = seg * 32 + lane;
         const bool on = ch < C;
         const int pc = BWD ? C - 1 - ch : ch;
@@ -184,7 +271,7 @@ __global__ void __launch_bounds__(32 * LINE_MAX_WARPS) k_line(const LineArgs<V> 
             ok[e] = on && i >= 1 && i <= g.nx - 2;
             all_ok = all_ok && ok[e];
         }
-        const bool edge = __any_sync(0xffffffffu, !all_ok);  // the warp holds a line end
+        const bool edge = __any_sync(ALL, !all_ok);  // the warp holds a line end
         // chunks before this one in its streamwise block
         int dist = ch;
         if (!GS && a.cb > 0) dist = BWD ? min(C, (pc / a.cb + 1) * a.cb) - 1 - pc : pc % a.cb;
@@ -220,100 +307,92 @@ __global__ void __launch_bounds__(32 * LINE_MAX_WARPS) k_line(const LineArgs<V> 
         const bool starts = dist == 0;
 
         // line pointers; logical row r of the block
-        const int jfirst = BWD ? J - 1 - j0 : j0;
-        const long long rstep = BWD ? -(long long)g.sx : (long long)g.sx;
-        const long long base = (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * k) + i0;
-        const V* inp = a.in[comp] + base;
-        V* outp = a.out[comp] + base;
+        V* outp = a.out[comp] + (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * k) + i0;
         V* hout = nullptr;
         if (GS) {
             const size_t hb = (size_t)comp * 2 * a.P;
             const long long hl = (long long)g.sx * (1 + jfirst) + i0;
-            if (kidx == 0 && slab > 0) hout = a.halo_out + (hb + a.P + (slab - 1)) * (size_t)g.ps + hl;
-            if (kidx == K - 1 && slab < a.P - 1) hout = a.halo_out + (hb + (slab + 1)) * (size_t)g.ps + hl;
+            if (kidx == 0 && cta.slab > 0) hout = a.halo_out + (hb + a.P + (cta.slab - 1)) * (size_t)g.ps + hl;
+            if (kidx == K - 1 && cta.slab < a.P - 1) hout = a.halo_out + (hb + (cta.slab + 1)) * (size_t)g.ps + hl;
         }
-        V* const my_mail = mail + (size_t)wid * a.rows;
-        const V* const prev_mail = mail + (size_t)(wid - 1) * a.rows;
+        volatile V* const my_mail = mail + (size_t)wid * a.rows;
+        const volatile V* const prev_mail = mail + (size_t)(seg > 0 ? wid - 1 : wid) * a.rows;
 
-        V pf[D][E], xj[E], x0[GS ? E : 1];
-#pragma unroll
-        for (int u = 0; u < D; ++u) {
-#pragma unroll
-            for (int e = 0; e < E; ++e) pf[u][e] = V(0);
-            if (on && u < nrow) line_load<V, E>(pf[u], inp + u * rstep, BWD);
-        }
+        V gr[E], xj[E], x0[GS ? E : 1];
 #pragma unroll
         for (int e = 0; e < E; ++e) xj[e] = V(0);
-        bool dead = false;
 
-        auto row = [&](const int r, V(&in)[E]) {
-            V f[E];
+        // Row q's right-hand side with the plane below's share (ring slot s,
+        // phase ph): ask() looks without waiting, get() waits.  An ask that came
+        // too early has read a stale slot, and get() follows.  Lanes beyond the
+        // line read what is there: no point of the line depends on them.
+        const V* const slot0 = ring + (BWD ? 31 - lane : lane) * E;
+        const V* const below0 = ring + (32 + lane) * E;
+        auto take = [&](int s, V(&o)[E]) {
+            line_read<V, E>(o, slot0 + s * 64 * E, BWD);
+            if (below) {
+                V xk[E];
+                line_read<V, E>(xk, below0 + s * 64 * E, false);
 #pragma unroll
-            for (int e = 0; e < E; ++e) f[e] = fma(cj, xj[e], in[e]);
-            if (on && r + D < nrow) line_load<V, E>(in, inp + (r + D) * rstep, BWD);
+                for (int e = 0; e < E; ++e) o[e] = fma(ck, xk[e], o[e]);
+            }
+        };
+        auto ask = [&](int s, unsigned ph, V(&o)[E]) -> bool {
+            const bool rdy = __all_sync(ALL, mbar_test(&full[s], ph));
+            take(rdy ? s : (s ^ 1), o);  // the address waits for the test
+            return rdy;
+        };
+        auto get = [&](int s, unsigned ph, V(&o)[E]) -> bool {
+            if (!__all_sync(ALL, mbar_wait(&full[s], ph))) return false;
+            take(s, o);
+            return true;
+        };
+        // Row q has been read: its slot is armed for row q + XR, whose operands
+        // are fetched, and handed back to the plane below by halves.
+        auto done = [&](int q, int s) {
+            __syncwarp();
+            if (lane == 0 && q + XR < nrow) {
+                mbar_arrive_expect_tx(&full[s], lbytes);
+                line_fetch(fdst + s * 2 * LBYTES, fsrc, lbytes, fbar + 8u * s);
+            }
+            if (below && lane == 0 && s % H == H - 1 && q + H + 1 < nrow) mbar_arrive(&empty[s / H]);
+            fsrc += rstep;
+        };
+
+        // One row: gr holds its right-hand side and the plane below's share.
+        // What the next row needs from the plane below is looked at while this
+        // row's scan runs, and waited for only after this row has been handed on.
+        auto row = [&](const int r, const int u, const unsigned ph) -> bool {
+            V x[E];
+#pragma unroll
+            for (int e = 0; e < E; ++e) x[e] = fma(cj, xj[e], gr[e]);
             if (GS && r == nrow - 1) {  // periodic: the last row reads the first row's new values
 #pragma unroll
-                for (int e = 0; e < E; ++e) f[e] = fma(cj, x0[GS ? e : 0], f[e]);
+                for (int e = 0; e < E; ++e) x[e] = fma(cj, x0[GS ? e : 0], x[e]);
             }
-            // ---- the plane below
-            if (from_ring) {
-                const int s = r % LINE_XR;
-                if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (unsigned)(r / LINE_XR) & 1u))) { dead = true; return; }
-                V xk[E];
-                const V* src = ring + (s * 32 + lane) * E;
+            V c = seg > 0 ? prev_mail[r] : V(0);
+            // the line: local chain, scan over the lanes
 #pragma unroll
-                for (int e = 0; e < E; ++e) xk[e] = src[e];
-                __syncwarp();
-                if (lane == 0 && r + LINE_XR < nrow) {  // hand the slot back when it is written again
-                    mbar_arrive_expect_tx(&full[s], XBYTES);
-                    mbar_arrive_remote(dn_empty + 8u * s);
-                }
-#pragma unroll
-                for (int e = 0; e < E; ++e) f[e] = fma(ck, xk[e], f[e]);
-            } else if (from_xch) {
-                V xk[E];
-                long long spins = 0;
-                bool have;
-                do {
-                    const volatile typename B::U* src = reinterpret_cast<const volatile typename B::U*>(xin + r * xrow);
-                    have = true;
-#pragma unroll
-                    for (int e = 0; e < E; ++e) {
-                        const typename B::U v = src[e];
-                        have = have && v != ~(typename B::U)0;
-                        xk[e] = B::from(v);
-                    }
-                    if (++spins > SPIN_LIMIT) break;
-                } while (!__all_sync(0xffffffffu, have));
-                if (!__all_sync(0xffffffffu, have)) { dead = true; return; }
-                typename B::U* dst = reinterpret_cast<typename B::U*>(xin + r * xrow);
-#pragma unroll
-                for (int e = 0; e < E; ++e) dst[e] = ~(typename B::U)0;  // empty again for the next launch
-#pragma unroll
-                for (int e = 0; e < E; ++e) f[e] = fma(ck, xk[e], f[e]);
-            }
-            // ---- the line: local chain, scan over the lanes, carry of the segment before
-            V x[E];
-            x[0] = f[0];
-#pragma unroll
-            for (int e = 1; e < E; ++e) x[e] = fma(ci, x[e - 1], f[e]);
+            for (int e = 1; e < E; ++e) x[e] = fma(ci, x[e - 1], x[e]);
             V b = x[E - 1];
 #pragma unroll
             for (int l = 0; l < 5; ++l)
-                if (l < nlev) b = fma(lev[l], __shfl_up_sync(0xffffffffu, b, 1 << l), b);
-            V c = V(0);
+                if (l < nlev) b = fma(lev[l], __shfl_up_sync(ALL, b, 1 << l), b);
+            const int s1 = (u + 1) % XR;
+            const unsigned ph1 = u + 1 == XR ? ph ^ 1u : ph;
+            const bool more = r + 1 < nrow;
+            const bool rdy = !more || ask(s1, ph1, gr);
+            // the carry of the segment before
             if (seg > 0) {
-                const volatile typename B::U* m = reinterpret_cast<const volatile typename B::U*>(prev_mail + r);
-                typename B::U v;
                 long long spins = 0;
-                while ((v = *m) == ~(typename B::U)0)
-                    if (++spins > SPIN_LIMIT) break;
-                if (__any_sync(0xffffffffu, v == ~(typename B::U)0)) { dead = true; return; }
-                c = B::from(v);
+                while (__any_sync(ALL, line_empty(c))) {
+                    if (++spins > SPIN_LIMIT) return false;
+                    c = prev_mail[r];
+                }
                 b = fma(acar, c, b);
             }
-            if (seg < S - 1 && lane == 31) *const_cast<volatile V*>(my_mail + r) = line_flagged(b);
-            V y = __shfl_up_sync(0xffffffffu, b, 1);
+            if (seg < S - 1 && lane == 31) my_mail[r] = line_value(b);
+            V y = __shfl_up_sync(ALL, b, 1);
             if (lane == 0) y = c;
             if (starts) y = V(0);
 #pragma unroll
@@ -323,139 +402,132 @@ __global__ void __launch_bounds__(32 * LINE_MAX_WARPS) k_line(const LineArgs<V> 
 #pragma unroll
                 for (int e = 0; e < E; ++e) x[e] = ok[e] ? x[e] : V(0);
             }
-            // ---- hand the row to the plane above, then to global memory
+            // hand the row to the plane above, then to global memory
             if (to_ring) {
-                const int s = r % LINE_XR;
-                if (r >= LINE_XR &&
-                    !__all_sync(0xffffffffu, mbar_wait(&empty[s], (unsigned)(r / LINE_XR - 1) & 1u))) {
-                    dead = true;
-                    return;
-                }
-                xpush<E>(up_data + (unsigned)(s * XBYTES), up_full + 8u * s, x);
+                if (u % H == 0 && r >= XR &&
+                    !__all_sync(ALL, mbar_wait(&up_full[XR + u / H], ph ^ 1u)))
+                    return false;
+                line_store<V, E>(up_ring + u * 64 * E, x, false);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&up_full[u]);
             } else if (to_xch) {
-                volatile V* dst = xout + r * xrow;
+                V w[E];
 #pragma unroll
-                for (int e = 0; e < E; ++e) dst[e] = line_flagged(x[e]);
+                for (int e = 0; e < E; ++e) w[e] = line_value(x[e]);
+                xch_put<E>(xout, w);
+                xout += xrow;
             }
             if (on) {
                 if (!GS || !edge) {
-                    line_store<V, E>(outp + r * rstep, x, BWD);
-                    if (GS && hout) line_store<V, E>(hout + r * rstep, x, BWD);
+                    line_store<V, E>(outp, x, BWD);
+                    if (GS && hout) line_store<V, E>(hout, x, BWD);
                 } else {  // the faces i = 0 and nx-1 keep their boundary values
 #pragma unroll
                     for (int e = 0; e < E; ++e)
                         if (ok[e]) {
-                            outp[r * rstep + e] = x[e];
-                            if (hout) hout[r * rstep + e] = x[e];
+                            outp[e] = x[e];
+                            if (hout) hout[e] = x[e];
                         }
                 }
             }
+            outp += rstep;
+            if (GS && hout) hout += rstep;
 #pragma unroll
             for (int e = 0; e < E; ++e) xj[e] = x[e];
             if (GS && r == 0) {
 #pragma unroll
                 for (int e = 0; e < E; ++e) x0[GS ? e : 0] = x[e];
             }
+            if (!rdy && !get(s1, ph1, gr)) return false;
+            if (more) done(r + 1, s1);
+            return true;
         };
-        for (int r0 = 0; r0 < nrow && !dead; r0 += D) {
+        bool good = get(0, 0u, gr);
+        if (good) done(0, 0);
+        unsigned ph = 0;
+        for (int r0 = 0; r0 < nrow && good; r0 += XR, ph ^= 1u) {
 #pragma unroll
-            for (int u = 0; u < D; ++u)
-                if (r0 + u < nrow && !dead) row(r0 + u, pf[u]);
+            for (int u = 0; u < XR; ++u)
+                if (good && r0 + u < nrow) good = row(r0 + u, u, ph);
         }
-        if (dead && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
+        // (a warp that gave up has waited for a second: its own fetches have landed)
+        if (!good && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
         __syncwarp();
     }
-    cluster_sync_all();  // pushes into a CTA's shared memory have landed or will not come
+    __syncthreads();  // the last CTA to finish leaves the tickets as it found them
+    if (threadIdx.x == 0 && atomicAdd(a.ticket + 1, 1u) + 1 == gridDim.x) {
+        a.ticket[0] = 0u;
+        a.ticket[1] = 0u;
+    }
 }
 
 // ------------------------------------------------------------------ host
-template <typename V> constexpr int line_e() { return 4; }
-template <typename V> constexpr int line_d() { return sizeof(V) == 8 ? 4 : 8; }
+constexpr int LINE_E = 4;  // points per lane
 
 template <int MODE, typename V>
-static const void* line_fn() { return (const void*)k_line<MODE, V, line_e<V>(), line_d<V>()>; }
+static const void* line_fn() { return (const void*)k_line<MODE, V, LINE_E>; }
 
-static size_t line_smem(int S, int KP, int rows, size_t vsize, int E) {
+static size_t line_smem(int S, int KP, int rows, size_t vsize) {
     const size_t nw = (size_t)S * KP;
-    return nw * LINE_XR * 32 * E * vsize + nw * 2 * LINE_XR * 8 + nw * rows * vsize;
+    return nw * (LINE_XR * 64 * LINE_E * vsize + LINE_BARS * 8 + rows * vsize);
 }
 
-static void line_cfg(const tbl_handle* h, const LineShape& q, int nsets, cudaLaunchConfig_t& cfg,
-                     cudaLaunchAttribute* at) {
-    cfg = {};
-    cfg.gridDim = dim3((unsigned)(h->P * q.nblk * q.ngrp * q.nc), (unsigned)nsets);
-    cfg.blockDim = dim3((unsigned)(32 * q.S * q.KP));
-    cfg.dynamicSmemBytes = q.smem;
-    cfg.stream = h->stream;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)q.nc;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-}
-
-// Splits a slab column of Kmax planes over CTAs and clusters for one kernel.
-// False when the line sweeps do not take this grid.
-static bool line_plan(const tbl_handle* h, const void* fn, size_t vsize, int E, int rows, int nblk, int want_kp,
-                      LineShape& q) {
-    const int C = (h->g.nx - 2) / E + 1;
-    int kmax = 1;
-    for (int r = 0; r < h->P; ++r) kmax = std::max(kmax, h->en[r] - h->bn[r] + 1);
+// Splits the slab columns over CTAs of KP planes for one kernel.  False when
+// the line sweeps do not take the grid: lines of more than LINE_MAX_WARPS
+// warps, or rows that the mailboxes have no room for.
+static bool line_plan(const tbl_handle* h, const void* fn, size_t vsize, int rows, int nblk, int kp, LineShape& q) {
+    const int C = (h->g.nx - 2) / LINE_E + 1;
     q = LineShape();
     q.S = (C + 31) / 32;
+    if (q.S > LINE_MAX_WARPS) return false;
+    q.KP = std::min(kp, LINE_MAX_WARPS / q.S);
+    q.NC = std::min(q.S, LINE_MAX_COURIERS);
     q.rows = rows;
     q.nblk = nblk;
-    if (q.S > LINE_MAX_WARPS || (long long)q.S * rows > LINE_MAX_SLOTS) return false;
-    const int kp_max = std::max(1, LINE_MAX_WARPS / q.S);
-    for (q.KP = std::min(want_kp, kp_max); q.KP <= kp_max; ++q.KP)
-        for (int most = 16; most >= 8; most -= 8) {  // 16 CTAs where the device takes such clusters
-            if ((long long)q.S * q.KP * rows > LINE_MAX_SLOTS) return false;
-            const int ctas = (kmax + q.KP - 1) / q.KP;
-            q.ngrp = (ctas + most - 1) / most;
-            q.nc = (ctas + q.ngrp - 1) / q.ngrp;
-            q.smem = line_smem(q.S, q.KP, rows, vsize, E);
-            cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute at[1];
-            line_cfg(h, q, 1, cfg, at);
-            int ncl = 0;
-            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, LINE_MAX_SMEM) != cudaSuccess ||
-                cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-                cudaOccupancyMaxActiveClusters(&ncl, fn, &cfg) != cudaSuccess) {
-                (void)cudaGetLastError();
-                continue;
-            }
-            // the clusters of a column wait on one another: all of a launch's clusters must be resident
-            q.sets = ncl < 1 ? 0 : q.ngrp == 1 ? 3 : std::min(3, ncl / (h->P * nblk * q.ngrp));
-            if (q.sets >= 1) return true;
-        }
-    return false;
+    q.smem = line_smem(q.S, q.KP, rows, vsize);
+    if (q.smem > LINE_MAX_SMEM) return false;
+    for (int r = 0; r < h->P; ++r) q.ncta += (h->en[r] - h->bn[r] + 1 + q.KP - 1) / q.KP * nblk;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, LINE_MAX_SMEM) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
+// The CTAs of a launch, the lowest of every column first.
+static int line_table(const tbl_handle* h, LineShape& q) {
+    std::vector<LineCta> t;
+    for (int kg = 0; (int)t.size() < q.ncta; ++kg)
+        for (int r = 0; r < h->P; ++r)
+            if (kg * q.KP < h->en[r] - h->bn[r] + 1)
+                for (int blk = 0; blk < q.nblk; ++blk) t.push_back({r, blk, kg});
+    TBL_CUDA_TRY(cudaMalloc(&q.ctas, t.size() * sizeof(LineCta)));
+    TBL_CUDA_TRY(cudaMemcpy(q.ctas, t.data(), t.size() * sizeof(LineCta), cudaMemcpyHostToDevice));
+    return TBL_OK;
 }
 
 template <typename V>
 static int line_init(tbl_handle* h) {
     const int J = h->g.ny - 2;
-    const int kp = sizeof(V) == 8 ? 1 : 1;
+    const int kp = sizeof(V) == 8 ? 1 : 2;
     const bool span = (h->cfg.flags & TBL_FLAG_SSOR_SPAN_BLOCKS) != 0;
     const int brows = span ? std::min(32, J) : J, nblk = span ? (J + 31) / 32 : 1;
-    h->line[0].S = h->line[1].S = h->line[2].S = 0;
     LineShape q[3];
-    if (line_plan(h, line_fn<0, V>(), sizeof(V), line_e<V>(), J, 1, kp, q[0])) h->line[0] = q[0];
-    if (line_plan(h, line_fn<1, V>(), sizeof(V), line_e<V>(), brows, nblk, kp, q[1]) &&
-        line_plan(h, line_fn<2, V>(), sizeof(V), line_e<V>(), brows, nblk, kp, q[2])) {
-        h->line[1] = q[1];
-        h->line[2] = q[2];
-    }
-    size_t words = 0;
+    const bool gs = line_plan(h, line_fn<0, V>(), sizeof(V), J, 1, kp, q[0]);
+    const bool ssor = line_plan(h, line_fn<1, V>(), sizeof(V), brows, nblk, kp, q[1]) &&
+                      line_plan(h, line_fn<2, V>(), sizeof(V), brows, nblk, kp, q[2]);
     for (int m = 0; m < 3; ++m) {
-        const LineShape& s = h->line[m];
-        if (s.S > 0)
-            words = std::max(words, (size_t)(m == 0 ? std::min(3, s.sets) : 1) * h->P * s.nblk * (s.ngrp - 1) * s.rows *
-                                        32 * line_e<V>() * s.S);
+        if (m == 0 ? !gs : !ssor) continue;
+        h->line[m] = q[m];
+        const int st = line_table(h, h->line[m]);
+        if (st != TBL_OK) return st;
     }
-    if (words > 0) {
+    if (gs || ssor) {
+        const size_t words = (size_t)(gs ? 3 : 1) * h->g.nz * J * 32 * LINE_E * q[gs ? 0 : 1].S;
         TBL_CUDA_TRY(cudaMalloc(&h->line_xch, words * sizeof(V)));
         TBL_CUDA_TRY(cudaMemset(h->line_xch, 0xff, words * sizeof(V)));
+        TBL_CUDA_TRY(cudaMalloc(&h->line_ticket, 2 * sizeof(unsigned)));
+        TBL_CUDA_TRY(cudaMemset(h->line_ticket, 0, 2 * sizeof(unsigned)));
     }
     return TBL_OK;
 }
@@ -469,8 +541,10 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
     LineArgs<V> a = {};
     a.g = h->g;
     a.slabs = h->slabs;
+    a.ctas = q.ctas;
+    a.ticket = h->line_ticket;
     a.err = h->err;
-    a.S = q.S; a.KP = q.KP; a.nc = q.nc; a.ngrp = q.ngrp; a.nblk = q.nblk; a.rows = q.rows;
+    a.S = q.S; a.KP = q.KP; a.NC = q.NC; a.rows = q.rows;
     a.P = h->P;
     a.Ab = h->Ab; a.At = h->At; a.rAp = h->rAp;
     a.aw = 1.0 / (h->cfg.dx * h->cfg.dx);
@@ -482,10 +556,9 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
 
 template <int MODE, typename V>
 static int line_launch(tbl_handle* h, const LineShape& q, LineArgs<V>& a, int nsets) {
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at[1];
-    line_cfg(h, q, nsets, cfg, at);
-    TBL_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_line<MODE, V, line_e<V>(), line_d<V>()>, a));
+    a.nsets = nsets;
+    k_line<MODE, V, LINE_E><<<q.ncta * nsets, 32 * (q.S * q.KP + q.NC), q.smem, h->stream>>>(a);
+    TBL_CUDA_TRY(cudaGetLastError());
     h->launches++;
     return TBL_OK;
 }
@@ -499,13 +572,8 @@ int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], V* halo_out, c
     a.gsb = a.gsc + (sizeof(V) == 8 ? 7 : 4) * nz;
     a.halo_out = halo_out;
     for (int c = 0; c < 3; ++c) { a.out[c] = F[c]; a.in[c] = PRE[c]; }
-    for (int c0 = 0; c0 < ncomp; c0 += q.sets) {
-        const int n = std::min(ncomp - c0, q.sets);
-        for (int c = 0; c < n; ++c) a.comp[c] = comps[c0 + c];
-        const int s = line_launch<0, V>(h, q, a, n);
-        if (s != TBL_OK) return s;
-    }
-    return TBL_OK;
+    for (int c = 0; c < ncomp; ++c) a.comp[c] = comps[c];
+    return line_launch<0, V>(h, q, a, ncomp);
 }
 
 template <typename V>
@@ -518,7 +586,7 @@ int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* sk
     // streamwise blocks of the same points as the wavefront sweep's
     if (h->ssor_nib > 1) {
         const int ch = sweep_chunk(sizeof(V)), C = (h->g.nx - 2) / ch + 1;
-        a.cb = (C + h->ssor_nib - 1) / h->ssor_nib * (ch / line_e<V>());
+        a.cb = (C + h->ssor_nib - 1) / h->ssor_nib * (ch / LINE_E);
     }
     return bwd ? line_launch<2, V>(h, q, a, 1) : line_launch<1, V>(h, q, a, 1);
 }

@@ -34,6 +34,7 @@
 
 #include "tbl_internal.cuh"
 #include "tbl_kernels.cuh"
+#include "tbl_sync.cuh"
 
 namespace tbl {
 
@@ -72,17 +73,6 @@ struct SweepArgs {
                                 // column form one cluster along k), 0 = global flags
 };
 
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-constexpr long long SPIN_LIMIT = 1LL << 24;  // ~1 s of polling, then the wait gives up
-
 // Poll a global progress flag until it reports step >= target (returns the
 // step seen, or -2 on timeout).  Flags hold (epoch << 20) + step + 1.
 __device__ __forceinline__ long long wait_global(const unsigned long long* f, unsigned long long tag, long long target) {
@@ -117,7 +107,7 @@ constexpr int XR_SLOTS = 8;  // slots of the ring a CTA receives its plane-below
 // sweeps were slower).  Each lane's operand buffer holds 4 CH positions:
 // position q of the line at element q % (4 CH); chunks are copied two steps
 // ahead, so the live positions span 3 CH - 1 < 4 CH.
-template <typename Val> constexpr int sweep_ch() { return sizeof(Val) == 4 ? 8 : 4; }
+template <typename Val> constexpr int sweep_ch() { return sweep_chunk(sizeof(Val)); }
 // Dynamic shared memory of a sweep CTA: the plane-to-plane ring and the operand buffers.
 template <typename Val> constexpr size_t sweep_smem() {
     return sizeof(Val) * KG * (RING * 32 * sweep_ch<Val>() + 32 * 4 * sweep_ch<Val>()) +
@@ -154,86 +144,6 @@ constexpr int PUB = 4;   // global progress is published every PUB steps (and at
 // memory after a timeout: the producer reports its end (1) or abort (2) to
 // the consumer, and after an abort waits for the consumer's acknowledgement.
 constexpr int XR = XR_SLOTS;
-constexpr long long XLINGER = 1LL << 27;  // bounded wait for the partner at the end
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned mapa_rank(unsigned addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* b, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_remote(unsigned raddr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(raddr) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(b)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait for the completion of the phase of the given parity.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
-    long long spins = 0;
-    while (!mbar_try_wait(b, parity)) {
-        if (++spins > SPIN_LIMIT) return false;
-    }
-    return true;
-}
-// One lane's CH values of a step into the consumer's ring slot.
-template <int CH>
-__device__ __forceinline__ void xpush(unsigned rd, unsigned rb, const double (&v)[CH]) {
-#pragma unroll
-    for (int b = 0; b < CH / 2; ++b)
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
-                         rd + 16u * b),
-                     "d"(v[2 * b]), "d"(v[2 * b + 1]), "r"(rb)
-                     : "memory");
-}
-template <int CH>
-__device__ __forceinline__ void xpush(unsigned rd, unsigned rb, const float (&v)[CH]) {
-#pragma unroll
-    for (int b = 0; b < CH / 4; ++b)
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
-                         rd + 16u * b),
-                     "f"(v[4 * b]), "f"(v[4 * b + 1]), "f"(v[4 * b + 2]), "f"(v[4 * b + 3]), "r"(rb)
-                     : "memory");
-}
-__device__ __forceinline__ void st_remote_s32(unsigned raddr, int v) {
-    asm volatile("st.relaxed.cluster.shared::cluster.s32 [%0], %1;" ::"r"(raddr), "r"(v) : "memory");
-}
-__device__ __forceinline__ int ld_relaxed_cluster(const int* p) {
-    int v;
-    asm volatile("ld.relaxed.cluster.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
-    return v;
-}
-// Bounded wait until a word of this CTA (written by the partner CTA) is non-zero.
-__device__ __forceinline__ int wait_word(const int* p) {
-    for (long long spins = 0; spins < XLINGER; ++spins) {
-        const int v = ld_relaxed_cluster(p);
-        if (v) return v;
-        if (spins > 64) __nanosleep(64);
-    }
-    return 0;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 __device__ __forceinline__ int ld_acquire_cta(const int* p) {
     int v;
@@ -707,13 +617,17 @@ __global__ void k_gs_coef(int nz, double t, double aw_, double as_, const double
     pcf[4 * nz + k] = (float)pc[7 * nz + k];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_gs_pre(Geom g, const T* __restrict__ pc,
+// LINE: for the line-scan sweeps, which read nothing but these terms and
+// what they produce: also the old values of the row before the first one
+// (periodic) and of the plane below a slab, and the inflow boundary value
+// itself at i = 0.
+template <typename T, bool LINE>
+__global__ void __launch_bounds__(256) k_gs_pre(Geom g, const T* __restrict__ pc, const T* __restrict__ pbv,
                                                 const int* __restrict__ slab_of_k,
                                                 const SlabDesc* __restrict__ slabs, int P, int c0_, int c1_, int c2_,
                                                 Ptr3<T> Fs, Ptr3<T> Qs, Ptr3<T> PREs,
                                                 const T* __restrict__ halo_in) {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (LINE ? 0 : 1) + blockIdx.x * blockDim.x + threadIdx.x;
     const int K = g.nz - 2;
     const int ci = blockIdx.z / K, k = 1 + blockIdx.z % K;
     if (i > g.nx - 2) return;
@@ -721,19 +635,33 @@ __global__ void __launch_bounds__(256) k_gs_pre(Geom g, const T* __restrict__ pc
     const T* F = Fs.p[comp];
     const int nz = g.nz;
     const T p0 = pc[k], p1 = pc[nz + k], p2 = pc[2 * nz + k], p3 = pc[3 * nz + k];
+    const T pb = LINE ? pbv[k] : T(0);
     const int r = slab_of_k[k];
     const SlabDesc sl = slabs[r];
     const bool halo = k == sl.bn + sl.K - 1 && r < P - 1;
+    const bool below = LINE && k == sl.bn;
     for (int jr = 0; jr < ROWS_PER_BLOCK; ++jr) {  // a few rows per block: fewer, longer blocks
         const int j = 1 + blockIdx.y * ROWS_PER_BLOCK + jr;
         if (j > g.ny - 2) break;
         const long long line = (long long)g.sx * ((long long)j + (long long)g.ny * k);
+        T* out = const_cast<T*>(PREs.p[comp]) + line + i;
+        if (LINE && i == 0) {
+            *out = F[line];
+            continue;
+        }
         const int jp = (j == g.ny - 2) ? 1 : j + 1;
         const T* Fkp = halo ? halo_in + ((size_t)comp * 2 * P + 1 * P + r) * (size_t)g.ps + (size_t)g.sx * j
                             : F + line + g.ps;
         T x = fma(p1, F[line + i + 1], p0 * Qs.p[comp][line + i]);
         if (jp != 1) x = fma(p2, F[(long long)g.sx * ((long long)jp + (long long)g.ny * k) + i], x);
-        const_cast<T*>(PREs.p[comp])[line + i] = fma(p3, Fkp[i], x);
+        x = fma(p3, Fkp[i], x);
+        if (LINE && j == 1) x = fma(p2, F[(long long)g.sx * ((long long)(g.ny - 2) + (long long)g.ny * k) + i], x);
+        if (below) {
+            const T* Fkm = r > 0 ? halo_in + ((size_t)comp * 2 * P + r) * (size_t)g.ps + (size_t)g.sx * j
+                                 : F + line - g.ps;
+            x = fma(pb, Fkm[i], x);
+        }
+        *out = x;
     }
 }
 
@@ -1004,12 +932,16 @@ static int gs_pre_and_sweep(tbl_handle* h, T* const F[3], const T* const Q[3], T
     const Geom& g = h->g;
     Ptr3<T> Fs, Qs, Ps;
     for (int c = 0; c < 3; ++c) { Fs.p[c] = F[c]; Qs.p[c] = Q[c]; Ps.p[c] = PRE[c]; }
-    dim3 grid((g.nx - 2 + 255) / 256, (g.ny - 2 + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, (g.nz - 2) * ncomp);
     const T* pc = sizeof(T) == 8 ? (const T*)h->gs_coef : (const T*)h->gs_coef_f;
-    k_gs_pre<T><<<grid, 256, 0, h->stream>>>(g, pc, h->slab_of_k, h->slabs, h->P,
-                                             comps[0], ncomp > 1 ? comps[1] : 0, ncomp > 2 ? comps[2] : 0, Fs, Qs,
-                                             Ps, a.halo_in);
+    const T* pb = pc + (sizeof(T) == 8 ? 7 : 4) * (size_t)g.nz;
+    const bool line = h->line[SW_GS].S > 0;
+    dim3 grid((g.nx - 2 + (line ? 1 : 0) + 255) / 256, (g.ny - 2 + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK,
+              (g.nz - 2) * ncomp);
+    (line ? k_gs_pre<T, true> : k_gs_pre<T, false>)<<<grid, 256, 0, h->stream>>>(
+        g, pc, pb, h->slab_of_k, h->slabs, h->P, comps[0], ncomp > 1 ? comps[1] : 0, ncomp > 2 ? comps[2] : 0, Fs, Qs,
+        Ps, a.halo_in);
     h->launches++;
+    if (line) return launch_line_gs<T>(h, F, PRE, a.halo_out, comps, ncomp);
     return launch_sweep<SW_GS, T>(h, a, ncomp);
 }
 
@@ -1044,7 +976,7 @@ int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity) {
         const double* Q[3] = {h->Q[0], h->Q[1], h->Q[2]};
         return rb_gs<double>(h, F, Q, h->gs_coef, h->gs_coef + 7 * (size_t)nz, comps, ncomp);
     }
-    const int per = h->gs_comps_per_launch > 0 ? h->gs_comps_per_launch : 1;
+    const int per = h->line[SW_GS].S > 0 ? 3 : h->gs_comps_per_launch > 0 ? h->gs_comps_per_launch : 1;
     for (int c0 = 0; c0 < ncomp; c0 += per) {
         const int n = ncomp - c0 < per ? ncomp - c0 : per;
         const int s = launch_gs_sweep_chunk(h, comps + c0, n, parity);
@@ -1071,9 +1003,10 @@ int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int*
     const Geom& g = h->g;
     const double aw = 1.0 / (h->cfg.dx * h->cfg.dx), as = 1.0 / (h->cfg.dy * h->cfg.dy);
     k_lap<double, double, double><<<dim3((g.nx - 2 + 255) / 256, g.ny - 2, g.nz - 2), 256, 0, h->stream>>>(
-        g, aw, as, h->Ab, h->At, h->Ap, X, Q8, h->RH, h->lap_scale, skip);
+        g, aw, as, h->Ab, h->At, h->Ap, X, Q8, h->RH, h->ssor_scale, skip);
     h->launches++;
     if (h->cfg.flags & TBL_FLAG_RB_PRECOND) return TBL_OK;  // the red-black passes run in launch_ssor_bwd
+    if (h->line[SW_FWD].S > 0) return launch_line_ssor<double>(h, false, h->RH, h->RH, skip);
     SweepArgs<double> a = base_args<double>(h);
     a.RH = h->RH;
     a.skip = skip;
@@ -1096,6 +1029,7 @@ int launch_ssor_bwd(tbl_handle* h, double* out, const int* skip) {
     if (h->cfg.flags & TBL_FLAG_RB_PRECOND)
         return rb_ssor<double>(h, 1.0 / (h->cfg.dx * h->cfg.dx), 1.0 / (h->cfg.dy * h->cfg.dy), h->Ab, h->At,
                                h->lap_scale, h->RH, out);
+    if (h->line[SW_BWD].S > 0) return launch_line_ssor<double>(h, true, h->RH, out, skip);
     SweepArgs<double> a = base_args<double>(h);
     a.RH = h->RH;
     a.OUT = out;
@@ -1114,16 +1048,17 @@ int launch_ssor_fwd_f(tbl_handle* h, const float* Xf, const double* PCd, const d
     const double aw = 1.0 / (h->cfg.dx * h->cfg.dx), as = 1.0 / (h->cfg.dy * h->cfg.dy);
     if (PCd)
         k_lap<double, float, double><<<grid, 256, 0, h->stream>>>(g, aw, as, h->Ab, h->At, h->Ap, PCd, Q8, h->RHf,
-                                                                  h->coef_f + 3 * (size_t)g.nz, skip);
+                                                                  h->ssor_scale_f, skip);
     else {  // the inner Arnoldi matvec: TMA plane tiles
         const int s = launch_lap_tma<float>(h, Xf, h->RHf, (float)aw, (float)as, h->coef_f, h->coef_f + g.nz,
-                                            h->coef_f + 2 * (size_t)g.nz, h->coef_f + 3 * (size_t)g.nz, skip, denom,
+                                            h->coef_f + 2 * (size_t)g.nz, h->ssor_scale_f, skip, denom,
                                             vout);
         if (s != TBL_OK) return s;
         h->launches--;  // counted by launch_lap_tma
     }
     h->launches++;
     if (h->cfg.flags & TBL_FLAG_RB_PRECOND) return TBL_OK;
+    if (h->line[SW_FWD].S > 0) return launch_line_ssor<float>(h, false, h->RHf, h->RHf, skip);
     SweepArgs<float> a = base_args<float>(h);
     a.RH = h->RHf;
     a.skip = skip;
@@ -1136,6 +1071,7 @@ int launch_ssor_bwd_f(tbl_handle* h, float* out, const int* skip) {
         return rb_ssor<float>(h, (float)(1.0 / (h->cfg.dx * h->cfg.dx)), (float)(1.0 / (h->cfg.dy * h->cfg.dy)),
                               h->coef_f, h->coef_f + nz, h->coef_f + 3 * nz, h->RHf, out);
     }
+    if (h->line[SW_BWD].S > 0) return launch_line_ssor<float>(h, true, h->RHf, out, skip);
     SweepArgs<float> a = base_args<float>(h);
     a.RH = h->RHf;
     a.OUT = out;

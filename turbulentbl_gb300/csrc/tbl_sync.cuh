@@ -50,6 +50,18 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, unsigned pa
         : "memory");
     return ok != 0;
 }
+// Whether the phase of the given parity has completed (no waiting).
+__device__ __forceinline__ bool mbar_test(unsigned long long* b, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait for the completion of the phase of the given parity.
 __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
     long long spins = 0;
