@@ -85,7 +85,8 @@ struct LineCta {
     int slab, blk, kg;  // slab, span block, plane group
 };
 struct LineShape {
-    int S = 0, KP = 0, NC = 0;  // warps per line, planes per CTA, courier warps
+    int S = 0, E = 0;           // warps per line (0: not taken), points per lane
+    int KP = 0, NC = 0;         // planes per CTA, courier warps
     int nblk = 0, rows = 0;     // span blocks per slab, rows per block
     int ncta = 0;               // CTAs of a launch (one component)
     size_t smem = 0;
@@ -124,7 +125,8 @@ struct tbl_handle {
     double* ssor_scale;   // nz: the matvec's scale before an SSOR application: lap_scale, times the backward
     float* ssor_scale_f;  // sweep's constant w (2-w)/w where the line-scan sweeps run (FP64 and FP32)
     tbl::LineShape line[3];  // line-scan sweeps per mode (GS, forward, backward)
-    void* line_xch;          // their exchange between the CTAs of a column, empty words all ones
+    void* line_xch;          // their exchange between the CTAs of a column
+    size_t line_xdump;       // a row of it that nobody reads
     unsigned* line_ticket;   // their tickets [taken, finished]
     double* V;       // kmax+1 Krylov vectors, vol each
     double* uold1;   // U1 at i=1 before the inflow update, (ny, nz)

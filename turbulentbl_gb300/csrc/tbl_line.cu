@@ -24,13 +24,27 @@
 //     into a ring in shared memory, from another CTA through a global exchange
 //     buffer whose words are their own flags too, which a courier warp polls
 //     and copies into the ring (the loads of a poll in flight would otherwise
-//     stall the sweeping warps); the row's operands are fetched into the same
-//     ring slot by a bulk copy, and one mbarrier per slot covers both.
+//     stall the sweeping warps); the rows' operands are fetched by bulk copies,
+//     four rows at a time.
 //
 // CTAs take their planes by ticket, the lowest planes of all slabs first, so
 // that a CTA only ever waits for CTAs that have started: the launch needs no
 // co-residency.  All waits are bounded; a wait that gives up sets the error
 // word and the warps that depend on it give up in turn.
+//
+// What bounds it: the serial chain of J + K rows.  A row of an FP64 warp with 1
+// point per lane takes about 1100 cycles, of which 440 are the scan (114 a
+// level: an FP64 FMA of 64 and two shuffles) and 180 the FMAs before it; the
+// rest, and most of an FP32 row's 950, is the issue of about 190 instructions
+// from one warp per scheduler.  A hand-over to the next CTA takes about 1.2 us.
+// SSOR sweep, wavefront -> line scan: 130 -> 62 us (128 x 66 x 64, FP64, 8
+// slabs), 389 -> 185 us (512 x 130 x 128, FP64), 95 -> 47 us and 251 -> 100 us
+// (FP32); GS sweep of three components with its precomputed terms 620 -> 650 us
+// less the launches it saves at 512, 280 -> 90 us at 128 (FP64).
+// A first form with thread-block clusters (st.async into the next CTA's ring)
+// was slower at 512 (243 us): clusters of 15 CTAs doubled up on SMs.  Register
+// prefetch of the operands was slower too (their loads share scoreboards with
+// the shuffles: every row waited for them).
 #include <algorithm>
 
 #include "tbl_internal.cuh"
@@ -40,10 +54,13 @@
 namespace tbl {
 
 constexpr int LINE_XR = 8;           // ring slots (rows) per warp, in two halves that are handed back whole
-constexpr int LINE_MAX_WARPS = 12;   // sweeping warps of a CTA at most
+// sweeping warps of a CTA at most, so that the registers of E points per lane fit
+constexpr int line_max_warps(int E) { return E >= 4 ? 12 : 16; }
 constexpr int LINE_MAX_COURIERS = 4;
 constexpr int LINE_MAX_SMEM = 200 * 1024;
-constexpr int LINE_BARS = LINE_XR + 2;  // mbarriers per warp: a slot is full, a half is empty
+// mbarriers per warp: the plane below's row is in a slot; a half of the slots
+// has been read; a half's operands have landed
+constexpr int LINE_BARS = LINE_XR + 4;
 
 template <typename V>
 struct LineArgs {
@@ -88,54 +105,78 @@ __device__ __forceinline__ bool line_empty(V v) { return LineBits<V>::hi(v) == 0
 template <typename V>
 __device__ __forceinline__ V line_value(V v) { return line_empty(v) ? LineBits<V>::nan() : v; }
 
-// 16 bytes of the exchange buffer: each value is read and written whole.
-__device__ __forceinline__ void xch_ld(double* v, const double* p) {
+// E values of the exchange buffer; each value is read and written whole.
+__device__ __forceinline__ void xch_ld(double (&v)[1], const double* p) {
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v[0]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void xch_ld(double (&v)[2], const double* p) {
     asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p) : "memory");
 }
-__device__ __forceinline__ void xch_ld(float* v, const float* p) {
+__device__ __forceinline__ void xch_ld(double (&v)[4], const double* p) {
+    xch_ld(reinterpret_cast<double(&)[2]>(v[0]), p);
+    xch_ld(reinterpret_cast<double(&)[2]>(v[2]), p + 2);
+}
+__device__ __forceinline__ void xch_ld(float (&v)[2], const float* p) {
+    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void xch_ld(float (&v)[4], const float* p) {
     asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
                  : "l"(p)
                  : "memory");
 }
-__device__ __forceinline__ void xch_st(double* p, const double* v) {
+__device__ __forceinline__ void xch_put(double* p, const double (&v)[1]) {
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v[0]) : "memory");
+}
+__device__ __forceinline__ void xch_put(double* p, const double (&v)[2]) {
     asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v[0]), "d"(v[1]) : "memory");
 }
-__device__ __forceinline__ void xch_st(float* p, const float* v) {
+__device__ __forceinline__ void xch_put(double* p, const double (&v)[4]) {
+    xch_put(p, reinterpret_cast<const double(&)[2]>(v[0]));
+    xch_put(p + 2, reinterpret_cast<const double(&)[2]>(v[2]));
+}
+__device__ __forceinline__ void xch_put(float* p, const float (&v)[2]) {
+    asm volatile("st.relaxed.gpu.global.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v[0]), "f"(v[1]) : "memory");
+}
+__device__ __forceinline__ void xch_put(float* p, const float (&v)[4]) {
     asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
                  "f"(v[3])
                  : "memory");
 }
 template <int E, typename V>
 __device__ __forceinline__ bool xch_row(V (&w)[E], const V* p) {
-    constexpr int W = 16 / sizeof(V);
-#pragma unroll
-    for (int b = 0; b < E / W; ++b) xch_ld(w + b * W, p + b * W);
+    xch_ld(w, p);
     bool have = true;
 #pragma unroll
     for (int e = 0; e < E; ++e) have = have && !line_empty(w[e]);
     return __all_sync(0xffffffffu, have);
 }
-template <int E, typename V>
-__device__ __forceinline__ void xch_put(V* p, const V (&w)[E]) {
-    constexpr int W = 16 / sizeof(V);
-#pragma unroll
-    for (int b = 0; b < E / W; ++b) xch_st(p + b * W, w + b * W);
-}
 __device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 
-// E values of shared memory, in sweep order.
+// E values in memory order <-> in sweep order, by the widest accesses.
+template <int BYTES> struct LineWord { using T = int4; };
+template <> struct LineWord<8> { using T = int2; };
 template <typename V, int E>
 __device__ __forceinline__ void line_read(V (&v)[E], const V* p, bool rev) {
-    constexpr int W = 16 / sizeof(V);
+    using T = typename LineWord<E * sizeof(V)>::T;
+    constexpr int W = sizeof(T) / sizeof(V);
     V t[E];
 #pragma unroll
-    for (int b = 0; b < E / W; ++b)
-        *reinterpret_cast<int4*>(&t[b * W]) = *(reinterpret_cast<const int4*>(p) + b);
+    for (int b = 0; b < E / W; ++b) *reinterpret_cast<T*>(&t[b * W]) = *(reinterpret_cast<const T*>(p) + b);
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = rev ? t[E - 1 - e] : t[e];
+}
+template <typename V, int E>
+__device__ __forceinline__ void line_store(V* p, const V (&v)[E], bool rev) {
+    using T = typename LineWord<E * sizeof(V)>::T;
+    constexpr int W = sizeof(T) / sizeof(V);
+    V t[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) t[e] = rev ? v[E - 1 - e] : v[e];
+#pragma unroll
+    for (int b = 0; b < E / W; ++b) *(reinterpret_cast<T*>(p) + b) = *reinterpret_cast<const T*>(&t[b * W]);
 }
 // `bytes` of global memory into this CTA's shared memory, counted by a barrier.
 __device__ __forceinline__ void line_fetch(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
@@ -143,19 +184,16 @@ __device__ __forceinline__ void line_fetch(unsigned dst, const void* src, unsign
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+// Chunks of E points of a line, points 0 .. nx-2 at least, a whole number of
+// 16-byte words (a backward segment starts that many chunks from the end).
 template <typename V, int E>
-__device__ __forceinline__ void line_store(V* p, const V (&v)[E], bool rev) {
-    constexpr int W = 16 / sizeof(V);
-    V t[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) t[e] = rev ? v[E - 1 - e] : v[e];
-#pragma unroll
-    for (int b = 0; b < E / W; ++b)
-        *(reinterpret_cast<int4*>(p) + b) = *reinterpret_cast<const int4*>(&t[b * W]);
+__host__ __device__ constexpr int line_chunks(int nx) {
+    constexpr int M = E * sizeof(V) >= 16 ? 1 : 16 / (E * (int)sizeof(V));
+    return ((nx - 2) / E + 1 + M - 1) / M * M;
 }
 
 template <int MODE, typename V, int E>
-__global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) k_line(const LineArgs<V> a) {
+__global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 1) k_line(const LineArgs<V> a) {
     if (a.skip && *a.skip) return;  // every CTA reads the same word, written by an earlier launch
     using B = LineBits<V>;
     constexpr bool GS = MODE == 0, BWD = MODE == 2;
@@ -190,8 +228,8 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
     const int k = sl.bn + (sweeps ? kidx : 0);
     const bool below = kl > 0;  // a plane of the slab comes before this one
     unsigned long long* const full = bars + (sweeps ? wid : 0) * LINE_BARS;
-    unsigned long long* const empty = full + XR;
-    if (sweeps && lane < LINE_BARS) mbar_init(&full[lane], lane < XR && below ? 2 : 1);
+    unsigned long long *const empty = full + XR, *const opfull = full + XR + 2;
+    if (sweeps && lane < LINE_BARS) mbar_init(&full[lane], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
 
@@ -212,25 +250,19 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
             bool good = true;
             for (int r = 0; r < nrow && good; ++r, src += xrow)
                 for (int sg = wid - NW; sg < S; sg += a.NC) {
+                    V* const from = src + (size_t)sg * 32 * E;
+                    const int u = r & (XR - 1);
+                    unsigned long long* fb = bars + sg * LINE_BARS;
+                    if ((u & (H - 1)) == 0 && r >= XR)
+                        good = __all_sync(ALL, mbar_wait(&fb[XR + u / H], (unsigned)(r / XR - 1) & 1u));
                     V w[E];
                     long long spins = 0;
-                    while (!xch_row<E>(w, src + (size_t)sg * 32 * E))
-                        if (++spins > SPIN_LIMIT / 16) { good = false; break; }
+                    while (good && !xch_row<E>(w, from)) good = ++spins < SPIN_LIMIT / 16;
                     if (!good) break;
-                    xch_put<E>(src + (size_t)sg * 32 * E, none);
-                    const int u = r % XR;
-                    unsigned long long* fb = bars + sg * LINE_BARS;
-                    if (u % H == 0 && r >= XR &&
-                        !__all_sync(ALL, mbar_wait(&fb[XR + u / H], (unsigned)(r / XR - 1) & 1u))) {
-                        good = false;
-                        break;
-                    }
-                    V* dst = rings + (((size_t)sg * XR + u) * 64 + 32 + lane) * E;
-#pragma unroll
-                    for (int b = 0; b < E * (int)sizeof(V) / 16; ++b)
-                        reinterpret_cast<int4*>(dst)[b] = reinterpret_cast<const int4*>(w)[b];
+                    line_store<V, E>(rings + (((size_t)sg * XR + u) * 64 + 32 + lane) * E, w, false);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&fb[u]);
+                    xch_put(from, none);
                 }
             if (!good && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
         }
@@ -244,19 +276,25 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
 
         // the row's segment in global memory: chunks [c0, ..) of the line, at
         // chunk c0 - clo of the slot
-        const int C = (g.nx - 2) / E + 1;
+        const int C = line_chunks<V, E>(g.nx);
         const int clo = BWD ? C - 32 * (seg + 1) : 32 * seg, c0 = max(clo, 0);
         const unsigned lbytes =
             min((unsigned)(g.sx - E * c0), 32u * E - (unsigned)(E * (c0 - clo))) * (unsigned)sizeof(V);
         const long long rstep = BWD ? -(long long)g.sx : (long long)g.sx;
         const V* fsrc = a.in[comp] + (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * k) + E * c0;
-        const unsigned fdst = smem_u32(ring) + (unsigned)(c0 - clo) * E * (unsigned)sizeof(V), fbar = smem_u32(full);
-        if (lane == 0)
-            for (int q = 0; q < XR && q < nrow; ++q) {
-                mbar_arrive_expect_tx(&full[q], lbytes);
-                line_fetch(fdst + q * 2 * LBYTES, fsrc + q * rstep, lbytes, fbar + 8u * q);
-            }
-        fsrc += XR * rstep;
+        const unsigned fdst = smem_u32(ring) + (unsigned)(c0 - clo) * E * (unsigned)sizeof(V), fbar = smem_u32(opfull);
+        // lane 0: the operands of rows [q, q + H), the next that fsrc points to
+        auto fetch = [&](int q) {
+            const int hh = (q / H) & 1, n = min(H, nrow - q);
+            if (n <= 0) return;
+            mbar_arrive_expect_tx(&opfull[hh], lbytes * n);
+            for (int w = 0; w < n; ++w, fsrc += rstep)
+                line_fetch(fdst + (unsigned)(hh * H + w) * 2 * LBYTES, fsrc, lbytes, fbar + 8u * hh);
+        };
+        if (lane == 0) {
+            fetch(0);
+            fetch(H);
+        }
 
         // this lane's points: chunk ch of the line in sweep order, i = i0 .. i0 + E - 1
         const int ch = seg * 32 + lane;
@@ -322,10 +360,10 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
 #pragma unroll
         for (int e = 0; e < E; ++e) xj[e] = V(0);
 
-        // Row q's right-hand side with the plane below's share (ring slot s,
-        // phase ph): ask() looks without waiting, get() waits.  An ask that came
-        // too early has read a stale slot, and get() follows.  Lanes beyond the
-        // line read what is there: no point of the line depends on them.
+        // Row q's right-hand side with the plane below's share: ask() looks
+        // without waiting, get() waits.  An ask that came too early has read a
+        // stale slot, and get() follows.  Lanes beyond the line read what is
+        // there: no point of the line depends on them.
         const V* const slot0 = ring + (BWD ? 31 - lane : lane) * E;
         const V* const below0 = ring + (32 + lane) * E;
         auto take = [&](int s, V(&o)[E]) {
@@ -338,25 +376,29 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
             }
         };
         auto ask = [&](int s, unsigned ph, V(&o)[E]) -> bool {
-            const bool rdy = __all_sync(ALL, mbar_test(&full[s], ph));
+            bool rdy = true;
+            if (below) rdy = mbar_test(&full[s], ph);
+            if ((s & (H - 1)) == 0) rdy = mbar_test(&opfull[s / H], ph) && rdy;
+            rdy = __all_sync(ALL, rdy);
             take(rdy ? s : (s ^ 1), o);  // the address waits for the test
             return rdy;
         };
         auto get = [&](int s, unsigned ph, V(&o)[E]) -> bool {
-            if (!__all_sync(ALL, mbar_wait(&full[s], ph))) return false;
+            bool got = !below || mbar_wait(&full[s], ph);
+            if ((s & (H - 1)) == 0) got = mbar_wait(&opfull[s / H], ph) && got;
+            if (!__all_sync(ALL, got)) return false;
             take(s, o);
             return true;
         };
-        // Row q has been read: its slot is armed for row q + XR, whose operands
-        // are fetched, and handed back to the plane below by halves.
+        // The H rows up to q have been read: their slots are handed back to the
+        // plane below and fetch the operands of the rows XR later.
         auto done = [&](int q, int s) {
+            if ((s & (H - 1)) != H - 1) return;
             __syncwarp();
-            if (lane == 0 && q + XR < nrow) {
-                mbar_arrive_expect_tx(&full[s], lbytes);
-                line_fetch(fdst + s * 2 * LBYTES, fsrc, lbytes, fbar + 8u * s);
+            if (lane == 0) {
+                if (below && q + H + 1 < nrow) mbar_arrive(&empty[s / H]);
+                fetch(q + H + 1);
             }
-            if (below && lane == 0 && s % H == H - 1 && q + H + 1 < nrow) mbar_arrive(&empty[s / H]);
-            fsrc += rstep;
         };
 
         // One row: gr holds its right-hand side and the plane below's share.
@@ -378,9 +420,9 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
 #pragma unroll
             for (int l = 0; l < 5; ++l)
                 if (l < nlev) b = fma(lev[l], __shfl_up_sync(ALL, b, 1 << l), b);
+            const bool more = r + 1 < nrow;
             const int s1 = (u + 1) % XR;
             const unsigned ph1 = u + 1 == XR ? ph ^ 1u : ph;
-            const bool more = r + 1 < nrow;
             const bool rdy = !more || ask(s1, ph1, gr);
             // the carry of the segment before
             if (seg > 0) {
@@ -404,7 +446,7 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
             }
             // hand the row to the plane above, then to global memory
             if (to_ring) {
-                if (u % H == 0 && r >= XR &&
+                if ((u & (H - 1)) == 0 && r >= XR &&
                     !__all_sync(ALL, mbar_wait(&up_full[XR + u / H], ph ^ 1u)))
                     return false;
                 line_store<V, E>(up_ring + u * 64 * E, x, false);
@@ -414,7 +456,7 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
                 V w[E];
 #pragma unroll
                 for (int e = 0; e < E; ++e) w[e] = line_value(x[e]);
-                xch_put<E>(xout, w);
+                xch_put(xout, w);
                 xout += xrow;
             }
             if (on) {
@@ -443,7 +485,6 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
             return true;
         };
         bool good = get(0, 0u, gr);
-        if (good) done(0, 0);
         unsigned ph = 0;
         for (int r0 = 0; r0 < nrow && good; r0 += XR, ph ^= 1u) {
 #pragma unroll
@@ -462,32 +503,37 @@ __global__ void __launch_bounds__(32 * (LINE_MAX_WARPS + LINE_MAX_COURIERS), 1) 
 }
 
 // ------------------------------------------------------------------ host
-constexpr int LINE_E = 4;  // points per lane
-
+// Kernels by points per lane: 1, 2, 4 in FP64, 2, 4 in FP32.
 template <int MODE, typename V>
-static const void* line_fn() { return (const void*)k_line<MODE, V, LINE_E>; }
-
-static size_t line_smem(int S, int KP, int rows, size_t vsize) {
-    const size_t nw = (size_t)S * KP;
-    return nw * (LINE_XR * 64 * LINE_E * vsize + LINE_BARS * 8 + rows * vsize);
+static void (*line_fn(int E))(const LineArgs<V>) {
+    if constexpr (sizeof(V) == 8)
+        if (E == 1) return k_line<MODE, V, 1>;
+    return E == 2 ? k_line<MODE, V, 2> : k_line<MODE, V, 4>;
+}
+template <typename V>
+static int line_chunks_of(int E, int nx) {
+    return E == 1 ? line_chunks<V, 1>(nx) : E == 2 ? line_chunks<V, 2>(nx) : line_chunks<V, 4>(nx);
 }
 
 // Splits the slab columns over CTAs of KP planes for one kernel.  False when
-// the line sweeps do not take the grid: lines of more than LINE_MAX_WARPS
-// warps, or rows that the mailboxes have no room for.
-static bool line_plan(const tbl_handle* h, const void* fn, size_t vsize, int rows, int nblk, int kp, LineShape& q) {
-    const int C = (h->g.nx - 2) / LINE_E + 1;
+// the line sweeps do not take the grid: lines of more warps than a CTA may
+// have, or rows that the mailboxes have no room for.
+template <int MODE, typename V>
+static bool line_plan(const tbl_handle* h, int rows, int nblk, int E, int kp, LineShape& q) {
     q = LineShape();
-    q.S = (C + 31) / 32;
-    if (q.S > LINE_MAX_WARPS) return false;
-    q.KP = std::min(kp, LINE_MAX_WARPS / q.S);
+    q.E = E;
+    q.S = (line_chunks_of<V>(E, h->g.nx) + 31) / 32;
+    if (q.S > line_max_warps(E)) return false;
+    q.KP = std::min(kp, line_max_warps(E) / q.S);
     q.NC = std::min(q.S, LINE_MAX_COURIERS);
     q.rows = rows;
     q.nblk = nblk;
-    q.smem = line_smem(q.S, q.KP, rows, vsize);
+    const size_t nw = (size_t)q.S * q.KP;
+    q.smem = nw * (LINE_XR * 64 * E * sizeof(V) + LINE_BARS * 8 + rows * sizeof(V));
     if (q.smem > LINE_MAX_SMEM) return false;
     for (int r = 0; r < h->P; ++r) q.ncta += (h->en[r] - h->bn[r] + 1 + q.KP - 1) / q.KP * nblk;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, LINE_MAX_SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute((const void*)line_fn<MODE, V>(E), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             LINE_MAX_SMEM) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
@@ -508,22 +554,41 @@ static int line_table(const tbl_handle* h, LineShape& q) {
 
 template <typename V>
 static int line_init(tbl_handle* h) {
-    const int J = h->g.ny - 2;
-    const int kp = sizeof(V) == 8 ? 1 : 2;
+    const int J = h->g.ny - 2, nx = h->g.nx;
     const bool span = (h->cfg.flags & TBL_FLAG_SSOR_SPAN_BLOCKS) != 0;
     const int brows = span ? std::min(32, J) : J, nblk = span ? (J + 31) / 32 : 1;
+    // Points per lane and planes per CTA.  An FP64 row costs about 65 cycles
+    // per FMA a warp issues: few points per lane spread a line over more of the
+    // SM's four FP64 pipes, but every warp pays for the scan.  SSOR sweep at
+    // E = 1 / 2 / 4: 62 / 70 / 94 us at 128 x 66 x 64, 84 / 84 / 107 at
+    // 201 x 77 x 59, 263 / 185 / 198 at 512 x 130 x 128.  Where the three
+    // components of a GS sweep have more than two CTAs per SM the FP64 pipes
+    // are the bound and the fewest FMAs per point win (512 x 130 x 128: 770 /
+    // 510 / 450 us; 128 x 66 x 64, one CTA per SM: 68 / 82 / 114).  FP32 rows
+    // are bound by latency: 4 points, and 2 planes per CTA shorten the hand-over
+    // (SSOR at 512: 108 / 100 / 104 us with 1 / 2 / 3; GS 204 / 188 / 134).
+    int E[2] = {4, 4}, kp[2] = {3, 2};  // GS, SSOR
+    if (sizeof(V) == 8) {
+        E[1] = nx <= 130 ? 1 : 2;
+        E[0] = 3 * (h->g.nz - 2) > 2 * h->n_sm ? 4 : E[1];
+        kp[0] = E[0] == 4 ? 2 : 1;
+        kp[1] = 1;
+        for (int& e : E)
+            while (e < 4 && (line_chunks_of<V>(e, nx) + 31) / 32 > line_max_warps(e)) e *= 2;
+    }
     LineShape q[3];
-    const bool gs = line_plan(h, line_fn<0, V>(), sizeof(V), J, 1, kp, q[0]);
-    const bool ssor = line_plan(h, line_fn<1, V>(), sizeof(V), brows, nblk, kp, q[1]) &&
-                      line_plan(h, line_fn<2, V>(), sizeof(V), brows, nblk, kp, q[2]);
+    const bool gs = line_plan<0, V>(h, J, 1, E[0], kp[0], q[0]);
+    const bool ssor = line_plan<1, V>(h, brows, nblk, E[1], kp[1], q[1]) &&
+                      line_plan<2, V>(h, brows, nblk, E[1], kp[1], q[2]);
+    size_t words = 0;
     for (int m = 0; m < 3; ++m) {
         if (m == 0 ? !gs : !ssor) continue;
         h->line[m] = q[m];
         const int st = line_table(h, h->line[m]);
         if (st != TBL_OK) return st;
+        words = std::max(words, (size_t)(m == 0 ? 3 : 1) * h->g.nz * J * 32 * q[m].E * q[m].S);
     }
-    if (gs || ssor) {
-        const size_t words = (size_t)(gs ? 3 : 1) * h->g.nz * J * 32 * LINE_E * q[gs ? 0 : 1].S;
+    if (words > 0) {
         TBL_CUDA_TRY(cudaMalloc(&h->line_xch, words * sizeof(V)));
         TBL_CUDA_TRY(cudaMemset(h->line_xch, 0xff, words * sizeof(V)));
         TBL_CUDA_TRY(cudaMalloc(&h->line_ticket, 2 * sizeof(unsigned)));
@@ -557,7 +622,7 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
 template <int MODE, typename V>
 static int line_launch(tbl_handle* h, const LineShape& q, LineArgs<V>& a, int nsets) {
     a.nsets = nsets;
-    k_line<MODE, V, LINE_E><<<q.ncta * nsets, 32 * (q.S * q.KP + q.NC), q.smem, h->stream>>>(a);
+    line_fn<MODE, V>(q.E)<<<q.ncta * nsets, 32 * (q.S * q.KP + q.NC), q.smem, h->stream>>>(a);
     TBL_CUDA_TRY(cudaGetLastError());
     h->launches++;
     return TBL_OK;
@@ -586,7 +651,7 @@ int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* sk
     // streamwise blocks of the same points as the wavefront sweep's
     if (h->ssor_nib > 1) {
         const int ch = sweep_chunk(sizeof(V)), C = (h->g.nx - 2) / ch + 1;
-        a.cb = (C + h->ssor_nib - 1) / h->ssor_nib * (ch / LINE_E);
+        a.cb = (C + h->ssor_nib - 1) / h->ssor_nib * (ch / q.E);
     }
     return bwd ? line_launch<2, V>(h, q, a, 1) : line_launch<1, V>(h, q, a, 1);
 }

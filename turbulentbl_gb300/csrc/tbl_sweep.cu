@@ -1,6 +1,8 @@
-// tbl_sweep.cu -- pipelined wavefront sweeps (FP64): lexicographic
-// Gauss-Seidel for the implicit diffusion and the forward/backward block-SSOR
-// preconditioner of GMRES.
+// tbl_sweep.cu -- pipelined wavefront sweeps: lexicographic Gauss-Seidel for
+// the implicit diffusion and the forward/backward block-SSOR preconditioner of
+// GMRES, for the grids that the line-scan sweeps (tbl_line.cu) do not take:
+// lines of more warps than a CTA may have, or whose rings do not fit its shared
+// memory.
 //
 // The reference sweeps each MPI slab in lexicographic order (i fastest, then
 // j, then k; dnstbl2/dnstbl.f90:830-868, :1022-1042, :1115-1135).  A point
