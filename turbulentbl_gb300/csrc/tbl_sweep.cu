@@ -109,7 +109,8 @@ constexpr int XR_SLOTS = 8;  // slots of the ring a CTA receives its plane-below
 // sweeps were slower).  Each lane's operand buffer holds 4 CH positions:
 // position q of the line at element q % (4 CH); chunks are copied two steps
 // ahead, so the live positions span 3 CH - 1 < 4 CH.
-template <typename Val> constexpr int sweep_ch() { return sweep_chunk(sizeof(Val)); }
+template <typename Val> constexpr int sweep_ch() { return sizeof(Val) == 4 ? 8 : 4; }
+static_assert(sweep_ch<float>() == sweep_chunk(4) && sweep_ch<double>() == sweep_chunk(8), "the streamwise blocks' unit");
 // Dynamic shared memory of a sweep CTA: the plane-to-plane ring and the operand buffers.
 template <typename Val> constexpr size_t sweep_smem() {
     return sizeof(Val) * KG * (RING * 32 * sweep_ch<Val>() + 32 * 4 * sweep_ch<Val>()) +
