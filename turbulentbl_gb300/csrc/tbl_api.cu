@@ -118,7 +118,7 @@ static void free_all(tbl_handle* h) {
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
                     h->uold1, h->x3, h->jacinv, h->jac2, h->Ab, h->At, h->Ap, h->rAp, h->gs_coef, h->gs_coef_f, h->lap_scale, h->coef_f, h->ssor_scale, h->ssor_scale_f, h->line_xch, h->line_ticket, h->line[0].ctas, h->line[1].ctas, h->line[2].ctas, h->usum2, h->vsum2,
                     h->wsum2, h->wt, h->ume1, h->bltkns, h->newk, h->ufl_file, h->ufl_live, h->ufl_full,
-                    h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy,
+                    h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_G, h->gs_hs,
                     h->red.partial, h->red.count, h->halo, h->flags, h->ctas, h->slabs, h->err};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -210,6 +210,9 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
         for (int c = 0; c < 3; ++c) { TRY(dalloc(&h->U[c], vol)); TRY(dalloc(&h->Q[c], vol)); }
         TRY(dalloc(&h->Pr, vol)); TRY(dalloc(&h->RH, vol)); TRY(dalloc(&h->PRE, 3 * vol));
         TRY(dalloc(&h->V, vol * (size_t)(cfg->kmax + 1)));
+        TRY(dalloc(&h->gs_d, (size_t)cfg->kmax + 1));
+        TRY(dalloc(&h->gs_G, 8 * ((size_t)cfg->kmax + 1)));
+        TRY(dalloc(&h->gs_hs, (size_t)cfg->kmax + 1));
     }
     TRY(dalloc(&h->uold1, pl));
     TRY(dalloc(&h->x3, (size_t)nz)); TRY(dalloc(&h->jacinv, (size_t)nz)); TRY(dalloc(&h->jac2, (size_t)nz));
@@ -564,7 +567,7 @@ static int gmres_mixed(tbl_handle* h, std::vector<int32_t>& kits, tbl_step_stats
 
 // ------------------------------------------------------------ GMRES
 int gmres(tbl_handle* h, const int32_t* rec, std::vector<int32_t>& kits, tbl_step_stats& st) {
-    const int kmax = h->cfg.kmax, K1 = kmax + 1;
+    const int kmax = h->cfg.kmax;
     const size_t vol = (size_t)h->g.vol;
     double sumav = 1.0;
     int m = 0, iters = 0;
@@ -592,14 +595,10 @@ int gmres(tbl_handle* h, const int32_t* rec, std::vector<int32_t>& kits, tbl_ste
         if (m == 1 && std::isnan(rho)) { status = TBL_ERR_NAN; break; }
         if (m == 1 && !(rho > 0.0)) { status = TBL_ERR_ZERO_RHS; break; }
         sumav = h->hpin[2];
-        {
-            ProfScope ps(h, TBL_PROF_VEC, 2.0 * wN);
-            TRY(launch_scale_by_inv(h, V0, &h->sc->rho));
-        }
         int kit = 0;
         const int target = rec ? rec[m] : 0;
-        // One Arnoldi step (:1059-1191): preconditioned matvec, MGS, Givens,
-        // normalisation.  With skip, every kernel returns at once when an
+        // One Arnoldi step (:1059-1191): preconditioned matvec, MGS, Givens; the
+        // basis vectors are not divided by their norms.  With skip, every kernel returns at once when an
         // earlier step's Givens stopped the cycle.
         auto arnoldi_step = [&](int k, const int* skip) -> int {
             double* W = h->V + (size_t)k * vol;
@@ -611,23 +610,10 @@ int gmres(tbl_handle* h, const int32_t* rec, std::vector<int32_t>& kits, tbl_ste
                 ProfScope ps(h, TBL_PROF_SSOR_BWD, 2.0 * wN);
                 TRY(launch_ssor_bwd(h, W, skip));
             }
-            double* hcol = h->h + (size_t)K1 * (k - 1);
             {
-                // passes: <v1,w>; (k-1) x {w -= h v_k; <v_k+1,w>}; w -= h v_k, ||w||
-                ProfScope ps(h, TBL_PROF_MGS, (2.0 + 4.0 * (k - 1) + 3.0) * wN);
-                TRY(launch_mgs(h, W, nullptr, nullptr, V0, &hcol[0], 0, skip));
-                for (int kk = 1; kk <= k - 1; ++kk)
-                    TRY(launch_mgs(h, W, h->V + (size_t)(kk - 1) * vol, &hcol[kk - 1], h->V + (size_t)kk * vol,
-                                   &hcol[kk], 0, skip));
-                TRY(launch_mgs(h, W, h->V + (size_t)(k - 1) * vol, &hcol[k - 1], nullptr, &hcol[k], 1, skip));
-            }
-            {
-                ProfScope ps(h, TBL_PROF_SMALL, 0.0);
-                TRY(launch_givens(h, k, skip, h->cfg.errtol));
-            }
-            {
-                ProfScope ps(h, TBL_PROF_VEC, 2.0 * wN);
-                TRY(launch_scale_by_inv(h, W, &h->sc->red[8], skip));
+                // every basis vector twice, w once more than twice per block of 8, then the Givens rotation
+                ProfScope ps(h, TBL_PROF_MGS, (2.0 * k + 2.0 * ((k + 7) / 8) + 1.0) * wN);
+                TRY(launch_gs(h, W, k, skip, h->cfg.errtol));
             }
             return TBL_OK;
         };

@@ -47,10 +47,7 @@ int launch_lap_tma(tbl_handle* h, const T* X, T* R, T aw, T as, const T* Ab, con
 
 // tbl_krylov.cu
 int launch_dot(tbl_handle* h, const double* a, const double* b, double* out, int op);
-int launch_mgs(tbl_handle* h, double* w, const double* vk, const double* hk, const double* vn, double* out, int op,
-               const int* skip = nullptr);
-int launch_scale_by_inv(tbl_handle* h, double* w, const double* denom, const int* skip = nullptr);
-int launch_givens(tbl_handle* h, int kit, const int* skip = nullptr, double stop_at = 0.0);
+int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at);
 int launch_backsub_update(tbl_handle* h, int kit);
 int launch_restart_init(tbl_handle* h, int first);
 int launch_ppe_resid(tbl_handle* h);

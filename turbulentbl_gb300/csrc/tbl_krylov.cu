@@ -56,80 +56,238 @@ __device__ __forceinline__ void st_keep(double2* a, double2 v, unsigned long lon
                  : "memory");
 }
 
-// One modified Gram-Schmidt pass (:1140-1150):
-//   w -= (*hk) * vk          (skipped when vk == nullptr)
-//   *out = sum(vn * w)       (vn == nullptr: sum(w*w), op 1 takes the sqrt)
-// Two elements per thread per iteration on a grid of MGS_BLOCKS_PER_SM
-// blocks per SM.  The basis vectors stream through with evict-first loads;
-// w, read and written by every pass of an Arnoldi step (69 MB at
-// 512x130x128, inside the 129 MB L2), is loaded and stored evict-last so
-// that it stays in L2 from pass to pass.  With everything evict-first a
-// pass ran at 1.01 of the measured copy bandwidth in a stand-alone copy
-// (0.78 with one element, default caching and 8 blocks per SM).
-constexpr int MGS_BLOCKS_PER_SM = 4;
-__global__ void __launch_bounds__(RED_THREADS) k_mgs(long long n2, double2* __restrict__ w,
-                                                  const double2* __restrict__ vk, const double* __restrict__ hk,
-                                                  const double2* __restrict__ vn, RedWork rw, int slot, double* out,
-                                                  int op, const int* __restrict__ skip) {
-    if (skip && *skip) return;  // an Arnoldi step enqueued ahead of a converged one
-    __shared__ double s_red[RED_THREADS / 32];
-    const double hv = vk ? *hk : 0.0;
-    const unsigned long long keep = l2_keep_policy();
-    double acc = 0.0;
-    const long long st = (long long)gridDim.x * blockDim.x;
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (; q + st < n2; q += 2 * st) {
-        double2 x0 = ld_keep(w + q, keep), x1 = ld_keep(w + q + st, keep);
-        if (vk) {
-            const double2 v0 = __ldcs(vk + q), v1 = __ldcs(vk + q + st);
-            x0.x = x0.x - hv * v0.x;
-            x0.y = x0.y - hv * v0.y;
-            x1.x = x1.x - hv * v1.x;
-            x1.y = x1.y - hv * v1.y;
-            st_keep(w + q, x0, keep);
-            st_keep(w + q + st, x1, keep);
+// Warp sum of 16 FP64 values per lane, as a reduce-scatter: at each of the
+// offsets 16, 8, 4, 2 a lane keeps half of its values, sends the other half to
+// lane ^ offset and adds what it receives; a last exchange with lane ^ 1
+// completes the sums.  Lane l then holds the warp total of value l >> 1: 16
+// FP64 additions per lane instead of the 80 of 16 shuffle trees (FP64 runs at
+// 1/64 of the FP32 rate on this GPU).  Fixed order: deterministic.
+__device__ __forceinline__ double warp_reduce_scatter16(double (&a)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 8; half >= 1; half >>= 1) {
+        const bool up = (lane & (2 * half)) != 0;  // keeps the upper half of the current values
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const double keep = up ? a[i + half] : a[i];
+            const double send = up ? a[i] : a[i + half];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
         }
-        const double2 y0 = vn ? __ldcs(vn + q) : x0, y1 = vn ? __ldcs(vn + q + st) : x1;
-        acc += y0.x * x0.x;
-        acc += y0.y * x0.y;
-        acc += y1.x * x1.x;
-        acc += y1.y * x1.y;
     }
-    if (q < n2) {
-        double2 x = ld_keep(w + q, keep);
-        if (vk) {
-            const double2 v = __ldcs(vk + q);
-            x.x = x.x - hv * v.x;
-            x.y = x.y - hv * v.y;
-            st_keep(w + q, x, keep);
-        }
-        const double2 y = vn ? __ldcs(vn + q) : x;
-        acc += y.x * x.x;
-        acc += y.y * x.y;
-    }
-    double bt = block_sum(acc, s_red);
-    grid_finish(bt, rw, slot, gridDim.x, blockIdx.x, out, op);
+    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
-// w /= *denom when *denom != 0 (:1158-1161); multiplies by the reciprocal
-__global__ void k_scale_inv(long long n2, double2* __restrict__ w, const double* __restrict__ denom,
-                            const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    const double d = *denom;
-    if (!(d > 0.0 || d < 0.0)) return;
-    const double r = 1.0 / d;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n2; q += (long long)gridDim.x * blockDim.x) {
-        double2 x = w[q];
-        x.x *= r;
-        x.y *= r;
-        w[q] = x;
+// Givens rotations for column kit (1-based) (:1165-1189) by one thread.  h2:
+// the column, kit + 1 values, c2, s2: the rotations so far; staged in shared
+// memory, so that the chain of kit rotations does not wait for global loads.
+// H: the column in global memory (h2 may be H itself).  With ahead (Arnoldi
+// steps enqueued ahead) the cycle stops when the estimate sumav reaches stop_at
+// (the host's loop test, evaluated on the same double).
+__device__ __forceinline__ void givens_column(int kit, const double* h2, const double* c2, const double* s2, double* H,
+                                              double* gg, double* gc, double* gs, DevScalars* sc, bool ahead,
+                                              double stop_at) {
+    double cur = h2[0];
+    for (int i = 0; i < kit - 1; ++i) {
+        const double nx = h2[i + 1];
+        H[i] = c2[i] * cur - s2[i] * nx;
+        cur = s2[i] * cur + c2[i] * nx;
     }
+    const double last = h2[kit];
+    double diag = cur, sub = last;
+    const double nu = sqrt(cur * cur + last * last);
+    double gk = gg[kit - 1], gkp = gg[kit];
+    if (nu > 0.0) {
+        const double c = cur / nu, s = -last / nu;
+        gc[kit - 1] = c;
+        gs[kit - 1] = s;
+        diag = c * cur - s * last;
+        sub = 0.0;
+        const double a = c * gk - s * gkp, b = s * gk + c * gkp;
+        gk = a;
+        gkp = b;
+        gg[kit - 1] = gk;
+        gg[kit] = gkp;
+    }
+    H[kit - 1] = diag;
+    H[kit] = sub;
+    const double rho = fabs(gkp);
+    sc->rho = rho;
+    sc->sumav = rho / sc->sumnor;
+    if (ahead && !(sc->sumav > stop_at)) sc->stop = 1;
+}
+
+// ---------------------------------------------------- Gram-Schmidt (FP64)
+// Modified Gram-Schmidt (:1140-1161) over blocks of 8 basis vectors.  One pass
+// takes a block's projections off w and forms the next block's dot products:
+//   w -= sum_i (h_i d_i / d_k) v_i   (i in the previous block)
+//   S_i = <v_i, w>                   (i in the next block), or <w, w> at the end
+// Inside a block the dots are all taken against the same w; the modified
+// Gram-Schmidt coefficients follow from h_i = c_i - sum_{j<i} <v_i, v_j> h_j,
+// the products of a block's vectors being formed once, with the pass in which
+// their last one is the newest (the product of the block's projections, also
+// when the basis has lost orthogonality).
+// The basis vectors are kept as they come out of this, not divided by their
+// norms: v_i d_i with d_i = 1 / |v_i| is the reference's unit vector, and w =
+// M^-1 A v_k, so c_i = d_i d_k S_i.  The division pass is gone.
+//
+// Bound: two FP64 FMAs per element and basis vector (28.8 us a vector at
+// 512 x 130 x 128 and 600 G FMA/s) and two reads of every basis vector (28 us
+// at 5 TB/s), against 43.6 us a vector with one pass per vector; on small grids
+// the number of launches, a ninth as many.
+constexpr int GSB = 8;
+struct GsPass {
+    long long n2;
+    double2* w;
+    const double2* V;      // basis, n2 apart
+    int p0, np, q0, nq;    // previous and next block: first vector, vectors
+    int k;                 // vectors in the basis
+    double *d, *G;         // 1/|v_i|; <v_i, v_j> / (|v_i| |v_j|), j in i's block, [i][GSB]
+    double *hcol, *hs;     // Hessenberg column; h_i d_i / d_k
+    double* partial;       // [16][max_blocks]
+    unsigned* count;
+    int max_blocks;
+    int K1;
+    double *h, *gg, *gc, *gs;
+    DevScalars* sc;
+    const int* skip;
+    double stop_at;
+    int staged;
+};
+
+// NP, NQ: 8 for a full block, 0 for none, -1 for a block of fewer.  GRAM: the
+// next block holds the newest vector (its last).
+template <int NP, int NQ, bool GRAM>
+__global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
+    if (a.skip && *a.skip) return;  // an Arnoldi step enqueued ahead of a converged one
+    constexpr int NW = RED_THREADS / 32;
+    __shared__ double s_red[16 * NW];
+    __shared__ double s_val[16];
+    extern __shared__ double s_h[];  // 3 (k + 1) values, unless they do not fit (a.staged)
+    __shared__ bool s_last;
+    const int np = NP >= 0 ? NP : a.np, nq = NQ >= 0 ? NQ : a.nq;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned long long keep = l2_keep_policy();
+    double hp[NP != 0 ? GSB : 1];
+    if (NP != 0)
+#pragma unroll
+        for (int e = 0; e < GSB; ++e) hp[e] = e < np ? a.hs[a.p0 + e] : 0.0;
+    double acc[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+    const long long st = (long long)gridDim.x * blockDim.x;
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < a.n2; q += st) {
+        double2 x = ld_keep(a.w + q, keep);
+        double2 y[NQ != 0 ? GSB : 1];
+        if (NP != 0) {
+            double2 v[GSB];
+#pragma unroll
+            for (int e = 0; e < GSB; ++e)
+                if (e < np) v[e] = __ldcs(a.V + (long long)(a.p0 + e) * a.n2 + q);
+            if (NQ != 0)
+#pragma unroll
+                for (int e = 0; e < GSB; ++e)
+                    if (e < nq) y[e] = __ldcs(a.V + (long long)(a.q0 + e) * a.n2 + q);
+#pragma unroll
+            for (int e = 0; e < GSB; ++e)
+                if (e < np) {
+                    x.x = fma(-hp[e], v[e].x, x.x);
+                    x.y = fma(-hp[e], v[e].y, x.y);
+                }
+            st_keep(a.w + q, x, keep);
+        } else {
+#pragma unroll
+            for (int e = 0; e < GSB; ++e)
+                if (e < nq) y[e] = __ldcs(a.V + (long long)(a.q0 + e) * a.n2 + q);
+        }
+        if (NQ != 0) {
+            double2 m = make_double2(0.0, 0.0);
+            if (GRAM)
+#pragma unroll
+                for (int e = 0; e < GSB; ++e)
+                    if (e == nq - 1) m = y[e];
+#pragma unroll
+            for (int e = 0; e < GSB; ++e)
+                if (e < nq) {
+                    acc[e] = fma(y[e].y, x.y, fma(y[e].x, x.x, acc[e]));
+                    if (GRAM && e < nq - 1) acc[8 + e] = fma(y[e].y, m.y, fma(y[e].x, m.x, acc[8 + e]));
+                }
+        } else {
+            acc[0] = fma(x.y, x.y, fma(x.x, x.x, acc[0]));
+        }
+    }
+    const double tot = warp_reduce_scatter16(acc);  // value lane >> 1
+    if ((lane & 1) == 0) s_red[(lane >> 1) * NW + wid] = tot;
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        double t = 0.0;
+        for (int q = 0; q < NW; ++q) t += s_red[threadIdx.x * NW + q];
+        a.partial[(size_t)threadIdx.x * a.max_blocks + blockIdx.x] = t;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(a.count, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    // the last block: every value's partials in a fixed order, one warp per value
+    __threadfence();
+    for (int v = wid; v < 16; v += NW) {
+        if (NQ == 0 ? v > 0 : (v < 8 ? v >= nq : !GRAM || v - 8 >= nq - 1)) continue;
+        const double* p = a.partial + (size_t)v * a.max_blocks;
+        double t = 0.0;
+        for (int q = lane; q < (int)gridDim.x; q += 32) t += __ldcg(p + q);
+        t = warp_sum(t);
+        if (lane == 0) s_val[v] = t;
+    }
+    double* const hc = a.h + (size_t)a.K1 * (a.k - 1);
+    if (NQ == 0 && a.staged)  // the Givens rotations' inputs meanwhile
+        for (int i = threadIdx.x; i < a.k; i += blockDim.x) {
+            s_h[i] = hc[i];
+            s_h[a.k + 1 + i] = a.gc[i];
+            s_h[2 * (a.k + 1) + i] = a.gs[i];
+        }
+    __syncthreads();
+    const double dk = a.d[a.k - 1];
+    if (NQ != 0) {
+        if (wid == 0) {
+            const int i = a.q0 + lane;
+            const double di = lane < nq ? a.d[i] : 0.0;
+            double c = lane < nq ? di * dk * s_val[lane] : 0.0;
+            double grow[GSB];  // this lane's row of the block's products
+#pragma unroll
+            for (int j = 0; j < GSB - 1; ++j) {
+                grow[j] = 0.0;
+                if (lane < nq && j < lane) {
+                    if (GRAM && lane == nq - 1) {
+                        grow[j] = a.d[a.q0 + j] * dk * s_val[8 + j];
+                        a.G[(size_t)i * GSB + j] = grow[j];
+                    } else {
+                        grow[j] = a.G[(size_t)i * GSB + j];
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < GSB - 1; ++j) c = fma(-grow[j], __shfl_sync(0xffffffffu, c, j), c);
+            if (lane < nq) {
+                a.hcol[i] = c;
+                a.hs[i] = c * di / dk;
+            }
+        }
+    } else if (threadIdx.x == 0) {
+        const double nh = sqrt(s_val[0]), nrm = dk * nh;
+        a.d[a.k] = nh > 0.0 ? 1.0 / nh : 1.0;
+        double* const h2 = a.staged ? s_h : hc;
+        h2[a.k] = nrm;
+        givens_column(a.k, h2, a.staged ? s_h + a.k + 1 : a.gc, a.staged ? s_h + 2 * (a.k + 1) : a.gs, hc, a.gg, a.gc,
+                      a.gs, a.sc, a.skip != nullptr, a.stop_at);
+    }
+    if (threadIdx.x == 0) *a.count = 0u;
 }
 
 // Start of a restart (:958-963, :1048-1056): zero h, c, s, g, y; g(1) = rho;
 // sumnor at the first restart; sumav = rho/sumnor.
+// d: 1/|v_i| of the basis vectors, kept as they come (FP64), or null.
 __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double* gs, double* gy, DevScalars* sc,
-                               int first) {
+                               int first, double* d) {
     for (int q = threadIdx.x; q < K1 * K1; q += blockDim.x) h[q] = 0.0;
     for (int q = threadIdx.x; q < K1; q += blockDim.x) { gg[q] = 0.0; gc[q] = 0.0; gs[q] = 0.0; gy[q] = 0.0; }
     __syncthreads();
@@ -139,54 +297,40 @@ __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double
         if (first) sc->sumnor = rho;
         sc->sumav = rho / sc->sumnor;
         gg[0] = rho;
+        if (d) d[0] = rho > 0.0 ? 1.0 / rho : 1.0;
     }
 }
 
-// Givens rotations for column kit (1-based) (:1165-1189).  h(kit+1,kit) holds
-// the norm of the orthogonalised vector; it is saved for the normalisation.
-// With skip (Arnoldi steps enqueued ahead): returns at once when a previous
-// step stopped the cycle, and stops it itself when the estimate sumav reaches
-// stop_at (the host's loop test, evaluated on the same double).
-__global__ void k_givens(int K1, int kit, double* h, double* gg, double* gc, double* gs, DevScalars* sc,
-                         const int* skip, double stop_at) {
-    if (threadIdx.x != 0) return;
+// The same as a kernel (mixed precision, kit <= 63); h(kit+1,kit), the norm of
+// the orthogonalised vector, is saved for the normalisation.
+__global__ void __launch_bounds__(64) k_givens(int K1, int kit, double* h, double* gg, double* gc, double* gs,
+                                               DevScalars* sc, const int* skip, double stop_at) {
     if (skip && *skip) return;
-    auto H = [&](int a, int b) -> double& { return h[(a - 1) + K1 * (b - 1)]; };
-    sc->red[8] = H(kit + 1, kit);
-    if (kit > 1) {
-        for (int i = 1; i <= kit - 1; ++i) {
-            double hik = gc[i - 1] * H(i, kit) - gs[i - 1] * H(i + 1, kit);
-            double hipk = gs[i - 1] * H(i, kit) + gc[i - 1] * H(i + 1, kit);
-            H(i, kit) = hik;
-            H(i + 1, kit) = hipk;
-        }
+    __shared__ double s_h[3][64];
+    double* H = h + (size_t)K1 * (kit - 1);
+    const int i = threadIdx.x;
+    if (i <= kit) s_h[0][i] = H[i];
+    if (i < kit) {
+        s_h[1][i] = gc[i];
+        s_h[2][i] = gs[i];
     }
-    double nu = sqrt(H(kit, kit) * H(kit, kit) + H(kit + 1, kit) * H(kit + 1, kit));
-    if (nu > 0.0) {
-        gc[kit - 1] = H(kit, kit) / nu;
-        gs[kit - 1] = -H(kit + 1, kit) / nu;
-        H(kit, kit) = gc[kit - 1] * H(kit, kit) - gs[kit - 1] * H(kit + 1, kit);
-        H(kit + 1, kit) = 0.0;
-        double gk = gc[kit - 1] * gg[kit - 1] - gs[kit - 1] * gg[kit];
-        double gkp = gs[kit - 1] * gg[kit - 1] + gc[kit - 1] * gg[kit];
-        gg[kit - 1] = gk;
-        gg[kit] = gkp;
-    }
-    double rho = fabs(gg[kit]);
-    sc->rho = rho;
-    sc->sumav = rho / sc->sumnor;
-    if (skip && !(sc->sumav > stop_at)) sc->stop = 1;
+    __syncthreads();
+    if (i != 0) return;
+    sc->red[8] = s_h[0][kit];
+    givens_column(kit, s_h[0], s_h[1], s_h[2], H, gg, gc, gs, sc, skip != nullptr, stop_at);
 }
 
-// y from the triangular h (:1193-1200), one thread
-__global__ void k_backsub(int K1, int kit, const double* h, const double* gg, double* gy) {
-    if (threadIdx.x != 0) return;
-    auto H = [&](int a, int b) -> double { return h[(a - 1) + K1 * (b - 1)]; };
-    gy[kit - 1] = gg[kit - 1] / H(kit, kit);
-    for (int i = kit - 1; i >= 1; --i) {
-        double yi = gg[i - 1];
-        for (int k = i + 1; k <= kit; ++k) yi = yi - H(i, k) * gy[k - 1];
-        gy[i - 1] = yi / H(i, i);
+// y from the triangular h (:1193-1200), one warp, a column at a time; with d
+// the coefficients of the basis vectors as they are kept, y_i / |v_i|.
+__global__ void __launch_bounds__(32) k_backsub(int K1, int kit, const double* h, double* gg, double* gy,
+                                                const double* d) {
+    const int lane = threadIdx.x;
+    for (int i = kit - 1; i >= 0; --i) {
+        const double* H = h + (size_t)K1 * i;
+        __syncwarp();
+        const double y = gg[i] / H[i];
+        for (int j = lane; j < i; j += 32) gg[j] -= H[j] * y;
+        if (lane == 0) gy[i] = d ? y * d[i] : y;
     }
 }
 
@@ -298,40 +442,59 @@ int launch_dot(tbl_handle* h, const double* a, const double* b, double* out, int
     return TBL_OK;
 }
 
-int launch_mgs(tbl_handle* h, double* w, const double* vk, const double* hk, const double* vn, double* out, int op,
-               const int* skip) {
-    int nb = MGS_BLOCKS_PER_SM * (h->n_sm > 0 ? h->n_sm : 148);
-    if (nb > red_blocks(h)) nb = red_blocks(h);
-    k_mgs<<<nb, RED_THREADS, 0, h->stream>>>(h->g.vol / 2, (double2*)w, (const double2*)vk, hk, (const double2*)vn,
-                                             h->red, 7, out, op, skip);
-    h->launches++;
-    return TBL_OK;
-}
-
-int launch_scale_by_inv(tbl_handle* h, double* w, const double* denom, const int* skip) {
-    int nb = red_blocks(h);
-    k_scale_inv<<<nb, RED_THREADS, 0, h->stream>>>(h->g.vol / 2, (double2*)w, denom, skip);
-    h->launches++;
+// Orthogonalises w against the k vectors of the basis, then the Givens rotation
+// of the column.
+int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) {
+    GsPass a = {};
+    a.n2 = h->g.vol / 2;
+    a.w = (double2*)w;
+    a.V = (const double2*)h->V;
+    a.k = k;
+    a.K1 = h->cfg.kmax + 1;
+    a.d = h->gs_d;
+    a.G = h->gs_G;
+    a.hs = h->gs_hs;
+    a.h = h->h;
+    a.hcol = h->h + (size_t)a.K1 * (k - 1);
+    a.gg = h->gg; a.gc = h->gc; a.gs = h->gs; a.sc = h->sc;
+    a.partial = h->red.partial;
+    a.count = h->red.count + 15;
+    a.max_blocks = h->red.max_blocks;
+    a.skip = skip;
+    a.stop_at = stop_at;
+    const size_t stage = 3 * (size_t)(k + 1) * sizeof(double);
+    a.staged = stage <= 40 * 1024;
+    long long nb = (a.n2 + RED_THREADS - 1) / RED_THREADS;
+    const long long wave = 2LL * (h->n_sm > 0 ? h->n_sm : 148);
+    if (nb > wave) nb = wave;
+    const int nblk = (k + GSB - 1) / GSB, rest = k - (nblk - 1) * GSB;  // vectors of the last block
+    auto run = [&](void (*fn)(const GsPass), bool last) {
+        fn<<<(unsigned)nb, RED_THREADS, last && a.staged ? stage : 0, h->stream>>>(a);
+        h->launches++;
+    };
+    for (int b = 0; b <= nblk; ++b) {
+        a.p0 = (b - 1) * GSB;
+        a.np = b == 0 ? 0 : b == nblk ? rest : GSB;
+        a.q0 = b * GSB;
+        a.nq = b == nblk ? 0 : b == nblk - 1 ? rest : GSB;
+        const bool gram = b == nblk - 1, full = a.nq == GSB;
+        if (b == nblk) run(a.np == GSB ? k_gs_pass<8, 0, false> : k_gs_pass<-1, 0, false>, true);
+        else if (b == 0) run(!gram ? k_gs_pass<0, 8, false> : full ? k_gs_pass<0, 8, true> : k_gs_pass<0, -1, true>, false);
+        else run(!gram ? k_gs_pass<8, 8, false> : full ? k_gs_pass<8, 8, true> : k_gs_pass<8, -1, true>, false);
+    }
     return TBL_OK;
 }
 
 int launch_restart_init(tbl_handle* h, int first) {
     const int K1 = h->cfg.kmax + 1;
-    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first);
-    h->launches++;
-    return TBL_OK;
-}
-
-int launch_givens(tbl_handle* h, int kit, const int* skip, double stop_at) {
-    const int K1 = h->cfg.kmax + 1;
-    k_givens<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gc, h->gs, h->sc, skip, stop_at);
+    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, h->gs_d);
     h->launches++;
     return TBL_OK;
 }
 
 int launch_backsub_update(tbl_handle* h, int kit) {
     const int K1 = h->cfg.kmax + 1;
-    k_backsub<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy);
+    k_backsub<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy, h->gs_d);
     int nb = red_blocks(h);
     k_update<<<nb, RED_THREADS, 0, h->stream>>>(h->g.vol / 2, (double2*)h->PC, (const double2*)h->V, h->g.vol / 2,
                                                 h->gy, kit);
@@ -352,27 +515,6 @@ constexpr int LSG_G = 8;  // basis vectors per group (grid.y) of the dot pass
 
 __device__ __forceinline__ float dot4f(float4 a, float4 b) {
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)));
-}
-
-// Warp sum of 16 FP64 values per lane, as a reduce-scatter: at each of the
-// offsets 16, 8, 4, 2 a lane keeps half of its values, sends the other half to
-// lane ^ offset and adds what it receives; a last exchange with lane ^ 1
-// completes the sums.  Lane l then holds the warp total of value l >> 1: 16
-// FP64 additions per lane instead of the 80 of 16 shuffle trees (FP64 runs at
-// 1/64 of the FP32 rate on this GPU).  Fixed order: deterministic.
-__device__ __forceinline__ double warp_reduce_scatter16(double (&a)[16]) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int half = 8; half >= 1; half >>= 1) {
-        const bool up = (lane & (2 * half)) != 0;  // keeps the upper half of the current values
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-            const double keep = up ? a[i + half] : a[i];
-            const double send = up ? a[i] : a[i + half];
-            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
-        }
-    }
-    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
 // d[i] = <v_i, w>, g[i] = <v_i, v_{nv-1}> for the G basis vectors of group
@@ -562,7 +704,7 @@ int launch_scale_by_inv_f(tbl_handle* h, float* w, const double* denom, const in
 
 int launch_backsub_update_f(tbl_handle* h, int kit) {
     const int K1 = h->cfg.mixed_kmax + 1;
-    k_backsub<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy);
+    k_backsub<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy, h->gs_d);
     int nb = red_blocks(h);
     k_update_f<<<nb, RED_THREADS, 0, h->stream>>>(h->g.vol / 4, h->PC, (const float4*)h->Vf, h->g.vol / 4, h->gy,
                                                   kit);
@@ -571,13 +713,13 @@ int launch_backsub_update_f(tbl_handle* h, int kit) {
 }
 
 int launch_restart_init_k(tbl_handle* h, int first, int K1) {
-    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first);
+    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, nullptr);
     h->launches++;
     return TBL_OK;
 }
 
 int launch_givens_k(tbl_handle* h, int kit, int K1, const int* skip, double stop_at) {
-    k_givens<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gc, h->gs, h->sc, skip, stop_at);
+    k_givens<<<1, 64, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gc, h->gs, h->sc, skip, stop_at);
     h->launches++;
     return TBL_OK;
 }
