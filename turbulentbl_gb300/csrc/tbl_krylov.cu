@@ -56,25 +56,30 @@ __device__ __forceinline__ void st_keep(double2* a, double2 v, unsigned long lon
                  : "memory");
 }
 
-// Warp sum of 16 FP64 values per lane, as a reduce-scatter: at each of the
-// offsets 16, 8, 4, 2 a lane keeps half of its values, sends the other half to
-// lane ^ offset and adds what it receives; a last exchange with lane ^ 1
-// completes the sums.  Lane l then holds the warp total of value l >> 1: 16
-// FP64 additions per lane instead of the 80 of 16 shuffle trees (FP64 runs at
-// 1/64 of the FP32 rate on this GPU).  Fixed order: deterministic.
-__device__ __forceinline__ double warp_reduce_scatter16(double (&a)[16]) {
+// Warp sums of N FP64 values per lane (N = 16, 8 or 1), as a reduce-scatter:
+// at each of the offsets 16, 8, .. a lane keeps half of its values, sends the
+// other half to lane ^ offset and adds what it receives; when one is left the
+// remaining offsets complete it.  Lane l then holds the warp total of value
+// l / (32 / N): 16 FP64 additions per lane for 16 values instead of the 80 of 16
+// shuffle trees (FP64 runs at 1/64 of the FP32 rate on this GPU).  Fixed order:
+// deterministic.
+template <int N>
+__device__ __forceinline__ double warp_reduce_scatter(double (&a)[N]) {
     const int lane = threadIdx.x & 31;
+    int off = 16;
 #pragma unroll
-    for (int half = 8; half >= 1; half >>= 1) {
-        const bool up = (lane & (2 * half)) != 0;  // keeps the upper half of the current values
+    for (int half = N / 2; half >= 1; half >>= 1, off >>= 1) {
+        const bool up = (lane & off) != 0;  // keeps the upper half of the current values
 #pragma unroll
         for (int i = 0; i < half; ++i) {
             const double keep = up ? a[i + half] : a[i];
             const double send = up ? a[i] : a[i + half];
-            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
         }
     }
-    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+#pragma unroll
+    for (int o = 32 / (2 * N); o >= 1; o >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+    return a[0];
 }
 
 // Givens rotations for column kit (1-based) (:1165-1189) by one thread.  h2:
@@ -139,7 +144,7 @@ struct GsPass {
     long long n2;
     double2* w;
     const double2* V;      // basis, n2 apart
-    int p0, np, q0, nq;    // previous and next block: first vector, vectors
+    int p0, q0;            // first vector of the previous and of the next block
     int k;                 // vectors in the basis
     double *d, *G;         // 1/|v_i|; <v_i, v_j> / (|v_i| |v_j|), j in i's block, [i][GSB]
     double *hcol, *hs;     // Hessenberg column; h_i d_i / d_k
@@ -154,71 +159,51 @@ struct GsPass {
     int staged;
 };
 
-// NP, NQ: 8 for a full block, 0 for none, -1 for a block of fewer.  GRAM: the
-// next block holds the newest vector (its last).
+// NP, NQ: vectors of the two blocks (0: none).  GRAM: the next block holds the
+// newest vector (its last).
 template <int NP, int NQ, bool GRAM>
 __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     if (a.skip && *a.skip) return;  // an Arnoldi step enqueued ahead of a converged one
     constexpr int NW = RED_THREADS / 32;
+    constexpr int NV = NQ == 0 ? 1 : GRAM && NQ > 1 ? 16 : 8;  // sums of the pass
     __shared__ double s_red[16 * NW];
     __shared__ double s_val[16];
     extern __shared__ double s_h[];  // 3 (k + 1) values, unless they do not fit (a.staged)
     __shared__ bool s_last;
-    const int np = NP >= 0 ? NP : a.np, nq = NQ >= 0 ? NQ : a.nq;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned long long keep = l2_keep_policy();
-    double hp[NP != 0 ? GSB : 1];
-    if (NP != 0)
+    double hp[NP > 0 ? NP : 1];
 #pragma unroll
-        for (int e = 0; e < GSB; ++e) hp[e] = e < np ? a.hs[a.p0 + e] : 0.0;
-    double acc[16];
+    for (int e = 0; e < NP; ++e) hp[e] = a.hs[a.p0 + e];
+    double acc[NV];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+    for (int e = 0; e < NV; ++e) acc[e] = 0.0;
     const long long st = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < a.n2; q += st) {
         double2 x = ld_keep(a.w + q, keep);
-        double2 y[NQ != 0 ? GSB : 1];
-        if (NP != 0) {
-            double2 v[GSB];
+        double2 v[NP > 0 ? NP : 1], y[NQ > 0 ? NQ : 1];
 #pragma unroll
-            for (int e = 0; e < GSB; ++e)
-                if (e < np) v[e] = __ldcs(a.V + (long long)(a.p0 + e) * a.n2 + q);
-            if (NQ != 0)
+        for (int e = 0; e < NP; ++e) v[e] = __ldcs(a.V + (long long)(a.p0 + e) * a.n2 + q);
 #pragma unroll
-                for (int e = 0; e < GSB; ++e)
-                    if (e < nq) y[e] = __ldcs(a.V + (long long)(a.q0 + e) * a.n2 + q);
+        for (int e = 0; e < NQ; ++e) y[e] = __ldcs(a.V + (long long)(a.q0 + e) * a.n2 + q);
 #pragma unroll
-            for (int e = 0; e < GSB; ++e)
-                if (e < np) {
-                    x.x = fma(-hp[e], v[e].x, x.x);
-                    x.y = fma(-hp[e], v[e].y, x.y);
-                }
-            st_keep(a.w + q, x, keep);
-        } else {
-#pragma unroll
-            for (int e = 0; e < GSB; ++e)
-                if (e < nq) y[e] = __ldcs(a.V + (long long)(a.q0 + e) * a.n2 + q);
+        for (int e = 0; e < NP; ++e) {
+            x.x = fma(-hp[e], v[e].x, x.x);
+            x.y = fma(-hp[e], v[e].y, x.y);
         }
-        if (NQ != 0) {
-            double2 m = make_double2(0.0, 0.0);
-            if (GRAM)
+        if (NP > 0) st_keep(a.w + q, x, keep);
 #pragma unroll
-                for (int e = 0; e < GSB; ++e)
-                    if (e == nq - 1) m = y[e];
+        for (int e = 0; e < NQ; ++e) acc[e] = fma(y[e].y, x.y, fma(y[e].x, x.x, acc[e]));
+        if (NV == 16)
 #pragma unroll
-            for (int e = 0; e < GSB; ++e)
-                if (e < nq) {
-                    acc[e] = fma(y[e].y, x.y, fma(y[e].x, x.x, acc[e]));
-                    if (GRAM && e < nq - 1) acc[8 + e] = fma(y[e].y, m.y, fma(y[e].x, m.x, acc[8 + e]));
-                }
-        } else {
-            acc[0] = fma(x.y, x.y, fma(x.x, x.x, acc[0]));
-        }
+            for (int e = 0; e < NQ - 1; ++e)
+                acc[8 + e] = fma(y[e].y, y[NQ - 1].y, fma(y[e].x, y[NQ - 1].x, acc[8 + e]));
+        if (NQ == 0) acc[0] = fma(x.y, x.y, fma(x.x, x.x, acc[0]));
     }
-    const double tot = warp_reduce_scatter16(acc);  // value lane >> 1
-    if ((lane & 1) == 0) s_red[(lane >> 1) * NW + wid] = tot;
+    const double tot = warp_reduce_scatter<NV>(acc);  // value lane / (32 / NV)
+    if (lane % (32 / NV) == 0) s_red[lane / (32 / NV) * NW + wid] = tot;
     __syncthreads();
-    if (threadIdx.x < 16) {
+    if (threadIdx.x < NV) {
         double t = 0.0;
         for (int q = 0; q < NW; ++q) t += s_red[threadIdx.x * NW + q];
         a.partial[(size_t)threadIdx.x * a.max_blocks + blockIdx.x] = t;
@@ -230,8 +215,8 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     if (!s_last) return;
     // the last block: every value's partials in a fixed order, one warp per value
     __threadfence();
-    for (int v = wid; v < 16; v += NW) {
-        if (NQ == 0 ? v > 0 : (v < 8 ? v >= nq : !GRAM || v - 8 >= nq - 1)) continue;
+    for (int v = wid; v < NV; v += NW) {
+        if (NQ > 0 && (v < 8 ? v >= NQ : v - 8 >= NQ - 1)) continue;
         const double* p = a.partial + (size_t)v * a.max_blocks;
         double t = 0.0;
         for (int q = lane; q < (int)gridDim.x; q += 32) t += __ldcg(p + q);
@@ -250,14 +235,14 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     if (NQ != 0) {
         if (wid == 0) {
             const int i = a.q0 + lane;
-            const double di = lane < nq ? a.d[i] : 0.0;
-            double c = lane < nq ? di * dk * s_val[lane] : 0.0;
+            const double di = lane < NQ ? a.d[i] : 0.0;
+            double c = lane < NQ ? di * dk * s_val[lane] : 0.0;
             double grow[GSB];  // this lane's row of the block's products
 #pragma unroll
             for (int j = 0; j < GSB - 1; ++j) {
                 grow[j] = 0.0;
-                if (lane < nq && j < lane) {
-                    if (GRAM && lane == nq - 1) {
+                if (lane < NQ && j < lane) {
+                    if (GRAM && lane == NQ - 1) {
                         grow[j] = a.d[a.q0 + j] * dk * s_val[8 + j];
                         a.G[(size_t)i * GSB + j] = grow[j];
                     } else {
@@ -267,7 +252,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
             }
 #pragma unroll
             for (int j = 0; j < GSB - 1; ++j) c = fma(-grow[j], __shfl_sync(0xffffffffu, c, j), c);
-            if (lane < nq) {
+            if (lane < NQ) {
                 a.hcol[i] = c;
                 a.hs[i] = c * di / dk;
             }
@@ -442,6 +427,34 @@ int launch_dot(tbl_handle* h, const double* a, const double* b, double* out, int
     return TBL_OK;
 }
 
+// The pass that forms the dots of the last block, n vectors, and the pass that
+// takes its projections off and forms the norm.
+template <int NP>
+static void (*gs_newest(int n))(const GsPass) {
+    switch (n) {
+        case 1: return k_gs_pass<NP, 1, true>;
+        case 2: return k_gs_pass<NP, 2, true>;
+        case 3: return k_gs_pass<NP, 3, true>;
+        case 4: return k_gs_pass<NP, 4, true>;
+        case 5: return k_gs_pass<NP, 5, true>;
+        case 6: return k_gs_pass<NP, 6, true>;
+        case 7: return k_gs_pass<NP, 7, true>;
+        default: return k_gs_pass<NP, 8, true>;
+    }
+}
+static void (*gs_last(int n))(const GsPass) {
+    switch (n) {
+        case 1: return k_gs_pass<1, 0, false>;
+        case 2: return k_gs_pass<2, 0, false>;
+        case 3: return k_gs_pass<3, 0, false>;
+        case 4: return k_gs_pass<4, 0, false>;
+        case 5: return k_gs_pass<5, 0, false>;
+        case 6: return k_gs_pass<6, 0, false>;
+        case 7: return k_gs_pass<7, 0, false>;
+        default: return k_gs_pass<8, 0, false>;
+    }
+}
+
 // Orthogonalises w against the k vectors of the basis, then the Givens rotation
 // of the column.
 int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) {
@@ -468,19 +481,15 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
     const long long wave = 2LL * (h->n_sm > 0 ? h->n_sm : 148);
     if (nb > wave) nb = wave;
     const int nblk = (k + GSB - 1) / GSB, rest = k - (nblk - 1) * GSB;  // vectors of the last block
-    auto run = [&](void (*fn)(const GsPass), bool last) {
-        fn<<<(unsigned)nb, RED_THREADS, last && a.staged ? stage : 0, h->stream>>>(a);
-        h->launches++;
-    };
     for (int b = 0; b <= nblk; ++b) {
         a.p0 = (b - 1) * GSB;
-        a.np = b == 0 ? 0 : b == nblk ? rest : GSB;
         a.q0 = b * GSB;
-        a.nq = b == nblk ? 0 : b == nblk - 1 ? rest : GSB;
-        const bool gram = b == nblk - 1, full = a.nq == GSB;
-        if (b == nblk) run(a.np == GSB ? k_gs_pass<8, 0, false> : k_gs_pass<-1, 0, false>, true);
-        else if (b == 0) run(!gram ? k_gs_pass<0, 8, false> : full ? k_gs_pass<0, 8, true> : k_gs_pass<0, -1, true>, false);
-        else run(!gram ? k_gs_pass<8, 8, false> : full ? k_gs_pass<8, 8, true> : k_gs_pass<8, -1, true>, false);
+        void (*fn)(const GsPass) = b == nblk        ? gs_last(rest)
+                                   : b == nblk - 1 ? (b == 0 ? gs_newest<0>(rest) : gs_newest<GSB>(rest))
+                                   : b == 0        ? k_gs_pass<0, GSB, false>
+                                                   : k_gs_pass<GSB, GSB, false>;
+        fn<<<(unsigned)nb, RED_THREADS, b == nblk && a.staged ? stage : 0, h->stream>>>(a);
+        h->launches++;
     }
     return TBL_OK;
 }
@@ -555,7 +564,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_lsg_dots_f(long long n4, const 
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = e < 2 * G ? (double)(e % 2 == 0 ? fd[e / 2] : fg[e / 2]) : 0.0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const double tot = warp_reduce_scatter16(acc);  // value lane >> 1
+    const double tot = warp_reduce_scatter<16>(acc);  // value lane >> 1
     if ((lane & 1) == 0) s_red[(lane >> 1) * NW + wid] = tot;
     __syncthreads();
     if (threadIdx.x < 2 * G) {
