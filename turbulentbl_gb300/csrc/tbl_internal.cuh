@@ -138,8 +138,9 @@ struct tbl_handle {
     float* Vf;       // inner Krylov vectors
     float* RHf;      // inner SSOR work
     double* R64;     // FP64 outer residual
+    double* stage;   // FP64 copy of a field on its way to or from the host
     double* lsg_partial;        // low-synch Gram-Schmidt: per-block partials [2*8*groups][max_blocks]
-    double *lsg_L, *lsg_d, *lsg_g;  // (K1 x K1) strictly lower Gram matrix, Q^T w, Q^T v_new
+    double* lsg_L;   // (K1 x K1) strictly lower triangle of the basis' products
     // per-k coefficient arrays and mesh (nz)
     double *x3, *jacinv, *jac2, *Ab, *At, *Ap, *rAp;
     // recycling state

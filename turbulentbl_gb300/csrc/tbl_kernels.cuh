@@ -56,8 +56,7 @@ int launch_dot_f(tbl_handle* h, const float* a, const float* b, double* out, int
 int launch_scale_by_inv_f(tbl_handle* h, float* w, const double* denom, const int* skip = nullptr);
 int launch_backsub_update_f(tbl_handle* h, int kit);
 int launch_restart_init_k(tbl_handle* h, int first, int K1);
-int launch_givens_k(tbl_handle* h, int kit, int K1, const int* skip = nullptr, double stop_at = 0.0);
-int launch_lsg_f(tbl_handle* h, float* W, int kit, double* hcol, const int* skip = nullptr);
+int launch_lsg_f(tbl_handle* h, float* W, int kit, const int* skip, double stop_at);
 
 // tbl_api.cu
 int readback(tbl_handle* h, const void* dev, size_t bytes);

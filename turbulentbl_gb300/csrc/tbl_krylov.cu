@@ -286,25 +286,6 @@ __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double
     }
 }
 
-// The same as a kernel (mixed precision, kit <= 63); h(kit+1,kit), the norm of
-// the orthogonalised vector, is saved for the normalisation.
-__global__ void __launch_bounds__(64) k_givens(int K1, int kit, double* h, double* gg, double* gc, double* gs,
-                                               DevScalars* sc, const int* skip, double stop_at) {
-    if (skip && *skip) return;
-    __shared__ double s_h[3][64];
-    double* H = h + (size_t)K1 * (kit - 1);
-    const int i = threadIdx.x;
-    if (i <= kit) s_h[0][i] = H[i];
-    if (i < kit) {
-        s_h[1][i] = gc[i];
-        s_h[2][i] = gs[i];
-    }
-    __syncthreads();
-    if (i != 0) return;
-    sc->red[8] = s_h[0][kit];
-    givens_column(kit, s_h[0], s_h[1], s_h[2], H, gg, gc, gs, sc, skip != nullptr, stop_at);
-}
-
 // y from the triangular h (:1193-1200), one warp, a column at a time; with d
 // the coefficients of the basis vectors as they are kept, y_i / |v_i|.
 __global__ void __launch_bounds__(32) k_backsub(int K1, int kit, const double* h, double* gg, double* gy,
@@ -525,175 +506,194 @@ constexpr int LSG_G = 8;  // basis vectors per group (grid.y) of the dot pass
 __device__ __forceinline__ float dot4f(float4 a, float4 b) {
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)));
 }
-
-// d[i] = <v_i, w>, g[i] = <v_i, v_{nv-1}> for the G basis vectors of group
-// blockIdx.y (first vector g0 + G*blockIdx.y).  The products are FP32 (the
-// vectors are); each thread sums its share (about 16 float4 loads, 64
-// products) in FP32, and from these per-thread partials on every sum is FP64:
-// the warp's, the block's and k_lsg_reduce's (each value's block partials,
-// fixed order).  An FP64 sum per float4 instead cost the mixed step 14 ms at
-// 512 x 130 x 128 (22% of its Gram-Schmidt time).  (Finishing in
-// the last block -- a fence, an atomic, then the 2G sums -- cost as much as
-// the pass's loads, hence the separate reduction.)
+// The pass's share of G basis vectors: S_e = <v_e, w>, T_e = <v_e, l> with l the
+// newest basis vector, interleaved in acc.  The products are FP32 (the vectors
+// are); each thread sums its share (about 16 float4 loads, 64 products) in FP32,
+// and from these per-thread partials on every sum is FP64.  An FP64 sum per
+// float4 instead cost the mixed step 14 ms at 512 x 130 x 128 (22% of its
+// Gram-Schmidt time).
 template <int G>
-__global__ void __launch_bounds__(RED_THREADS) k_lsg_dots_f(long long n4, const float4* __restrict__ w,
-                                                            const float4* __restrict__ V, long long vstride4, int nv,
-                                                            int g0, double* __restrict__ partial, int max_blocks,
-                                                            const int* __restrict__ skip) {
-    static_assert(2 * G <= 16, "the warp reduce-scatter takes 16 values");
-    if (skip && *skip) return;
-    constexpr int NW = RED_THREADS / 32;
-    __shared__ double s_red[16 * NW];
-    const int grp = g0 / LSG_G + blockIdx.y;  // slot index of this group
-    const int i0 = g0 + blockIdx.y * G;
-    const float4* vl = V + (long long)(nv - 1) * vstride4;
+__device__ __forceinline__ void lsg_dots(long long n4, const float4* __restrict__ w, const float4* __restrict__ l,
+                                         const float4* __restrict__ V, long long vstride4, double (&acc)[16]) {
     float fd[G], fg[G];
 #pragma unroll
     for (int e = 0; e < G; ++e) { fd[e] = 0.f; fg[e] = 0.f; }
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += stride) {
-        const float4 x = w[q], l = vl[q];
+        const float4 x = w[q], y = l[q];
 #pragma unroll
         for (int e = 0; e < G; ++e) {
-            const float4 v = __ldcs(V + (long long)(i0 + e) * vstride4 + q);  // read once: evict first
+            const float4 v = __ldcs(V + (long long)e * vstride4 + q);  // read once: evict first
             fd[e] += dot4f(v, x);
-            fg[e] += dot4f(v, l);
+            fg[e] += dot4f(v, y);
         }
     }
-    double acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = e < 2 * G ? (double)(e % 2 == 0 ? fd[e / 2] : fg[e / 2]) : 0.0;
+}
+
+struct LsgArgs {
+    long long n4;
+    float4* w;
+    const float4* V;  // basis, n4 apart
+    int nv;           // its vectors
+    double* partial;  // [16 per group][max_blocks]
+    unsigned* count;
+    int max_blocks;
+    int K1;
+    double *L, *hcol;  // strictly lower triangle of the basis' products; Hessenberg column
+    double *h, *gg, *gc, *gs;
+    DevScalars* sc;
+    const int* skip;
+    double stop_at;
+};
+
+// d = Q^T w and the newest row of L, one group of LSG_G basis vectors per
+// blockIdx.y, then in the last block to finish the Hessenberg column t from
+// (I + L) t = d: the block partials of each value summed by one warp (lanes
+// strided over the blocks, four loads in flight per lane, then the shuffle
+// tree), the forward substitution by columns in one warp.  Three launches per
+// Arnoldi step (sums, solve, Givens; 30 us at 128 x 66 x 64) became the tails of
+// the two passes; L's older rows are fetched while the sums are formed.
+__global__ void __launch_bounds__(RED_THREADS) k_lsg_dots_f(const LsgArgs a) {
+    if (a.skip && *a.skip) return;
+    constexpr int NW = RED_THREADS / 32;
+    __shared__ double s_red[16 * NW];
+    __shared__ double s_d[64];
+    extern __shared__ double sL[];  // nv x nv
+    __shared__ bool s_last;
+    const int nv = a.nv, i0 = LSG_G * blockIdx.y, left = nv - i0;
+    const float4 *l = a.V + (long long)(nv - 1) * a.n4, *V = a.V + (long long)i0 * a.n4;
+    double acc[16];
+    switch (left < LSG_G ? left : LSG_G) {
+        case 1: lsg_dots<1>(a.n4, a.w, l, V, a.n4, acc); break;
+        case 2: lsg_dots<2>(a.n4, a.w, l, V, a.n4, acc); break;
+        case 3: lsg_dots<3>(a.n4, a.w, l, V, a.n4, acc); break;
+        case 4: lsg_dots<4>(a.n4, a.w, l, V, a.n4, acc); break;
+        case 5: lsg_dots<5>(a.n4, a.w, l, V, a.n4, acc); break;
+        case 6: lsg_dots<6>(a.n4, a.w, l, V, a.n4, acc); break;
+        case 7: lsg_dots<7>(a.n4, a.w, l, V, a.n4, acc); break;
+        default: lsg_dots<8>(a.n4, a.w, l, V, a.n4, acc); break;
+    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double tot = warp_reduce_scatter<16>(acc);  // value lane >> 1
     if ((lane & 1) == 0) s_red[(lane >> 1) * NW + wid] = tot;
     __syncthreads();
-    if (threadIdx.x < 2 * G) {
-        double a = 0.0;
-        for (int k = 0; k < NW; ++k) a += s_red[threadIdx.x * NW + k];
-        partial[((size_t)grp * 2 * LSG_G + threadIdx.x) * max_blocks + blockIdx.x] = a;
+    if (threadIdx.x < 16) {
+        double t = 0.0;
+        for (int k = 0; k < NW; ++k) t += s_red[threadIdx.x * NW + k];
+        a.partial[((size_t)blockIdx.y * 16 + threadIdx.x) * a.max_blocks + blockIdx.x] = t;
+        __threadfence();
     }
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(a.count, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int r = nv - 1, nb = gridDim.x;
+    for (int q = threadIdx.x; q < r * nv; q += blockDim.x)
+        if (q % nv < q / nv) sL[q] = a.L[(size_t)(q / nv) * a.K1 + q % nv];
+    for (int v = wid; v < 2 * nv; v += NW) {  // d_i for even v, the new row's <v_i, l> for odd v
+        const double* p = a.partial + (size_t)v * a.max_blocks;
+        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+        int b = lane;
+        for (; b + 96 < nb; b += 128) {
+            a0 += __ldcg(p + b);
+            a1 += __ldcg(p + b + 32);
+            a2 += __ldcg(p + b + 64);
+            a3 += __ldcg(p + b + 96);
+        }
+        for (; b < nb; b += 32) a0 += __ldcg(p + b);
+        const double t = warp_sum((a0 + a1) + (a2 + a3));
+        const int i = v >> 1;
+        if (lane == 0) {
+            if ((v & 1) == 0) s_d[i] = t;
+            else if (i < r) {
+                sL[r * nv + i] = t;
+                a.L[(size_t)r * a.K1 + i] = t;
+            }
+        }
+    }
+    __syncthreads();
+    if (wid == 0) {  // nv <= 64: each lane owns rows lane and lane + 32
+        for (int j = 0; j < nv; ++j) {
+            const double tj = s_d[j];  // final: every earlier column has been applied
+            for (int i = j + 1 + lane; i < nv; i += 32) s_d[i] -= sL[i * nv + j] * tj;
+            __syncwarp();
+        }
+        for (int i = lane; i < nv; i += 32) a.hcol[i] = s_d[i];
+    }
+    if (threadIdx.x == 0) *a.count = 0u;
 }
 
-// The 2 nv values of the dot pass: one warp per value sums its nb block
-// partials (lanes strided over the blocks, four loads in flight per lane,
-// then the shuffle tree); d[i] for even slots, g[i] (i < nv-1) for odd.
-__global__ void __launch_bounds__(256) k_lsg_reduce(const double* __restrict__ partial, int max_blocks, int nb,
-                                                    int nv, double* __restrict__ dout, double* __restrict__ gout,
-                                                    const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    const int lane = threadIdx.x & 31;
-    const int v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // value 0 .. 2 nv - 1
-    if (v >= 2 * nv) return;
-    const int grp = v / (2 * LSG_G), within = v % (2 * LSG_G);
-    const double* p = partial + ((size_t)grp * 2 * LSG_G + within) * max_blocks;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int b = lane;
-    for (; b + 96 < nb; b += 128) {
-        a0 += p[b];
-        a1 += p[b + 32];
-        a2 += p[b + 64];
-        a3 += p[b + 96];
-    }
-    for (; b < nb; b += 32) a0 += p[b];
-    const double acc = warp_sum((a0 + a1) + (a2 + a3));
-    if (lane == 0) {
-        const int i = grp * LSG_G + within / 2;
-        if (within % 2 == 0) dout[i] = acc;
-        else if (i < nv - 1) gout[i] = acc;
-    }
-}
-
-// New row of L (row nv-1: <v_{nv-1}, v_j>, j < nv-1), then (I + L) t = d by
-// column-oriented forward substitution in shared memory, one warp (nv <= 64:
-// each lane owns rows lane and lane+32).  Rows of older vectors were written
-// when each was the newest.
-__global__ void __launch_bounds__(32) k_lsg_solve(int K1, int nv, double* __restrict__ Lm,
-                                                  const double* __restrict__ d, const double* __restrict__ gnew,
-                                                  double* __restrict__ hcol, const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    __shared__ double sL[64][65];
-    __shared__ double st[64];
-    const int lane = threadIdx.x, r = nv - 1;
-    for (int j = lane; j < r; j += 32) Lm[(size_t)r * K1 + j] = gnew[j];
-    __syncwarp();
-    for (int i = 0; i < nv; ++i)
-        for (int j = lane; j < i; j += 32) sL[i][j] = i == r ? gnew[j] : Lm[(size_t)i * K1 + j];
-    for (int i = lane; i < nv; i += 32) st[i] = d[i];
-    __syncwarp();
-    for (int j = 0; j < nv; ++j) {
-        const double tj = st[j];  // final: every earlier column has been applied
-        for (int i = j + 1 + lane; i < nv; i += 32) st[i] -= sL[i][j] * tj;
-        __syncwarp();
-    }
-    for (int i = lane; i < nv; i += 32) hcol[i] = st[i];
-}
-
-// w -= sum_i t_i v_i (FP32), then ||w|| -> *out (sqrt of the deterministic sum)
-__global__ void __launch_bounds__(RED_THREADS, 6) k_lsg_update_f(long long n4, float4* __restrict__ w,
-                                                              const float4* __restrict__ V, long long vstride4, int nv,
-                                                              const double* __restrict__ t, RedWork rw, int slot,
-                                                              double* out, const int* __restrict__ skip) {
-    if (skip && *skip) return;
+// w -= sum_i t_i v_i (FP32), then in the last block ||w|| (sqrt of the
+// deterministic sum) and the column's Givens rotation
+__global__ void __launch_bounds__(RED_THREADS, 6) k_lsg_update_f(const LsgArgs a, RedWork rw, int slot) {
+    if (a.skip && *a.skip) return;
     __shared__ double s_red[RED_THREADS / 32];
     __shared__ float s_t[64];
-    for (int i = threadIdx.x; i < nv && i < 64; i += blockDim.x) s_t[i] = (float)t[i];
+    __shared__ double s_h[3][64];
+    const int nv = a.nv;
+    for (int i = threadIdx.x; i < nv && i < 64; i += blockDim.x) s_t[i] = (float)a.hcol[i];
     __syncthreads();
     double acc = 0.0;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
-        float4 x = w[q];
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < a.n4;
+         q += (long long)gridDim.x * blockDim.x) {
+        float4 x = a.w[q];
 #pragma unroll 4
         for (int i = 0; i < nv; ++i) {
-            const float4 v = __ldcs(V + (long long)i * vstride4 + q);  // read once: evict first
+            const float4 v = __ldcs(a.V + (long long)i * a.n4 + q);  // read once: evict first
             const float ti = s_t[i];
             x.x = fmaf(-ti, v.x, x.x);
             x.y = fmaf(-ti, v.y, x.y);
             x.z = fmaf(-ti, v.z, x.z);
             x.w = fmaf(-ti, v.w, x.w);
         }
-        w[q] = x;
+        a.w[q] = x;
         acc += (double)dot4f(x, x);
     }
     const double bt = block_sum(acc, s_red);
-    grid_finish(bt, rw, slot, gridDim.x, blockIdx.x, out, 1);
+    if (!grid_finish(bt, rw, slot, gridDim.x, blockIdx.x, &s_h[0][nv], 1)) return;
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+        s_h[0][i] = a.hcol[i];
+        s_h[1][i] = a.gc[i];
+        s_h[2][i] = a.gs[i];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    a.sc->red[8] = s_h[0][nv];  // the next step's matvec divides by it
+    givens_column(nv, s_h[0], s_h[1], s_h[2], a.hcol, a.gg, a.gc, a.gs, a.sc, a.skip != nullptr, a.stop_at);
 }
 
-int launch_lsg_f(tbl_handle* h, float* W, int kit, double* hcol, const int* skip) {
-    const int K1 = h->cfg.mixed_kmax + 1;
-    if (kit > 64 || kit > K1) return TBL_ERR_BAD_ARG;
+// Orthogonalises W against the kit <= 63 vectors of the FP32 basis, then the
+// Givens rotation of the column.
+int launch_lsg_f(tbl_handle* h, float* W, int kit, const int* skip, double stop_at) {
+    LsgArgs a = {};
+    a.K1 = h->cfg.mixed_kmax + 1;
+    if (kit > 63 || kit > a.K1) return TBL_ERR_BAD_ARG;
     const int nb = red_blocks(h);
-    const long long n4 = h->g.vol / 4;
-    // dot pass: full groups of 8 vectors, then the remainder group; about 16
-    // float4 per thread
-    int nbd = (int)((n4 + RED_THREADS * 16 - 1) / (RED_THREADS * 16));
+    a.n4 = h->g.vol / 4;
+    a.w = (float4*)W;
+    a.V = (const float4*)h->Vf;
+    a.nv = kit;
+    a.partial = h->lsg_partial;
+    a.count = h->red.count + 15;
+    a.max_blocks = h->red.max_blocks;
+    a.L = h->lsg_L;
+    a.hcol = h->h + (size_t)a.K1 * (kit - 1);
+    a.gg = h->gg; a.gc = h->gc; a.gs = h->gs; a.sc = h->sc;
+    a.skip = skip;
+    a.stop_at = stop_at;
+    // about 16 float4 per thread
+    int nbd = (int)((a.n4 + RED_THREADS * 16 - 1) / (RED_THREADS * 16));
     if (nbd < 1) nbd = 1;
     if (nbd > nb) nbd = nb;
-    const int nfull = kit / LSG_G, rem = kit % LSG_G;
-    const float4* Wc = (const float4*)W;
-    const float4* Vc = (const float4*)h->Vf;
-    if (nfull > 0)
-        k_lsg_dots_f<LSG_G><<<dim3(nbd, nfull), RED_THREADS, 0, h->stream>>>(n4, Wc, Vc, n4, kit, 0,
-                                                                             h->lsg_partial, h->red.max_blocks, skip);
-    if (rem > 0) {
-        const int g0 = nfull * LSG_G;
-        switch (rem) {
-#define TBL_LSG_REM(R)                                                                                              \
-    case R:                                                                                                         \
-        k_lsg_dots_f<R><<<dim3(nbd, 1), RED_THREADS, 0, h->stream>>>(n4, Wc, Vc, n4, kit, g0, h->lsg_partial,       \
-                                                                    h->red.max_blocks, skip);                      \
-        break;
-            TBL_LSG_REM(1) TBL_LSG_REM(2) TBL_LSG_REM(3) TBL_LSG_REM(4) TBL_LSG_REM(5) TBL_LSG_REM(6)
-            TBL_LSG_REM(7)
-#undef TBL_LSG_REM
-        }
-    }
-    k_lsg_reduce<<<(2 * kit + 7) / 8, 256, 0, h->stream>>>(h->lsg_partial, h->red.max_blocks, nbd, kit, h->lsg_d,
-                                                            h->lsg_g, skip);
-    k_lsg_solve<<<1, 32, 0, h->stream>>>(K1, kit, h->lsg_L, h->lsg_d, h->lsg_g, hcol, skip);  // kit <= 63
+    k_lsg_dots_f<<<dim3(nbd, (kit + LSG_G - 1) / LSG_G), RED_THREADS, (size_t)kit * kit * sizeof(double),
+                   h->stream>>>(a);
     int nbu = 6 * (h->n_sm > 0 ? h->n_sm : 148);  // one resident wave at 6 blocks per SM
     if (nbu > nb) nbu = nb;
-    k_lsg_update_f<<<nbu, RED_THREADS, 0, h->stream>>>(n4, (float4*)W, (const float4*)h->Vf, n4, kit, hcol, h->red, 7,
-                                                      &hcol[kit], skip);
-    h->launches += 3 + (nfull > 0) + (rem > 0);
+    k_lsg_update_f<<<nbu, RED_THREADS, 0, h->stream>>>(a, h->red, 7);
+    h->launches += 2;
     return TBL_OK;
 }
 
@@ -723,12 +723,6 @@ int launch_backsub_update_f(tbl_handle* h, int kit) {
 
 int launch_restart_init_k(tbl_handle* h, int first, int K1) {
     k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, nullptr);
-    h->launches++;
-    return TBL_OK;
-}
-
-int launch_givens_k(tbl_handle* h, int kit, int K1, const int* skip, double stop_at) {
-    k_givens<<<1, 64, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gc, h->gs, h->sc, skip, stop_at);
     h->launches++;
     return TBL_OK;
 }
