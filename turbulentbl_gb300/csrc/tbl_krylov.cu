@@ -671,7 +671,6 @@ int launch_lsg_f(tbl_handle* h, float* W, int kit, const int* skip, double stop_
     LsgArgs a = {};
     a.K1 = h->cfg.mixed_kmax + 1;
     if (kit > 63 || kit > a.K1) return TBL_ERR_BAD_ARG;
-    const int nb = red_blocks(h);
     a.n4 = h->g.vol / 4;
     a.w = (float4*)W;
     a.V = (const float4*)h->Vf;
@@ -684,15 +683,19 @@ int launch_lsg_f(tbl_handle* h, float* W, int kit, const int* skip, double stop_
     a.gg = h->gg; a.gc = h->gc; a.gs = h->gs; a.sc = h->sc;
     a.skip = skip;
     a.stop_at = stop_at;
-    // about 16 float4 per thread
-    int nbd = (int)((a.n4 + RED_THREADS * 16 - 1) / (RED_THREADS * 16));
-    if (nbd < 1) nbd = 1;
-    if (nbd > nb) nbd = nb;
-    k_lsg_dots_f<<<dim3(nbd, (kit + LSG_G - 1) / LSG_G), RED_THREADS, (size_t)kit * kit * sizeof(double),
+    // about 16 float4 per thread, fewer where that leaves SMs without 4 blocks
+    // (16 rounds of load latency: 56 us a Gram-Schmidt at 128 x 66 x 64)
+    const int ngr = (kit + LSG_G - 1) / LSG_G, sms = h->n_sm > 0 ? h->n_sm : 148;
+    const long long one = (a.n4 + RED_THREADS - 1) / RED_THREADS;  // one float4 per thread
+    long long nbd = (one + 15) / 16;
+    if (nbd * ngr < 4 * sms) nbd = (4 * sms + ngr - 1) / ngr;
+    if (nbd > one) nbd = one;
+    if (nbd > h->red.max_blocks) nbd = h->red.max_blocks;
+    k_lsg_dots_f<<<dim3((unsigned)nbd, ngr), RED_THREADS, (size_t)kit * kit * sizeof(double),
                    h->stream>>>(a);
-    int nbu = 6 * (h->n_sm > 0 ? h->n_sm : 148);  // one resident wave at 6 blocks per SM
-    if (nbu > nb) nbu = nb;
-    k_lsg_update_f<<<nbu, RED_THREADS, 0, h->stream>>>(a, h->red, 7);
+    long long nbu = 6LL * sms;  // one resident wave at 6 blocks per SM
+    if (nbu > one) nbu = one;
+    k_lsg_update_f<<<(unsigned)nbu, RED_THREADS, 0, h->stream>>>(a, h->red, 7);
     h->launches += 2;
     return TBL_OK;
 }
