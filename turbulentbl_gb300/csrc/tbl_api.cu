@@ -130,7 +130,7 @@ static void free_all(tbl_handle* h) {
     for (void* p : mptrs)
         if (p) cudaFree(p);
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
-                    h->uold1, h->x3, h->jacinv, h->jac2, h->Ab, h->At, h->Ap, h->rAp, h->gs_coef, h->gs_coef_f, h->lap_scale, h->coef_f, h->ssor_scale, h->ssor_scale_f, h->line_xch, h->line_ticket, h->line[0].ctas, h->line[1].ctas, h->line[2].ctas, h->usum2, h->vsum2,
+                    h->uold1, h->x3, h->jacinv, h->jac2, h->Ab, h->At, h->Ap, h->rAp, h->gs_coef, h->gs_coef_f, h->lap_scale, h->coef_f, h->ssor_scale, h->line_xch, h->line_ticket, h->line[0].ctas, h->line[1].ctas, h->line[2].ctas, h->usum2, h->vsum2,
                     h->wsum2, h->wt, h->ume1, h->bltkns, h->newk, h->ufl_file, h->ufl_live, h->ufl_full,
                     h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_G, h->gs_hs,
                     h->red.partial, h->red.count, h->halo, h->flags, h->ctas, h->slabs, h->err};
@@ -236,7 +236,6 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
     TRY(dalloc(&h->lap_scale, (size_t)nz));
     TRY(dalloc(&h->coef_f, 4 * (size_t)nz));
     TRY(dalloc(&h->ssor_scale, (size_t)nz));
-    TRY(dalloc(&h->ssor_scale_f, (size_t)nz));
     TRY(dalloc(&h->usum2, n2)); TRY(dalloc(&h->vsum2, n2)); TRY(dalloc(&h->wsum2, n2)); TRY(dalloc(&h->wt, n2));
     TRY(dalloc(&h->ume1, (size_t)nz)); TRY(dalloc(&h->bltkns, (size_t)nx)); TRY(dalloc(&h->newk, (size_t)nz));
     TRY(dalloc(&h->ufl_file, 3 * pl)); TRY(dalloc(&h->ufl_live, 3 * pl));
@@ -313,13 +312,8 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
         const double w = cfg->omega;
         const bool fold = h->line[1].S > 0 && !(cfg->flags & TBL_FLAG_RB_PRECOND);
         std::vector<double> sc(nz, 0.0);
-        std::vector<float> sf(nz, 0.0f);
-        for (int k = 0; k < nz; ++k) {
-            sc[k] = -w * rAp[k] * (fold ? -(w * ((2 - w) / w)) : 1.0);
-            sf[k] = (float)sc[k];
-        }
+        for (int k = 0; k < nz; ++k) sc[k] = -w * rAp[k] * (fold ? -(w * ((2 - w) / w)) : 1.0);
         TBL_CUDA_TRY(cudaMemcpy(h->ssor_scale, sc.data(), nz * 8, cudaMemcpyHostToDevice));
-        TBL_CUDA_TRY(cudaMemcpy(h->ssor_scale_f, sf.data(), nz * 4, cudaMemcpyHostToDevice));
     }
     // the zero fills and copies above ran on the legacy stream, which the handle's stream does not wait for
     TBL_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));

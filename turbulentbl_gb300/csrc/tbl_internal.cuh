@@ -122,8 +122,8 @@ struct tbl_handle {
     float* gs_coef_f;   // 5 x nz: the update coefficients rounded to FP32 (+ the red-black U(k-1) one)
     double* lap_scale;  // nz: -w/Ap(k), the SSOR forward scaling folded into the matvec
     float* coef_f;      // 4 x nz FP32: Ab, At, Ap, -w/Ap (FP32 matvec)
-    double* ssor_scale;   // nz: the matvec's scale before an SSOR application: lap_scale, times the backward
-    float* ssor_scale_f;  // sweep's constant w (2-w)/w where the line-scan sweeps run (FP64 and FP32)
+    double* ssor_scale; // nz: the matvec's scale before an SSOR application: lap_scale, times the backward sweep's
+                        // constant w (2-w)/w where the line-scan sweeps run
     tbl::LineShape line[3];  // line-scan sweeps per mode (GS, forward, backward)
     void* line_xch;          // their exchange between the CTAs of a column
     size_t line_xdump;       // a row of it that nobody reads

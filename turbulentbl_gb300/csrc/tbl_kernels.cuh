@@ -40,10 +40,10 @@ int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], V* halo_out, c
 template <typename V>
 int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* skip);
 
-// tbl_lap.cu: R = scale(k) L7 X by TMA plane tiles (the Arnoldi matvec)
-template <typename T>
-int launch_lap_tma(tbl_handle* h, const T* X, T* R, T aw, T as, const T* Ab, const T* At, const T* Ap, const T* scale,
-                   const int* skip, const double* denom = nullptr, T* vout = nullptr);
+// tbl_lap.cu: R = scale(k) L7 X, or scale(k) (Q8 - L7 X) with Q8
+int launch_lap(tbl_handle* h, const double* X, const double* Q8, double* R, const int* skip);
+int launch_lap_f(tbl_handle* h, const float* X, float* R, const int* skip, const double* denom, float* vout);
+int launch_lap_resid_f(tbl_handle* h, const double* X, const double* Q8, float* R, const int* skip);
 
 // tbl_krylov.cu
 int launch_dot(tbl_handle* h, const double* a, const double* b, double* out, int op);

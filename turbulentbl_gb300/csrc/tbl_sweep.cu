@@ -733,33 +733,6 @@ __global__ void __launch_bounds__(256) k_rb_ssor(Geom g, T aw, T as, const T* __
     OUT[p] = pass == 1 ? cfac * (RH[p] + sk[k] * nb) : cfac * RH[p] + sk[k] * nb;
 }
 
-// r = L7 X (Q8 == nullptr) or r = Q8 - L7 X on the interior, written to R
-// (:1001-1006 restart residual, :1098-1101 Arnoldi matvec), global halos.
-// With rAp non-null the result is multiplied by the forward sweep's
-// coefficient -w/Ap(k) (rounded to the sweep's type first, as the sweep did).
-template <typename TI, typename TO, typename TC>
-// Coefficient tables come in the arithmetic type TC (and the scale in the
-// output type TO), so an FP32 matvec does no double-to-float conversion per
-// point (those run at the FP64 rate).
-__global__ void __launch_bounds__(256) k_lap(Geom g, TC aw, TC as, const TC* __restrict__ Ab,
-                                             const TC* __restrict__ At, const TC* __restrict__ Ap,
-                                             const TI* __restrict__ X, const double* __restrict__ Q8,
-                                             TO* __restrict__ R, const TO* __restrict__ scale,
-                                             const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
-    if (i > g.nx - 2) return;
-    const long long p = (long long)i + (long long)g.sx * ((long long)j + (long long)g.ny * k);
-    const int jm = j == 1 ? g.ny - 2 : j - 1, jp = j == g.ny - 2 ? 1 : j + 1;
-    const TC xjm = (TC)X[(long long)i + (long long)g.sx * ((long long)jm + (long long)g.ny * k)];
-    const TC xjp = (TC)X[(long long)i + (long long)g.sx * ((long long)jp + (long long)g.ny * k)];
-    TC lap = aw * (TC)X[p - 1] + aw * (TC)X[p + 1] + as * xjm + as * xjp + Ab[k] * (TC)X[p - g.ps] +
-             At[k] * (TC)X[p + g.ps] + Ap[k] * (TC)X[p];
-    const TO r = (TO)(Q8 ? ((TC)Q8[p] - (lap)) : lap);
-    R[p] = scale ? scale[k] * r : r;
-}
-
 // ------------------------------------------------------ bounded-wait self-test
 // One thread waits, with the sweeps' own bounded wait, on a progress flag that
 // nothing sets; the wait gives up after SPIN_LIMIT polls and reports
@@ -1003,11 +976,8 @@ static int launch_gs_sweep_chunk(tbl_handle* h, const int* comps, int ncomp, int
 
 // Forward SSOR sweep of r = L7 X (Q8 == nullptr) or r = Q8 - L7 X.
 int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int* skip) {
-    const Geom& g = h->g;
-    const double aw = 1.0 / (h->cfg.dx * h->cfg.dx), as = 1.0 / (h->cfg.dy * h->cfg.dy);
-    k_lap<double, double, double><<<dim3((g.nx - 2 + 255) / 256, g.ny - 2, g.nz - 2), 256, 0, h->stream>>>(
-        g, aw, as, h->Ab, h->At, h->Ap, X, Q8, h->RH, h->ssor_scale, skip);
-    h->launches++;
+    const int st = launch_lap(h, X, Q8, h->RH, skip);
+    if (st != TBL_OK) return st;
     if (h->cfg.flags & TBL_FLAG_RB_PRECOND) return TBL_OK;  // the red-black passes run in launch_ssor_bwd
     if (h->line[SW_FWD].S > 0) return launch_line_ssor<double>(h, false, h->RH, h->RH, skip);
     SweepArgs<double> a = base_args<double>(h);
@@ -1046,20 +1016,8 @@ int launch_ssor_bwd(tbl_handle* h, double* out, const int* skip) {
 // which the matvec applies, writing the normalised vector to vout).
 int launch_ssor_fwd_f(tbl_handle* h, const float* Xf, const double* PCd, const double* Q8, const int* skip,
                       const double* denom, float* vout) {
-    const Geom& g = h->g;
-    dim3 grid((g.nx - 2 + 255) / 256, g.ny - 2, g.nz - 2);
-    const double aw = 1.0 / (h->cfg.dx * h->cfg.dx), as = 1.0 / (h->cfg.dy * h->cfg.dy);
-    if (PCd)
-        k_lap<double, float, double><<<grid, 256, 0, h->stream>>>(g, aw, as, h->Ab, h->At, h->Ap, PCd, Q8, h->RHf,
-                                                                  h->ssor_scale_f, skip);
-    else {  // the inner Arnoldi matvec: TMA plane tiles
-        const int s = launch_lap_tma<float>(h, Xf, h->RHf, (float)aw, (float)as, h->coef_f, h->coef_f + g.nz,
-                                            h->coef_f + 2 * (size_t)g.nz, h->ssor_scale_f, skip, denom,
-                                            vout);
-        if (s != TBL_OK) return s;
-        h->launches--;  // counted by launch_lap_tma
-    }
-    h->launches++;
+    const int st = PCd ? launch_lap_resid_f(h, PCd, Q8, h->RHf, skip) : launch_lap_f(h, Xf, h->RHf, skip, denom, vout);
+    if (st != TBL_OK) return st;
     if (h->cfg.flags & TBL_FLAG_RB_PRECOND) return TBL_OK;
     if (h->line[SW_FWD].S > 0) return launch_line_ssor<float>(h, false, h->RHf, h->RHf, skip);
     SweepArgs<float> a = base_args<float>(h);
