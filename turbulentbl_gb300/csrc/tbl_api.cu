@@ -341,16 +341,17 @@ int gs_solve(tbl_handle* h, const int* target, tbl_step_stats& st, bool zero_ok)
     double restart_at[3] = {1.0, 1.0, 1.0};
     if (mixed)
         for (int c = 0; c < 3; ++c) TRY(launch_gs_delta_init(h, c));
+    TRY(launch_gs_coef(h));
     TRY(launch_halo_init(h, parity));
-    const int nb = red_blocks(h);
+    const bool line = h->line[0].S > 0 && !(h->cfg.flags & TBL_FLAG_RB_ORDER);
     for (int it = 1; it <= mmax; ++it) {
         int comps[3], n = 0;
         for (int c = 0; c < 3; ++c)
             if (active[c]) comps[n++] = c;
         if (it % 2 == 1) {  // residual check every other sweep (:781-828)
             {
-                ProfScope ps(h, TBL_PROF_GS_RESID, 2.0 * 8.0 * h->npts * n);
-                TRY(launch_gs_resid(h, comps, n, nb > 512 ? 512 : nb));
+                ProfScope ps(h, TBL_PROF_GS_RESID, (line ? 3.0 : 2.0) * 8.0 * h->npts * n);
+                TRY(launch_gs_parts(h, comps, n, line, true));  // with what the next sweep needs
             }
             TRY(readback(h, &h->sc->red[0], 3 * sizeof(double)));
             const double* red = h->hpin;
@@ -378,6 +379,7 @@ int gs_solve(tbl_handle* h, const int* target, tbl_step_stats& st, bool zero_ok)
                 comps[m++] = c;
                 if (mixed && sumav[c] <= kRestartDrop * restart_at[c]) {
                     TRY(launch_gs_delta_restart(h, c));
+                    if (line) TRY(launch_gs_parts(h, &c, 1, true, false));
                     restart_at[c] = sumav[c];
                     restarted = true;
                 }
@@ -388,7 +390,7 @@ int gs_solve(tbl_handle* h, const int* target, tbl_step_stats& st, bool zero_ok)
         }
         {
             ProfScope ps(h, TBL_PROF_GS_SWEEP, 3.0 * 8.0 * h->npts * n);
-            TRY(launch_gs_sweep(h, comps, n, parity));
+            TRY(launch_gs_sweep(h, comps, n, parity, it % 2 == 1));
         }
         parity ^= 1;
         for (int q = 0; q < n; ++q) sweeps[comps[q]]++;

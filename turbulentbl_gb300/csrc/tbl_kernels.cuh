@@ -8,7 +8,6 @@ namespace tbl {
 int launch_save_uold(tbl_handle* h);
 int launch_inflow(tbl_handle* h);
 int launch_conv_q(tbl_handle* h);
-int launch_gs_resid(tbl_handle* h, const int* comps, int ncomp, int nblocks);
 int launch_div(tbl_handle* h);
 int launch_pc_zero_faces(tbl_handle* h);
 int launch_project_bcs(tbl_handle* h);
@@ -24,7 +23,12 @@ int launch_gs_delta_restart(tbl_handle* h, int comp);
 // tbl_sweep.cu
 int build_sweep_ctas(tbl_handle* h);
 int check_cooperative(tbl_handle* h);
-int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity);
+// tbl_gs.cu
+int launch_gs_parts(tbl_handle* h, const int* comps, int ncomp, bool pre, bool resid);
+
+// tbl_sweep.cu
+int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity, bool have_pre);
+int launch_gs_coef(tbl_handle* h);
 int launch_halo_init(tbl_handle* h, int parity);
 int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int* skip = nullptr);
 int launch_ssor_bwd(tbl_handle* h, double* out, const int* skip = nullptr);
@@ -36,7 +40,7 @@ int selftest_bounded_wait(int* observed, double* seconds);
 // tbl_line.cu: line-scan sweeps, where h->line[mode].S > 0
 int line_create(tbl_handle* h);
 template <typename V>
-int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], V* halo_out, const int* comps, int ncomp);
+int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], const int* comps, int ncomp);
 template <typename V>
 int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* skip);
 

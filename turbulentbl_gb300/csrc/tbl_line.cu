@@ -80,8 +80,6 @@ struct LineArgs {
     V* out[3];         // GS: fields; SSOR: out[0]
     const V* in[3];    // GS: precomputed old-value terms; SSOR: in[0]
     int comp[3];
-    V* halo_out;       // GS: [comp][side][slab] planes of the next sweep's halo
-    int P;
     V* xch;            // [set][plane][span row][32 E S], empty words all ones
 };
 
@@ -346,13 +344,6 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
 
         // line pointers; logical row r of the block
         V* outp = a.out[comp] + (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * k) + i0;
-        V* hout = nullptr;
-        if (GS) {
-            const size_t hb = (size_t)comp * 2 * a.P;
-            const long long hl = (long long)g.sx * (1 + jfirst) + i0;
-            if (kidx == 0 && cta.slab > 0) hout = a.halo_out + (hb + a.P + (cta.slab - 1)) * (size_t)g.ps + hl;
-            if (kidx == K - 1 && cta.slab < a.P - 1) hout = a.halo_out + (hb + (cta.slab + 1)) * (size_t)g.ps + hl;
-        }
         volatile V* const my_mail = mail + (size_t)wid * a.rows;
         const volatile V* const prev_mail = mail + (size_t)(seg > 0 ? wid - 1 : wid) * a.rows;
 
@@ -462,18 +453,15 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
             if (on) {
                 if (!GS || !edge) {
                     line_store<V, E>(outp, x, BWD);
-                    if (GS && hout) line_store<V, E>(hout, x, BWD);
                 } else {  // the faces i = 0 and nx-1 keep their boundary values
 #pragma unroll
                     for (int e = 0; e < E; ++e)
                         if (ok[e]) {
                             outp[e] = x[e];
-                            if (hout) hout[e] = x[e];
                         }
                 }
             }
             outp += rstep;
-            if (GS && hout) hout += rstep;
 #pragma unroll
             for (int e = 0; e < E; ++e) xj[e] = x[e];
             if (GS && r == 0) {
@@ -610,7 +598,6 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
     a.ticket = h->line_ticket;
     a.err = h->err;
     a.S = q.S; a.KP = q.KP; a.NC = q.NC; a.rows = q.rows;
-    a.P = h->P;
     a.Ab = h->Ab; a.At = h->At; a.rAp = h->rAp;
     a.aw = 1.0 / (h->cfg.dx * h->cfg.dx);
     a.as = 1.0 / (h->cfg.dy * h->cfg.dy);
@@ -629,13 +616,12 @@ static int line_launch(tbl_handle* h, const LineShape& q, LineArgs<V>& a, int ns
 }
 
 template <typename V>
-int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], V* halo_out, const int* comps, int ncomp) {
+int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], const int* comps, int ncomp) {
     const LineShape& q = h->line[0];
     const size_t nz = (size_t)h->g.nz;
     LineArgs<V> a = line_args<V>(h, q);
     a.gsc = sizeof(V) == 8 ? (const V*)h->gs_coef : (const V*)h->gs_coef_f;
     a.gsb = a.gsc + (sizeof(V) == 8 ? 7 : 4) * nz;
-    a.halo_out = halo_out;
     for (int c = 0; c < 3; ++c) { a.out[c] = F[c]; a.in[c] = PRE[c]; }
     for (int c = 0; c < ncomp; ++c) a.comp[c] = comps[c];
     return line_launch<0, V>(h, q, a, ncomp);
@@ -656,8 +642,8 @@ int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* sk
     return bwd ? line_launch<2, V>(h, q, a, 1) : line_launch<1, V>(h, q, a, 1);
 }
 
-template int launch_line_gs<double>(tbl_handle*, double* const[3], double* const[3], double*, const int*, int);
-template int launch_line_gs<float>(tbl_handle*, float* const[3], float* const[3], float*, const int*, int);
+template int launch_line_gs<double>(tbl_handle*, double* const[3], double* const[3], const int*, int);
+template int launch_line_gs<float>(tbl_handle*, float* const[3], float* const[3], const int*, int);
 template int launch_line_ssor<double>(tbl_handle*, bool, const double*, double*, const int*);
 template int launch_line_ssor<float>(tbl_handle*, bool, const float*, float*, const int*);
 

@@ -302,51 +302,6 @@ __global__ void __launch_bounds__(128) k_conv_q_br(Geom g, ConvCoef<double> c, c
     Q3[p] = q7 - (c.dt * g3);
 }
 
-// ---------------------------------------------------------- GS residual
-// L1 norm of the residual of (1 - dt/Re L7) U = Q over all slabs' interiors,
-// with current (global) halos (dnstbl2/dnstbl.f90:781-828).  blockIdx.y picks
-// the component from `comps`; result -> sc->red[comp].
-struct GsCoef {
-    double cE, cW, cN, cS;  // t*Av{e,w,n,s}, t = -dt/Re
-};
-
-// One block per (plane, row) at a time; the per-plane coefficients come from
-// the table k_gs_coef fills at the start of every GS solve ([d|cT|cB] at
-// 4nz..7nz, the same values as 1 + t Ap(k), t At(k), t Ab(k)).  A row's |res|
-// is summed in T, the rows in FP64.
-template <typename T>
-__global__ void __launch_bounds__(RED_THREADS) k_gs_resid(Geom g, GsCoef gc, const double* __restrict__ pc,
-                                                          const T* __restrict__ U0, const T* __restrict__ U1,
-                                                          const T* __restrict__ U2, const T* __restrict__ Q0,
-                                                          const T* __restrict__ Q1, const T* __restrict__ Q2,
-                                                          int3 comps, int ncomp, RedWork rw, DevScalars* sc) {
-    __shared__ double s_red[RED_THREADS / 32];
-    const int cid = blockIdx.y;
-    const int comp = cid == 0 ? comps.x : (cid == 1 ? comps.y : comps.z);
-    const T* F = comp == 0 ? U0 : (comp == 1 ? U1 : U2);
-    const T* Qc = comp == 0 ? Q0 : (comp == 1 ? Q1 : Q2);
-    const int J = g.ny - 2, nk = g.nz - 2, nz = g.nz;
-    const int rows = J * nk;
-    const T cE = (T)gc.cE, cW = (T)gc.cW, cN = (T)gc.cN, cS = (T)gc.cS;
-    double acc = 0.0;
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-        const int j = 1 + r % J, k = 1 + r / J;
-        const T d = (T)pc[4 * nz + k], cT = (T)pc[5 * nz + k], cB = (T)pc[6 * nz + k];
-        const long long row = idx(g, 0, j, k);
-        const long long rjp = idx(g, 0, jp1(g, j), k), rjm = idx(g, 0, jm1(g, j), k);
-        T racc = T(0);
-        for (int i = 1 + threadIdx.x; i <= g.nx - 2; i += blockDim.x) {
-            const long long p = row + i;
-            T res = Qc[p] - d * F[p] - cE * F[p + 1] - cW * F[p - 1] - cN * F[rjp + i] - cS * F[rjm + i] -
-                    cT * F[p + g.ps] - cB * F[p - g.ps];
-            racc += abs(res);
-        }
-        acc += (double)racc;
-    }
-    double bt = block_sum(acc, s_red);
-    grid_finish(bt, rw, comp, gridDim.x, blockIdx.x, &sc->red[comp], 0);
-}
-
 // ------------------------------------------------------------ divergence
 // Q8 = div(U*)/dt (dnstbl2/dnstbl.f90:905-935)
 template <typename T>
@@ -870,22 +825,6 @@ int launch_conv_q(tbl_handle* h) {
 
 // GS residual of the listed components.  In mixed precision the iteration is
 // on the increment D (delta form) with right-hand side r0 stored in Qf.
-int launch_gs_resid(tbl_handle* h, const int* comps, int ncomp, int nblocks) {
-    const Geom& g = h->g;
-    const double t = -h->cfg.dt / (h->cfg.re);
-    const double aw = 1.0 / (h->cfg.dx * h->cfg.dx), as = 1.0 / (h->cfg.dy * h->cfg.dy);
-    GsCoef gc{t * aw, t * aw, t * as, t * as};
-    int3 cs = make_int3(comps[0], ncomp > 1 ? comps[1] : 0, ncomp > 2 ? comps[2] : 0);
-    if (mixed(h))
-        k_gs_resid<float><<<dim3(nblocks, ncomp), RED_THREADS, 0, h->stream>>>(
-            g, gc, h->gs_coef, h->Df[0], h->Df[1], h->Df[2], h->Qf[0], h->Qf[1], h->Qf[2], cs, ncomp, h->red, h->sc);
-    else
-        k_gs_resid<double><<<dim3(nblocks, ncomp), RED_THREADS, 0, h->stream>>>(
-            g, gc, h->gs_coef, h->U[0], h->U[1], h->U[2], h->Q[0], h->Q[1], h->Q[2], cs, ncomp, h->red, h->sc);
-    LAUNCH_COUNT(h);
-    return TBL_OK;
-}
-
 // Mixed precision, delta form of the Gauss-Seidel solve of (I + t L7) U = Q:
 // the FP32 sweeps iterate on an increment D with right-hand side r = Q - A U.
 // In exact arithmetic U + D are the reference's iterates (a sweep is affine),

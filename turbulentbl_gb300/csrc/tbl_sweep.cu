@@ -620,17 +620,14 @@ __global__ void k_gs_coef(int nz, double t, double aw_, double as_, const double
     pcf[4 * nz + k] = (float)pc[7 * nz + k];
 }
 
-// LINE: for the line-scan sweeps, which read nothing but these terms and
-// what they produce: also the old values of the row before the first one
-// (periodic) and of the plane below a slab, and the inflow boundary value
-// itself at i = 0.
-template <typename T, bool LINE>
-__global__ void __launch_bounds__(256) k_gs_pre(Geom g, const T* __restrict__ pc, const T* __restrict__ pbv,
+// (The line-scan sweeps' terms come from tbl_gs.cu.)
+template <typename T>
+__global__ void __launch_bounds__(256) k_gs_pre(Geom g, const T* __restrict__ pc,
                                                 const int* __restrict__ slab_of_k,
                                                 const SlabDesc* __restrict__ slabs, int P, int c0_, int c1_, int c2_,
                                                 Ptr3<T> Fs, Ptr3<T> Qs, Ptr3<T> PREs,
                                                 const T* __restrict__ halo_in) {
-    const int i = (LINE ? 0 : 1) + blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int K = g.nz - 2;
     const int ci = blockIdx.z / K, k = 1 + blockIdx.z % K;
     if (i > g.nx - 2) return;
@@ -638,33 +635,19 @@ __global__ void __launch_bounds__(256) k_gs_pre(Geom g, const T* __restrict__ pc
     const T* F = Fs.p[comp];
     const int nz = g.nz;
     const T p0 = pc[k], p1 = pc[nz + k], p2 = pc[2 * nz + k], p3 = pc[3 * nz + k];
-    const T pb = LINE ? pbv[k] : T(0);
     const int r = slab_of_k[k];
     const SlabDesc sl = slabs[r];
     const bool halo = k == sl.bn + sl.K - 1 && r < P - 1;
-    const bool below = LINE && k == sl.bn;
     for (int jr = 0; jr < ROWS_PER_BLOCK; ++jr) {  // a few rows per block: fewer, longer blocks
         const int j = 1 + blockIdx.y * ROWS_PER_BLOCK + jr;
         if (j > g.ny - 2) break;
         const long long line = (long long)g.sx * ((long long)j + (long long)g.ny * k);
-        T* out = const_cast<T*>(PREs.p[comp]) + line + i;
-        if (LINE && i == 0) {
-            *out = F[line];
-            continue;
-        }
         const int jp = (j == g.ny - 2) ? 1 : j + 1;
         const T* Fkp = halo ? halo_in + ((size_t)comp * 2 * P + 1 * P + r) * (size_t)g.ps + (size_t)g.sx * j
                             : F + line + g.ps;
         T x = fma(p1, F[line + i + 1], p0 * Qs.p[comp][line + i]);
         if (jp != 1) x = fma(p2, F[(long long)g.sx * ((long long)jp + (long long)g.ny * k) + i], x);
-        x = fma(p3, Fkp[i], x);
-        if (LINE && j == 1) x = fma(p2, F[(long long)g.sx * ((long long)(g.ny - 2) + (long long)g.ny * k) + i], x);
-        if (below) {
-            const T* Fkm = r > 0 ? halo_in + ((size_t)comp * 2 * P + r) * (size_t)g.ps + (size_t)g.sx * j
-                                 : F + line - g.ps;
-            x = fma(pb, Fkm[i], x);
-        }
-        *out = x;
+        const_cast<T*>(PREs.p[comp])[line + i] = fma(p3, Fkp[i], x);
     }
 }
 
@@ -908,16 +891,12 @@ static int gs_pre_and_sweep(tbl_handle* h, T* const F[3], const T* const Q[3], T
     const Geom& g = h->g;
     Ptr3<T> Fs, Qs, Ps;
     for (int c = 0; c < 3; ++c) { Fs.p[c] = F[c]; Qs.p[c] = Q[c]; Ps.p[c] = PRE[c]; }
+    dim3 grid((g.nx - 2 + 255) / 256, (g.ny - 2 + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, (g.nz - 2) * ncomp);
     const T* pc = sizeof(T) == 8 ? (const T*)h->gs_coef : (const T*)h->gs_coef_f;
-    const T* pb = pc + (sizeof(T) == 8 ? 7 : 4) * (size_t)g.nz;
-    const bool line = h->line[SW_GS].S > 0;
-    dim3 grid((g.nx - 2 + (line ? 1 : 0) + 255) / 256, (g.ny - 2 + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK,
-              (g.nz - 2) * ncomp);
-    (line ? k_gs_pre<T, true> : k_gs_pre<T, false>)<<<grid, 256, 0, h->stream>>>(
-        g, pc, pb, h->slab_of_k, h->slabs, h->P, comps[0], ncomp > 1 ? comps[1] : 0, ncomp > 2 ? comps[2] : 0, Fs, Qs,
-        Ps, a.halo_in);
+    k_gs_pre<T><<<grid, 256, 0, h->stream>>>(g, pc, h->slab_of_k, h->slabs, h->P,
+                                             comps[0], ncomp > 1 ? comps[1] : 0, ncomp > 2 ? comps[2] : 0, Fs, Qs,
+                                             Ps, a.halo_in);
     h->launches++;
-    if (line) return launch_line_gs<T>(h, F, PRE, a.halo_out, comps, ncomp);
     return launch_sweep<SW_GS, T>(h, a, ncomp);
 }
 
@@ -940,7 +919,7 @@ static int rb_gs(tbl_handle* h, T* const F[3], const T* const Q[3], const T* pc,
     return TBL_OK;
 }
 
-int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity) {
+int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity, bool have_pre) {
     if (h->cfg.flags & TBL_FLAG_RB_ORDER) {
         const int nz = h->g.nz;
         if (h->cfg.precision == TBL_PREC_MIXED) {
@@ -952,7 +931,17 @@ int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity) {
         const double* Q[3] = {h->Q[0], h->Q[1], h->Q[2]};
         return rb_gs<double>(h, F, Q, h->gs_coef, h->gs_coef + 7 * (size_t)nz, comps, ncomp);
     }
-    const int per = h->line[SW_GS].S > 0 ? 3 : h->gs_comps_per_launch > 0 ? h->gs_comps_per_launch : 1;
+    if (h->line[SW_GS].S > 0) {
+        const int s = have_pre ? TBL_OK : launch_gs_parts(h, comps, ncomp, true, false);
+        if (s != TBL_OK) return s;
+        if (h->cfg.precision == TBL_PREC_MIXED) {
+            float* P[3] = {h->PREf, h->PREf + h->g.vol, h->PREf + 2 * h->g.vol};
+            return launch_line_gs<float>(h, h->Df, P, comps, ncomp);
+        }
+        double* P[3] = {h->PRE, h->PRE + h->g.vol, h->PRE + 2 * h->g.vol};
+        return launch_line_gs<double>(h, h->U, P, comps, ncomp);
+    }
+    const int per = h->gs_comps_per_launch > 0 ? h->gs_comps_per_launch : 1;
     for (int c0 = 0; c0 < ncomp; c0 += per) {
         const int n = ncomp - c0 < per ? ncomp - c0 : per;
         const int s = launch_gs_sweep_chunk(h, comps + c0, n, parity);
@@ -1058,14 +1047,22 @@ __global__ void k_halo_init(Geom g, const SlabDesc* __restrict__ slabs, int P, c
         dst[q] = src[q];
 }
 
-int launch_halo_init(tbl_handle* h, int parity) {
-    const size_t hsz = (size_t)3 * 2 * h->P * h->g.ps;
-    // per-plane GS coefficients of the operator in use (the adjoint swaps in A^T)
+// Start of a Gauss-Seidel solve: the per-plane coefficients of the operator in
+// use (the adjoint swaps in A^T).
+int launch_gs_coef(tbl_handle* h) {
     k_gs_coef<<<(h->g.nz + 127) / 128, 128, 0, h->stream>>>(h->g.nz, -h->cfg.dt / (h->cfg.re),
                                                              1.0 / (h->cfg.dx * h->cfg.dx),
                                                              1.0 / (h->cfg.dy * h->cfg.dy), h->Ap, h->At, h->Ab,
                                                              h->gs_coef, h->gs_coef_f);
     h->launches++;
+    return TBL_OK;
+}
+
+// The wavefront sweeps' halo planes (the other sweeps run while no slab's
+// neighbours change, and read them in place).
+int launch_halo_init(tbl_handle* h, int parity) {
+    if (h->line[SW_GS].S > 0 || (h->cfg.flags & TBL_FLAG_RB_ORDER)) return TBL_OK;
+    const size_t hsz = (size_t)3 * 2 * h->P * h->g.ps;
     if (h->cfg.precision == TBL_PREC_MIXED)
         k_halo_init<float><<<dim3(32, 3 * 2 * h->P), 256, 0, h->stream>>>(
             h->g, h->slabs, h->P, h->Df[0], h->Df[1], h->Df[2], reinterpret_cast<float*>(h->halo) + (size_t)(parity & 1) * hsz);
