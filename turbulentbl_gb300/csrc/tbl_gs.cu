@@ -188,9 +188,10 @@ static int gs_parts(tbl_handle* h, T* const U[3], T* const Q[3], T* const PRE[3]
     const Geom& g = h->g;
     const int vec = 16 / (int)sizeof(T), planes = g.nz - 2;
     const int gx = (g.nx - 2) / (32 * vec) + 1, gy = (g.ny - 2 + GS_ROWS - 1) / GS_ROWS;
-    // planes per tile: about 8 blocks per SM over the components, one plane at least
+    // planes per tile: about 8 blocks per SM over the components (16 in FP64: 16.8
+    // against 17.5 ms of checks a step at 512 x 130 x 128), one plane at least
     const long long sms = h->n_sm > 0 ? h->n_sm : 148, tiles = (long long)gx * gy * ncomp;
-    const long long want = (8 * sms + tiles - 1) / tiles;
+    const long long want = ((sizeof(T) == 8 ? 16 : 8) * sms + tiles - 1) / tiles;
     const int kc = (int)std::min((long long)GS_KC, (planes + want - 1) / want), gz = (planes + kc - 1) / kc;
     const long long nb = std::min((long long)gx * gy * gz, (long long)h->red.max_blocks);
     const double t = -h->cfg.dt / (h->cfg.re);

@@ -100,8 +100,8 @@ template <> struct LineBits<float> {
 // high word are stored as another NaN.
 template <typename V>
 __device__ __forceinline__ bool line_empty(V v) { return LineBits<V>::hi(v) == 0xffffffffu; }
-template <typename V>
-__device__ __forceinline__ V line_value(V v) { return line_empty(v) ? LineBits<V>::nan() : v; }
+__device__ __forceinline__ double line_value(double v) { return line_empty(v) ? LineBits<double>::nan() : v; }
+__device__ __forceinline__ float line_value(float v) { return v; }  // FP32 arithmetic gives one NaN, 0x7fffffff
 
 // E values of the exchange buffer; each value is read and written whole.
 __device__ __forceinline__ void xch_ld(double (&v)[1], const double* p) {
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
             ok[e] = on && i >= 1 && i <= g.nx - 2;
             all_ok = all_ok && ok[e];
         }
-        const bool edge = __any_sync(ALL, !all_ok);  // the warp holds a line end
+        const bool whole = all_ok, edge = __any_sync(ALL, !all_ok);  // the warp holds a line end
         // chunks before this one in its streamwise block
         int dist = ch;
         if (!GS && a.cb > 0) dist = BWD ? min(C, (pc / a.cb + 1) * a.cb) - 1 - pc : pc % a.cb;
@@ -374,12 +374,12 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
             take(rdy ? s : (s ^ 1), o);  // the address waits for the test
             return rdy;
         };
-        auto get = [&](int s, unsigned ph, V(&o)[E]) -> bool {
-            bool got = !below || mbar_wait(&full[s], ph);
-            if ((s & (H - 1)) == 0) got = mbar_wait(&opfull[s / H], ph) && got;
-            if (!__all_sync(ALL, got)) return false;
+        bool dead = false;  // a wait gave up: nothing waits any more, and the results mean nothing
+        auto get = [&](int s, unsigned ph, V(&o)[E]) {
+            bool got = dead || !below || mbar_wait(&full[s], ph);
+            if ((s & (H - 1)) == 0) got = (dead || mbar_wait(&opfull[s / H], ph)) && got;
+            if (!__all_sync(ALL, got)) dead = true;
             take(s, o);
-            return true;
         };
         // The H rows up to q have been read: their slots are handed back to the
         // plane below and fetch the operands of the rows XR later.
@@ -395,7 +395,9 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
         // One row: gr holds its right-hand side and the plane below's share.
         // What the next row needs from the plane below is looked at while this
         // row's scan runs, and waited for only after this row has been handed on.
-        auto row = [&](const int r, const int u, const unsigned ph) -> bool {
+        // (Every branch and every instruction of a row counts: the chain of rows
+        // is one warp's issue.)
+        auto row = [&](const int r, const int u, const unsigned ph) {
             V x[E];
 #pragma unroll
             for (int e = 0; e < E; ++e) x[e] = fma(cj, xj[e], gr[e]);
@@ -408,9 +410,15 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
 #pragma unroll
             for (int e = 1; e < E; ++e) x[e] = fma(ci, x[e - 1], x[e]);
             V b = x[E - 1];
-#pragma unroll
-            for (int l = 0; l < 5; ++l)
-                if (l < nlev) b = fma(lev[l], __shfl_up_sync(ALL, b, 1 << l), b);
+            b = fma(lev[0], __shfl_up_sync(ALL, b, 1), b);
+            b = fma(lev[1], __shfl_up_sync(ALL, b, 2), b);
+            if (nlev > 2) {
+                b = fma(lev[2], __shfl_up_sync(ALL, b, 4), b);
+                if (nlev > 3) {
+                    b = fma(lev[3], __shfl_up_sync(ALL, b, 8), b);
+                    if (nlev > 4) b = fma(lev[4], __shfl_up_sync(ALL, b, 16), b);
+                }
+            }
             const bool more = r + 1 < nrow;
             const int s1 = (u + 1) % XR;
             const unsigned ph1 = u + 1 == XR ? ph ^ 1u : ph;
@@ -418,8 +426,8 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
             // the carry of the segment before
             if (seg > 0) {
                 long long spins = 0;
-                while (__any_sync(ALL, line_empty(c))) {
-                    if (++spins > SPIN_LIMIT) return false;
+                while (__any_sync(ALL, line_empty(c)) && !dead) {
+                    if (++spins > SPIN_LIMIT) dead = true;
                     c = prev_mail[r];
                 }
                 b = fma(acar, c, b);
@@ -431,15 +439,14 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
 #pragma unroll
             for (int e = 0; e < E - 1; ++e) x[e] = fma(cpw[e], y, x[e]);
             x[E - 1] = b;
-            if (edge) {
-#pragma unroll
-                for (int e = 0; e < E; ++e) x[e] = ok[e] ? x[e] : V(0);
-            }
+            // GS: the boundary value at i = 0 enters the line only.  The other points
+            // outside 1..nx-2 are zero (BWD) or come after the line's last.
+            if (GS && ch == 0) x[0] = V(0);
             // hand the row to the plane above, then to global memory
             if (to_ring) {
-                if ((u & (H - 1)) == 0 && r >= XR &&
+                if ((u & (H - 1)) == 0 && r >= XR && !dead &&
                     !__all_sync(ALL, mbar_wait(&up_full[XR + u / H], ph ^ 1u)))
-                    return false;
+                    dead = true;
                 line_store<V, E>(up_ring + u * 64 * E, x, false);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&up_full[u]);
@@ -450,37 +457,31 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
                 xch_put(xout, w);
                 xout += xrow;
             }
-            if (on) {
-                if (!GS || !edge) {
-                    line_store<V, E>(outp, x, BWD);
-                } else {  // the faces i = 0 and nx-1 keep their boundary values
+            if (whole) line_store<V, E>(outp, x, BWD);
+            if (E > 1 && edge) {  // a line end in the chunk: the points outside keep their values
 #pragma unroll
-                    for (int e = 0; e < E; ++e)
-                        if (ok[e]) {
-                            outp[e] = x[e];
-                        }
-                }
+                for (int e = 0; e < E; ++e)
+                    if (!whole && ok[e]) outp[BWD ? E - 1 - e : e] = x[e];
             }
             outp += rstep;
 #pragma unroll
             for (int e = 0; e < E; ++e) xj[e] = x[e];
-            if (GS && r == 0) {
+            if (GS && u == 0 && r == 0) {
 #pragma unroll
                 for (int e = 0; e < E; ++e) x0[GS ? e : 0] = x[e];
             }
-            if (!rdy && !get(s1, ph1, gr)) return false;
+            if (!rdy) get(s1, ph1, gr);
             if (more) done(r + 1, s1);
-            return true;
         };
-        bool good = get(0, 0u, gr);
+        get(0, 0u, gr);
         unsigned ph = 0;
-        for (int r0 = 0; r0 < nrow && good; r0 += XR, ph ^= 1u) {
+        for (int r0 = 0; r0 < nrow; r0 += XR, ph ^= 1u) {
 #pragma unroll
             for (int u = 0; u < XR; ++u)
-                if (good && r0 + u < nrow) good = row(r0 + u, u, ph);
+                if (r0 + u < nrow) row(r0 + u, u, ph);
         }
         // (a warp that gave up has waited for a second: its own fetches have landed)
-        if (!good && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
+        if (dead && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
         __syncwarp();
     }
     __syncthreads();  // the last CTA to finish leaves the tickets as it found them
