@@ -402,6 +402,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
 #pragma unroll
             for (int e = 0; e < E; ++e) x[e] = fma(cj, xj[e], gr[e]);
             if (GS && r == nrow - 1) {  // periodic: the last row reads the first row's new values
+                __syncwarp();           // (a branch: predicated FMAs would cost FP64 issue in every row)
 #pragma unroll
                 for (int e = 0; e < E; ++e) x[e] = fma(cj, x0[GS ? e : 0], x[e]);
             }
