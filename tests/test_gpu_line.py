@@ -1,8 +1,8 @@
 """The line-scan sweeps (tbl_line.cu) against the oracle where their split of
 a grid changes: one and several warps per line (a partial chunk, a last warp
-of one lane), 1, 2 and 4 points per lane, rows that fill the rings' halves
+of one lane), 1, 2, 4 and 8 points per lane, rows that fill the rings' halves
 exactly or leave a remainder, slabs of many and of few planes (one and several
-planes per CTA, an incomplete last CTA)."""
+planes per CTA, an incomplete last CTA, as many planes as registers allow)."""
 import numpy as np
 import pytest
 
@@ -19,7 +19,8 @@ def rel(a, b):
 
 @pytest.mark.parametrize("precision", [abi.TBL_PREC_FP64, abi.TBL_PREC_MIXED])
 @pytest.mark.parametrize("nx,nzs,nyw,P", [(34, 8, 14, 2), (35, 9, 30, 1), (130, 4, 18, 3), (131, 5, 17, 2),
-                                          (133, 16, 12, 1), (258, 13, 27, 4), (300, 7, 60, 8)])
+                                          (133, 16, 12, 1), (258, 13, 27, 4), (300, 7, 60, 8),
+                                          (390, 8, 110, 1), (40, 12, 110, 2), (520, 9, 13, 2), (1030, 6, 11, 1)])
 def test_steps_match_the_oracle(nx, nzs, nyw, P, precision):
     """Tolerances of the FP64 parity tests (1e-12) and of the mixed ones
     (1e-5, 1e-4 for p): the scan changes rounding only."""

@@ -46,6 +46,7 @@
 // prefetch of the operands was slower too (their loads share scoreboards with
 // the shuffles: every row waited for them).
 #include <algorithm>
+#include <climits>
 
 #include "tbl_internal.cuh"
 #include "tbl_kernels.cuh"
@@ -57,7 +58,7 @@ constexpr int LINE_XR = 8;           // ring slots (rows) per warp, in two halve
 // sweeping warps of a CTA at most, so that the registers of E points per lane fit
 constexpr int line_max_warps(int E) { return E >= 4 ? 12 : 16; }
 constexpr int LINE_MAX_COURIERS = 4;
-constexpr int LINE_MAX_SMEM = 200 * 1024;
+constexpr int LINE_MAX_SMEM = 222 * 1024;
 // mbarriers per warp: the plane below's row is in a slot; a half of the slots
 // has been read; a half's operands have landed
 constexpr int LINE_BARS = LINE_XR + 4;
@@ -123,6 +124,10 @@ __device__ __forceinline__ void xch_ld(float (&v)[4], const float* p) {
                  : "l"(p)
                  : "memory");
 }
+__device__ __forceinline__ void xch_ld(float (&v)[8], const float* p) {
+    xch_ld(reinterpret_cast<float(&)[4]>(v[0]), p);
+    xch_ld(reinterpret_cast<float(&)[4]>(v[4]), p + 4);
+}
 __device__ __forceinline__ void xch_put(double* p, const double (&v)[1]) {
     asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v[0]) : "memory");
 }
@@ -140,6 +145,10 @@ __device__ __forceinline__ void xch_put(float* p, const float (&v)[4]) {
     asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
                  "f"(v[3])
                  : "memory");
+}
+__device__ __forceinline__ void xch_put(float* p, const float (&v)[8]) {
+    xch_put(p, reinterpret_cast<const float(&)[4]>(v[0]));
+    xch_put(p + 4, reinterpret_cast<const float(&)[4]>(v[4]));
 }
 template <int E, typename V>
 __device__ __forceinline__ bool xch_row(V (&w)[E], const V* p) {
@@ -493,16 +502,17 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
 }
 
 // ------------------------------------------------------------------ host
-// Kernels by points per lane: 1, 2, 4 in FP64, 2, 4 in FP32.
+// Kernels by points per lane: 1, 2, 4 in FP64, 4, 8 in FP32.
 template <int MODE, typename V>
 static void (*line_fn(int E))(const LineArgs<V>) {
-    if constexpr (sizeof(V) == 8)
-        if (E == 1) return k_line<MODE, V, 1>;
-    return E == 2 ? k_line<MODE, V, 2> : k_line<MODE, V, 4>;
+    if constexpr (sizeof(V) == 8) return E == 1 ? k_line<MODE, V, 1> : E == 2 ? k_line<MODE, V, 2> : k_line<MODE, V, 4>;
+    else return E == 4 ? k_line<MODE, V, 4> : k_line<MODE, V, 8>;
 }
 template <typename V>
 static int line_chunks_of(int E, int nx) {
-    return E == 1 ? line_chunks<V, 1>(nx) : E == 2 ? line_chunks<V, 2>(nx) : line_chunks<V, 4>(nx);
+    if constexpr (sizeof(V) == 8)
+        return E == 1 ? line_chunks<V, 1>(nx) : E == 2 ? line_chunks<V, 2>(nx) : line_chunks<V, 4>(nx);
+    else return E == 4 ? line_chunks<V, 4>(nx) : line_chunks<V, 8>(nx);
 }
 
 // Splits the slab columns over CTAs of KP planes for one kernel.  False when
@@ -518,9 +528,10 @@ static bool line_plan(const tbl_handle* h, int rows, int nblk, int E, int kp, Li
     q.NC = std::min(q.S, LINE_MAX_COURIERS);
     q.rows = rows;
     q.nblk = nblk;
-    const size_t nw = (size_t)q.S * q.KP;
-    q.smem = nw * (LINE_XR * 64 * E * sizeof(V) + LINE_BARS * 8 + rows * sizeof(V));
-    if (q.smem > LINE_MAX_SMEM) return false;
+    const size_t plane = q.S * (LINE_XR * 64 * E * sizeof(V) + LINE_BARS * 8 + rows * sizeof(V));
+    q.KP = std::min(q.KP, (int)(LINE_MAX_SMEM / plane));
+    if (q.KP < 1) return false;
+    q.smem = q.KP * plane;
     for (int r = 0; r < h->P; ++r) q.ncta += (h->en[r] - h->bn[r] + 1 + q.KP - 1) / q.KP * nblk;
     if (cudaFuncSetAttribute((const void*)line_fn<MODE, V>(E), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              LINE_MAX_SMEM) != cudaSuccess) {
@@ -528,6 +539,32 @@ static bool line_plan(const tbl_handle* h, int rows, int nblk, int E, int kp, Li
         return false;
     }
     return true;
+}
+
+// A Gauss-Seidel launch sweeps three components at once, so its CTAs are
+// counted in waves of one per SM: a second CTA on an SM shares its FP64 pipes
+// or waits for its registers, and starts its chain late.  The plan takes the
+// fewest waves, and of those the fewest points per lane and then planes per
+// CTA.  FP64, E, KP = 2, 2 / 2, 3 / 4, 2 / 4, 3, us: 124 / 138 / 157 / 160 at
+// 256 x 98 x 96 (one wave each); 195 / 163 / 204 / 191 at 256 x 130 x 128 and
+// 363 / - / 342 / 293 at 512 x 130 x 128 (two, one, two, one).  FP32, 4, 2 /
+// 4, 3 / 8, 3 / 8, 4: 111 / 98 / 101 / 103 at 512 x 130 x 128 (two, one, one,
+// one), 119 / 131 / 116 / 99 at 512 x 102 x 190 (two, two, two, one), and from
+// two planes to three or four the hand-overs saved weigh as much.
+template <typename V>
+static bool line_plan_gs(const tbl_handle* h, int rows, int E0, LineShape& q) {
+    int best = INT_MAX;
+    for (int E = E0; E <= (sizeof(V) == 8 ? 4 : 8); E *= 2)
+        for (int kp = sizeof(V) == 8 ? 2 : 3; kp <= 4; ++kp) {
+            LineShape t;
+            if (!line_plan<0, V>(h, rows, 1, E, kp, t)) continue;
+            const int waves = (3 * t.ncta + h->n_sm - 1) / h->n_sm;
+            if (waves < best) {
+                best = waves;
+                q = t;
+            }
+        }
+    return best < INT_MAX;
 }
 
 // The CTAs of a launch, the lowest of every column first.
@@ -547,29 +584,27 @@ static int line_init(tbl_handle* h) {
     const int J = h->g.ny - 2, nx = h->g.nx;
     const bool span = (h->cfg.flags & TBL_FLAG_SSOR_SPAN_BLOCKS) != 0;
     const int brows = span ? std::min(32, J) : J, nblk = span ? (J + 31) / 32 : 1;
-    // Points per lane and planes per CTA.  An FP64 row costs about 65 cycles
-    // per FMA a warp issues: few points per lane spread a line over more of the
-    // SM's four FP64 pipes, but every warp pays for the scan.  SSOR sweep at
-    // E = 1 / 2 / 4: 62 / 70 / 94 us at 128 x 66 x 64, 84 / 84 / 107 at
-    // 201 x 77 x 59, 263 / 185 / 198 at 512 x 130 x 128.  Where the three
-    // components of a GS sweep have more than two CTAs per SM the FP64 pipes
-    // are the bound and the fewest FMAs per point win (512 x 130 x 128: 770 /
-    // 510 / 450 us; 128 x 66 x 64, one CTA per SM: 68 / 82 / 114).  FP32 rows
-    // are bound by latency: 4 points, and 2 planes per CTA shorten the hand-over
-    // (SSOR at 512: 108 / 100 / 104 us with 1 / 2 / 3; GS 204 / 188 / 134).
-    int E[2] = {4, 4}, kp[2] = {3, 2};  // GS, SSOR
+    // SSOR: points per lane and planes per CTA.  An FP64 row costs about 65
+    // cycles per FMA that a warp issues, so few points per lane spread a line
+    // over more of the SM's four FP64 pipes, but every warp pays for the scan.
+    // E = 1 / 2 / 4: 66 / 74 / 94 us at 128 x 66 x 64, 79 / 74 / 94 at
+    // 201 x 77 x 59, 300 / 207 / 214 at 512 x 130 x 128; 244 / 218 (E = 2 / 4)
+    // at 700 x 102 x 100.  FP32 rows are bound by latency: 4 points, and two
+    // planes per CTA save a hand-over (84 / 84 / 88 us with 1 / 2 / 3 at 512);
+    // from five warps a line on, the registers leave one CTA per SM and 8
+    // points are better (4 / 8 points: 198 / 139 at 768 x 194 x 144, 135 / 108
+    // at 600 x 130 x 128, 84 / 89 at 512).
+    int E, kp;
     if (sizeof(V) == 8) {
-        E[1] = nx <= 130 ? 1 : 2;
-        E[0] = 3 * (h->g.nz - 2) > 2 * h->n_sm ? 4 : E[1];
-        kp[0] = E[0] == 4 ? 2 : 1;
-        kp[1] = 1;
-        for (int& e : E)
-            while (e < 4 && (line_chunks_of<V>(e, nx) + 31) / 32 > line_max_warps(e)) e *= 2;
+        E = nx <= 130 ? 1 : nx <= 513 ? 2 : 4;
+        kp = 1;
+    } else {
+        E = nx <= 513 ? 4 : 8;
+        kp = 2;
     }
     LineShape q[3];
-    const bool gs = line_plan<0, V>(h, J, 1, E[0], kp[0], q[0]);
-    const bool ssor = line_plan<1, V>(h, brows, nblk, E[1], kp[1], q[1]) &&
-                      line_plan<2, V>(h, brows, nblk, E[1], kp[1], q[2]);
+    const bool ssor = line_plan<1, V>(h, brows, nblk, E, kp, q[1]) && line_plan<2, V>(h, brows, nblk, E, kp, q[2]);
+    const bool gs = line_plan_gs<V>(h, J, E, q[0]);
     size_t words = 0;
     for (int m = 0; m < 3; ++m) {
         if (m == 0 ? !gs : !ssor) continue;
