@@ -132,7 +132,7 @@ static void free_all(tbl_handle* h) {
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
                     h->uold1, h->x3, h->jacinv, h->jac2, h->Ab, h->At, h->Ap, h->rAp, h->gs_coef, h->gs_coef_f, h->lap_scale, h->coef_f, h->ssor_scale, h->line_xch, h->line_ticket, h->line[0].ctas, h->line[1].ctas, h->line[2].ctas, h->usum2, h->vsum2,
                     h->wsum2, h->wt, h->ume1, h->bltkns, h->newk, h->ufl_file, h->ufl_live, h->ufl_full,
-                    h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_G, h->gs_hs,
+                    h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_nd, h->gs_G, h->gs_hs,
                     h->red.partial, h->red.count, h->halo, h->flags, h->ctas, h->slabs, h->err};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -223,7 +223,7 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
         for (int c = 0; c < 3; ++c) { TRY(dalloc(&h->U[c], vol)); TRY(dalloc(&h->Q[c], vol)); }
         TRY(dalloc(&h->Pr, vol)); TRY(dalloc(&h->RH, vol)); TRY(dalloc(&h->PRE, 3 * vol));
         TRY(dalloc(&h->V, vol * (size_t)(cfg->kmax + 1)));
-        TRY(dalloc(&h->gs_d, (size_t)cfg->kmax + 1));
+        TRY(dalloc(&h->gs_d, (size_t)cfg->kmax + 1)); TRY(dalloc(&h->gs_nd, (size_t)cfg->kmax + 1));
         TRY(dalloc(&h->gs_G, 8 * ((size_t)cfg->kmax + 1)));
         TRY(dalloc(&h->gs_hs, (size_t)cfg->kmax + 1));
     }
@@ -249,7 +249,7 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
     TRY(dalloc(&h->gs, (size_t)K1)); TRY(dalloc(&h->gy, (size_t)K1));
     h->red.max_blocks = 2048;
     TRY(dalloc(&h->red.partial, (size_t)16 * h->red.max_blocks));
-    TRY(dalloc(&h->red.count, (size_t)16));
+    TRY(dalloc(&h->red.count, (size_t)24));
     TRY(dalloc(&h->halo, (size_t)2 * 3 * 2 * h->P * g.ps));
     TRY(dalloc(&h->err, 1));
     // mesh and per-k coefficients (:487-536); An* == Av*

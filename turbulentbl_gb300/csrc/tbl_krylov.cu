@@ -82,44 +82,103 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&a)[N]) {
     return a[0];
 }
 
-// Givens rotations for column kit (1-based) (:1165-1189) by one thread.  h2:
-// the column, kit + 1 values, c2, s2: the rotations so far; staged in shared
-// memory, so that the chain of kit rotations does not wait for global loads.
-// H: the column in global memory (h2 may be H itself).  With ahead (Arnoldi
-// steps enqueued ahead) the cycle stops when the estimate sumav reaches stop_at
-// (the host's loop test, evaluated on the same double).
-__device__ __forceinline__ void givens_column(int kit, const double* h2, const double* c2, const double* s2, double* H,
-                                              double* gg, double* gc, double* gs, DevScalars* sc, bool ahead,
-                                              double stop_at) {
-    double cur = h2[0];
-    for (int i = 0; i < kit - 1; ++i) {
-        const double nx = h2[i + 1];
-        H[i] = c2[i] * cur - s2[i] * nx;
-        cur = s2[i] * cur + c2[i] * nx;
+// The last block to publish its partials, known to all its threads; what the
+// blocks wrote before is visible to it.
+__device__ __forceinline__ bool last_arrival(unsigned* count, unsigned total, bool* s_last) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned t;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(count) : "memory");
+        *s_last = t == total - 1;
     }
-    const double last = h2[kit];
-    double diag = cur, sub = last;
-    const double nu = sqrt(cur * cur + last * last);
-    double gk = gg[kit - 1], gkp = gg[kit];
-    if (nu > 0.0) {
-        const double c = cur / nu, s = -last / nu;
-        gc[kit - 1] = c;
-        gs[kit - 1] = s;
-        diag = c * cur - s * last;
-        sub = 0.0;
-        const double a = c * gk - s * gkp, b = s * gk + c * gkp;
-        gk = a;
-        gkp = b;
-        gg[kit - 1] = gk;
-        gg[kit] = gkp;
-    }
-    H[kit - 1] = diag;
-    H[kit] = sub;
-    const double rho = fabs(gkp);
-    sc->rho = rho;
-    sc->sumav = rho / sc->sumnor;
-    if (ahead && !(sc->sumav > stop_at)) sc->stop = 1;
+    __syncthreads();
+    return *s_last;
 }
+
+// Block partials of N consecutive values, in a fixed order, by one warp: lanes
+// strided over the blocks.  Lane l has the total of value l / (32 / N).
+template <int N>
+__device__ __forceinline__ double sum_partials(const double* p, int max_blocks, int nb) {
+    double t[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) t[e] = 0.0;
+#pragma unroll 4
+    for (int q = threadIdx.x & 31; q < nb; q += 32)
+#pragma unroll
+        for (int e = 0; e < N; ++e) t[e] += __ldcg(p + (size_t)e * max_blocks + q);
+    return warp_reduce_scatter<N>(t);
+}
+
+// Givens rotations for column kit (1-based) (:1165-1189) by one warp.  The
+// rotations so far are a chain, cur = s_i cur + c_i h_{i+1}, of one FMA each
+// when the lanes have formed c_i h_{i+1} before (an FP64 instruction of one
+// thread takes as long as one of a warp: four of them a rotation, 5 us at 40
+// rotations); the quotients are one division on three lanes.  The global loads
+// of the first 32 rotations are made before the sums that last waits for.
+struct Givens {
+    int kit;
+    double *H, *gg, *gc, *gs;  // H: the column, its first kit values set
+    DevScalars* sc;
+    bool ahead;  // Arnoldi steps enqueued ahead: the cycle stops when the estimate sumav
+    double stop_at;  // reaches stop_at (the host's loop test, evaluated on the same double)
+    double h0, nx, c, s, gk, gkp, sumnor;
+    __device__ __forceinline__ void load(int base) {
+        const int i = base + (threadIdx.x & 31);
+        const bool on = i < kit - 1;
+        nx = on ? H[i + 1] : 0.0;
+        c = on ? gc[i] : 0.0;
+        s = on ? gs[i] : 0.0;
+    }
+    __device__ __forceinline__ void prefetch() {
+        load(0);
+        h0 = H[0];
+        gk = gg[kit - 1];
+        gkp = gg[kit];
+        sumnor = sc->sumnor;
+    }
+    // last: the subdiagonal value; returns 1 / rec
+    __device__ __forceinline__ double column(double last, double rec) {
+        const int lane = threadIdx.x & 31;
+        double cur = h0;
+        for (int base = 0; base < kit - 1; base += 32) {
+            if (base > 0) load(base);
+            const int n = min(32, kit - 1 - base);
+            const double p = c * nx, q = s * nx;
+            double mine = 0.0;
+#pragma unroll 4
+            for (int t = 0; t < n; ++t) {
+                if (lane == t) mine = cur;
+                cur = fma(__shfl_sync(0xffffffffu, s, t), cur, __shfl_sync(0xffffffffu, p, t));
+            }
+            if (lane < n) H[base + lane] = fma(c, mine, -q);
+        }
+        const double nu = sqrt(cur * cur + last * last);
+        const double quot = (lane == 0 ? cur : lane == 1 ? -last : 1.0) / (lane < 2 ? nu : rec);
+        const double cn = __shfl_sync(0xffffffffu, quot, 0), sn = __shfl_sync(0xffffffffu, quot, 1);
+        double diag = cur, sub = last, a = gk, b = gkp;
+        if (nu > 0.0) {
+            diag = cn * cur - sn * last;
+            sub = 0.0;
+            a = cn * gk - sn * gkp;
+            b = sn * gk + cn * gkp;
+        }
+        const double rho = fabs(b), sumav = rho / sumnor;
+        if (lane == 0) {
+            if (nu > 0.0) {
+                gc[kit - 1] = cn;
+                gs[kit - 1] = sn;
+                gg[kit - 1] = a;
+                gg[kit] = b;
+            }
+            H[kit - 1] = diag;
+            H[kit] = sub;
+            sc->rho = rho;
+            sc->sumav = sumav;
+            if (ahead && !(sumav > stop_at)) sc->stop = 1;
+        }
+        return __shfl_sync(0xffffffffu, quot, 2);
+    }
+};
 
 // ---------------------------------------------------- Gram-Schmidt (FP64)
 // Modified Gram-Schmidt (:1140-1161) over blocks of 8 basis vectors.  One pass
@@ -146,7 +205,7 @@ struct GsPass {
     const double2* V;      // basis, n2 apart
     int p0, q0;            // first vector of the previous and of the next block
     int k;                 // vectors in the basis
-    double *d, *G;         // 1/|v_i|; <v_i, v_j> / (|v_i| |v_j|), j in i's block, [i][GSB]
+    double *d, *nd, *G;    // 1/|v_i|; |v_i|; <v_i, v_j> / (|v_i| |v_j|), j in i's block, [i][GSB]
     double *hcol, *hs;     // Hessenberg column; h_i d_i / d_k
     double* partial;       // [16][max_blocks]
     unsigned* count;
@@ -156,7 +215,6 @@ struct GsPass {
     DevScalars* sc;
     const int* skip;
     double stop_at;
-    int staged;
 };
 
 // NP, NQ: vectors of the two blocks (0: none).  GRAM: the next block holds the
@@ -168,7 +226,6 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     constexpr int NV = NQ == 0 ? 1 : GRAM && NQ > 1 ? 16 : 8;  // sums of the pass
     __shared__ double s_red[16 * NW];
     __shared__ double s_val[16];
-    extern __shared__ double s_h[];  // 3 (k + 1) values, unless they do not fit (a.staged)
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned long long keep = l2_keep_policy();
@@ -203,76 +260,79 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     const double tot = warp_reduce_scatter<NV>(acc);  // value lane / (32 / NV)
     if (lane % (32 / NV) == 0) s_red[lane / (32 / NV) * NW + wid] = tot;
     __syncthreads();
-    if (threadIdx.x < NV) {
-        double t = 0.0;
-        for (int q = 0; q < NW; ++q) t += s_red[threadIdx.x * NW + q];
-        a.partial[(size_t)threadIdx.x * a.max_blocks + blockIdx.x] = t;
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(a.count, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    // the last block: every value's partials in a fixed order, one warp per value
-    __threadfence();
-    for (int v = wid; v < NV; v += NW) {
-        if (NQ > 0 && (v < 8 ? v >= NQ : v - 8 >= NQ - 1)) continue;
-        const double* p = a.partial + (size_t)v * a.max_blocks;
-        double t = 0.0;
-        for (int q = lane; q < (int)gridDim.x; q += 32) t += __ldcg(p + q);
-        t = warp_sum(t);
-        if (lane == 0) s_val[v] = t;
-    }
-    double* const hc = a.h + (size_t)a.K1 * (a.k - 1);
-    if (NQ == 0 && a.staged)  // the Givens rotations' inputs meanwhile
-        for (int i = threadIdx.x; i < a.k; i += blockDim.x) {
-            s_h[i] = hc[i];
-            s_h[a.k + 1 + i] = a.gc[i];
-            s_h[2 * (a.k + 1) + i] = a.gs[i];
-        }
-    __syncthreads();
-    const double dk = a.d[a.k - 1];
-    if (NQ != 0) {
-        if (wid == 0) {
-            const int i = a.q0 + lane;
-            const double di = lane < NQ ? a.d[i] : 0.0;
-            double c = lane < NQ ? di * dk * s_val[lane] : 0.0;
-            double grow[GSB];  // this lane's row of the block's products
+    if (threadIdx.x < (NV * NW > 32 ? NV * NW : 32)) {
+        double t = s_red[threadIdx.x];
 #pragma unroll
-            for (int j = 0; j < GSB - 1; ++j) {
-                grow[j] = 0.0;
-                if (lane < NQ && j < lane) {
-                    if (GRAM && lane == NQ - 1) {
-                        grow[j] = a.d[a.q0 + j] * dk * s_val[8 + j];
-                        a.G[(size_t)i * GSB + j] = grow[j];
-                    } else {
-                        grow[j] = a.G[(size_t)i * GSB + j];
-                    }
+        for (int o = NW / 2; o >= 1; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x % NW == 0 && threadIdx.x / NW < NV)
+            a.partial[(size_t)(threadIdx.x / NW) * a.max_blocks + blockIdx.x] = t;
+    }
+    if (!last_arrival(a.count, gridDim.x, &s_last)) return;
+    // the last block: what the solve or the rotations need, fetched while the
+    // other warps sum the partials, two values a warp
+    const int i = a.q0 + lane;
+    double di = 0.0, dk = 0.0, nk = 0.0, grow[GSB];
+    Givens gv = {a.k, a.h + (size_t)a.K1 * (a.k - 1), a.gg, a.gc, a.gs, a.sc, a.skip != nullptr, a.stop_at};
+    if (wid == 0) {
+        dk = a.d[a.k - 1];
+        nk = a.nd[a.k - 1];
+        if (NQ == 0) {
+            gv.prefetch();
+        } else {
+            di = lane < NQ ? a.d[i] : 0.0;
+#pragma unroll
+            for (int j = 0; j < GSB - 1; ++j)  // this lane's row of the block's products
+                grow[j] = lane < NQ - GRAM && j < lane ? a.G[(size_t)i * GSB + j] : 0.0;
+        }
+    }
+    if (NV == 1) {
+        if (wid == 0) {
+            const double t = sum_partials<1>(a.partial, a.max_blocks, gridDim.x);
+            if (lane == 0) s_val[0] = t;
+        }
+        __syncwarp();
+    } else {
+        if (2 * wid < NV) {
+            const double t = sum_partials<2>(a.partial + (size_t)(2 * wid) * a.max_blocks, a.max_blocks, gridDim.x);
+            if (lane % 16 == 0) s_val[2 * wid + lane / 16] = t;
+        }
+        __syncthreads();
+    }
+    if (wid != 0) return;
+    if (NQ != 0) {
+        double c = lane < NQ ? di * dk * s_val[lane] : 0.0;
+        if (GRAM && NQ > 1) {
+#pragma unroll
+            for (int j = 0; j < NQ - 1; ++j) {
+                const double dj = __shfl_sync(0xffffffffu, di, j);
+                if (lane == NQ - 1) {
+                    grow[j] = dj * dk * s_val[8 + j];
+                    a.G[(size_t)i * GSB + j] = grow[j];
                 }
             }
-#pragma unroll
-            for (int j = 0; j < GSB - 1; ++j) c = fma(-grow[j], __shfl_sync(0xffffffffu, c, j), c);
-            if (lane < NQ) {
-                a.hcol[i] = c;
-                a.hs[i] = c * di / dk;
-            }
         }
-    } else if (threadIdx.x == 0) {
-        const double nh = sqrt(s_val[0]), nrm = dk * nh;
-        a.d[a.k] = nh > 0.0 ? 1.0 / nh : 1.0;
-        double* const h2 = a.staged ? s_h : hc;
-        h2[a.k] = nrm;
-        givens_column(a.k, h2, a.staged ? s_h + a.k + 1 : a.gc, a.staged ? s_h + 2 * (a.k + 1) : a.gs, hc, a.gg, a.gc,
-                      a.gs, a.sc, a.skip != nullptr, a.stop_at);
+#pragma unroll
+        for (int j = 0; j < GSB - 1; ++j) c = fma(-grow[j], __shfl_sync(0xffffffffu, c, j), c);
+        if (lane < NQ) {
+            a.hcol[i] = c;
+            a.hs[i] = c * di * nk;
+        }
+    } else {
+        const double nh = sqrt(s_val[0]);
+        const double r = gv.column(dk * nh, nh);
+        if (lane == 0) {
+            a.d[a.k] = nh > 0.0 ? r : 1.0;
+            a.nd[a.k] = nh > 0.0 ? nh : 1.0;
+        }
     }
-    if (threadIdx.x == 0) *a.count = 0u;
+    if (lane == 0) *a.count = 0u;
 }
 
 // Start of a restart (:958-963, :1048-1056): zero h, c, s, g, y; g(1) = rho;
 // sumnor at the first restart; sumav = rho/sumnor.
-// d: 1/|v_i| of the basis vectors, kept as they come (FP64), or null.
+// d, nd: 1/|v_i| and |v_i| of the basis vectors, kept as they come (FP64), or null.
 __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double* gs, double* gy, DevScalars* sc,
-                               int first, double* d) {
+                               int first, double* d, double* nd) {
     for (int q = threadIdx.x; q < K1 * K1; q += blockDim.x) h[q] = 0.0;
     for (int q = threadIdx.x; q < K1; q += blockDim.x) { gg[q] = 0.0; gc[q] = 0.0; gs[q] = 0.0; gy[q] = 0.0; }
     __syncthreads();
@@ -282,21 +342,49 @@ __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double
         if (first) sc->sumnor = rho;
         sc->sumav = rho / sc->sumnor;
         gg[0] = rho;
-        if (d) d[0] = rho > 0.0 ? 1.0 / rho : 1.0;
+        if (d) {
+            d[0] = rho > 0.0 ? 1.0 / rho : 1.0;
+            nd[0] = rho > 0.0 ? rho : 1.0;
+        }
     }
 }
 
-// y from the triangular h (:1193-1200), one warp, a column at a time; with d
-// the coefficients of the basis vectors as they are kept, y_i / |v_i|.
-__global__ void __launch_bounds__(32) k_backsub(int K1, int kit, const double* h, double* gg, double* gy,
-                                                const double* d) {
-    const int lane = threadIdx.x;
-    for (int i = kit - 1; i >= 0; --i) {
-        const double* H = h + (size_t)K1 * i;
-        __syncwarp();
-        const double y = gg[i] / H[i];
-        for (int j = lane; j < i; j += 32) gg[j] -= H[j] * y;
-        if (lane == 0) gy[i] = d ? y * d[i] : y;
+// y from the triangular h (:1193-1200), 32 columns at a time: one warp solves
+// the triangle in registers (the column chain is a multiplication, a shuffle and
+// an FMA), then all threads take the 32 columns off the rows above.  A column at
+// a time through global memory took 54 us at 36 columns.  With d the
+// coefficients of the basis vectors as they are kept, y_i / |v_i|.
+__global__ void __launch_bounds__(128) k_backsub(int K1, int kit, const double* h, double* gg, double* gy,
+                                                 const double* d) {
+    __shared__ double s_y[32];
+    for (int base = (kit - 1) / 32 * 32; base >= 0; base -= 32) {
+        const int n = min(32, kit - base);
+        if (threadIdx.x < 32) {
+            const int lane = threadIdx.x, row = base + lane;
+            double H[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) H[i] = i < n && lane <= i ? h[(size_t)K1 * (base + i) + row] : 0.0;
+            double g = lane < n ? gg[row] : 0.0, diag = 1.0;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (lane == i && i < n) diag = H[i];
+            const double inv = 1.0 / diag;
+#pragma unroll
+            for (int i = 31; i >= 0; --i) {
+                const double y = __shfl_sync(0xffffffffu, g * inv, i);
+                if (lane < i) g = fma(-H[i], y, g);
+            }
+            const double y = lane < n ? g / diag : 0.0;
+            s_y[lane] = y;
+            if (lane < n) gy[row] = d ? y * d[row] : y;
+        }
+        __syncthreads();
+        for (int j = threadIdx.x; j < base; j += blockDim.x) {
+            double g = gg[j];
+            for (int i = 0; i < n; ++i) g = fma(-h[(size_t)K1 * (base + i) + j], s_y[i], g);
+            gg[j] = g;
+        }
+        __syncthreads();
     }
 }
 
@@ -305,6 +393,7 @@ __global__ void k_update(long long n2, double2* __restrict__ pc, const double2* 
                          const double* __restrict__ gy, int kit) {
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n2; q += (long long)gridDim.x * blockDim.x) {
         double2 x = pc[q];
+#pragma unroll 4
         for (int i = 0; i < kit; ++i) {
             double2 v = V[(long long)i * vstride2 + q];
             double y = gy[i];
@@ -446,6 +535,7 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
     a.k = k;
     a.K1 = h->cfg.kmax + 1;
     a.d = h->gs_d;
+    a.nd = h->gs_nd;
     a.G = h->gs_G;
     a.hs = h->gs_hs;
     a.h = h->h;
@@ -456,8 +546,6 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
     a.max_blocks = h->red.max_blocks;
     a.skip = skip;
     a.stop_at = stop_at;
-    const size_t stage = 3 * (size_t)(k + 1) * sizeof(double);
-    a.staged = stage <= 40 * 1024;
     long long nb = (a.n2 + RED_THREADS - 1) / RED_THREADS;
     const long long wave = 2LL * (h->n_sm > 0 ? h->n_sm : 148);
     if (nb > wave) nb = wave;
@@ -469,7 +557,7 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
                                    : b == nblk - 1 ? (b == 0 ? gs_newest<0>(rest) : gs_newest<GSB>(rest))
                                    : b == 0        ? k_gs_pass<0, GSB, false>
                                                    : k_gs_pass<GSB, GSB, false>;
-        fn<<<(unsigned)nb, RED_THREADS, b == nblk && a.staged ? stage : 0, h->stream>>>(a);
+        fn<<<(unsigned)nb, RED_THREADS, 0, h->stream>>>(a);
         h->launches++;
     }
     return TBL_OK;
@@ -477,14 +565,14 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
 
 int launch_restart_init(tbl_handle* h, int first) {
     const int K1 = h->cfg.kmax + 1;
-    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, h->gs_d);
+    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, h->gs_d, h->gs_nd);
     h->launches++;
     return TBL_OK;
 }
 
 int launch_backsub_update(tbl_handle* h, int kit) {
     const int K1 = h->cfg.kmax + 1;
-    k_backsub<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy, h->gs_d);
+    k_backsub<<<1, 128, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy, h->gs_d);
     int nb = red_blocks(h);
     k_update<<<nb, RED_THREADS, 0, h->stream>>>(h->g.vol / 2, (double2*)h->PC, (const double2*)h->V, h->g.vol / 2,
                                                 h->gy, kit);
@@ -515,21 +603,30 @@ __device__ __forceinline__ float dot4f(float4 a, float4 b) {
 template <int G>
 __device__ __forceinline__ void lsg_dots(long long n4, const float4* __restrict__ w, const float4* __restrict__ l,
                                          const float4* __restrict__ V, long long vstride4, double (&acc)[16]) {
-    float fd[G], fg[G];
 #pragma unroll
-    for (int e = 0; e < G; ++e) { fd[e] = 0.f; fg[e] = 0.f; }
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += stride) {
-        const float4 x = w[q], y = l[q];
+    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+    const long long stride = (long long)gridDim.y * blockDim.x;
+    for (long long q = (long long)blockIdx.y * blockDim.x + threadIdx.x; q < n4;) {
+        float fd[G], fg[G];
+#pragma unroll
+        for (int e = 0; e < G; ++e) { fd[e] = 0.f; fg[e] = 0.f; }
+        for (int n = 0; n < 16 && q < n4; ++n, q += stride) {
+            const float4 x = w[q], y = l[q];
+            float4 v[G];
+#pragma unroll
+            for (int e = 0; e < G; ++e) v[e] = __ldcs(V + (long long)e * vstride4 + q);  // read once: evict first
+#pragma unroll
+            for (int e = 0; e < G; ++e) {
+                fd[e] += dot4f(v[e], x);
+                fg[e] += dot4f(v[e], y);
+            }
+        }
 #pragma unroll
         for (int e = 0; e < G; ++e) {
-            const float4 v = __ldcs(V + (long long)e * vstride4 + q);  // read once: evict first
-            fd[e] += dot4f(v, x);
-            fg[e] += dot4f(v, y);
+            acc[2 * e] += (double)fd[e];
+            acc[2 * e + 1] += (double)fg[e];
         }
     }
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = e < 2 * G ? (double)(e % 2 == 0 ? fd[e / 2] : fg[e / 2]) : 0.0;
 }
 
 struct LsgArgs {
@@ -538,7 +635,7 @@ struct LsgArgs {
     const float4* V;  // basis, n4 apart
     int nv;           // its vectors
     double* partial;  // [16 per group][max_blocks]
-    unsigned* count;
+    unsigned* count;  // [0] groups done, [1 + group] blocks done
     int max_blocks;
     int K1;
     double *L, *hcol;  // strictly lower triangle of the basis' products; Hessenberg column
@@ -548,24 +645,23 @@ struct LsgArgs {
     double stop_at;
 };
 
-// d = Q^T w and the newest row of L, one group of LSG_G basis vectors per
-// blockIdx.y, then in the last block to finish the Hessenberg column t from
-// (I + L) t = d: the block partials of each value summed by one warp (lanes
-// strided over the blocks, four loads in flight per lane, then the shuffle
-// tree), the forward substitution by columns in one warp.  Three launches per
-// Arnoldi step (sums, solve, Givens; 30 us at 128 x 66 x 64) became the tails of
-// the two passes; L's older rows are fetched while the sums are formed.
-__global__ void __launch_bounds__(RED_THREADS) k_lsg_dots_f(const LsgArgs a) {
+// d = Q^T w and the newest row of L, the basis in groups of at most LSG_G
+// vectors, one per blockIdx.x (the groups of a stretch of w run together and
+// share it in L2: 275 -> 263 us at 40 vectors, 512 x 130 x 128).  The last block
+// of a group sums its block partials, the last group solves (I + L) t = d for
+// the Hessenberg column: a forward substitution in one warp's registers, L
+// fetched into shared memory while the sums are formed.
+__global__ void __launch_bounds__(RED_THREADS, 2) k_lsg_dots_f(const LsgArgs a) {
     if (a.skip && *a.skip) return;
     constexpr int NW = RED_THREADS / 32;
     __shared__ double s_red[16 * NW];
-    __shared__ double s_d[64];
-    extern __shared__ double sL[];  // nv x nv
+    extern __shared__ double sL[];  // nv columns of nv (odd) values
     __shared__ bool s_last;
-    const int nv = a.nv, i0 = LSG_G * blockIdx.y, left = nv - i0;
+    const int nv = a.nv, ngr = gridDim.x, grp = blockIdx.x;
+    const int i0 = grp * nv / ngr, G = (grp + 1) * nv / ngr - i0;
     const float4 *l = a.V + (long long)(nv - 1) * a.n4, *V = a.V + (long long)i0 * a.n4;
     double acc[16];
-    switch (left < LSG_G ? left : LSG_G) {
+    switch (G) {
         case 1: lsg_dots<1>(a.n4, a.w, l, V, a.n4, acc); break;
         case 2: lsg_dots<2>(a.n4, a.w, l, V, a.n4, acc); break;
         case 3: lsg_dots<3>(a.n4, a.w, l, V, a.n4, acc); break;
@@ -579,90 +675,100 @@ __global__ void __launch_bounds__(RED_THREADS) k_lsg_dots_f(const LsgArgs a) {
     const double tot = warp_reduce_scatter<16>(acc);  // value lane >> 1
     if ((lane & 1) == 0) s_red[(lane >> 1) * NW + wid] = tot;
     __syncthreads();
-    if (threadIdx.x < 16) {
-        double t = 0.0;
-        for (int k = 0; k < NW; ++k) t += s_red[threadIdx.x * NW + k];
-        a.partial[((size_t)blockIdx.y * 16 + threadIdx.x) * a.max_blocks + blockIdx.x] = t;
-        __threadfence();
+    double* const part = a.partial + (size_t)grp * 16 * a.max_blocks;
+    if (threadIdx.x < 16 * NW) {
+        double t = s_red[threadIdx.x];
+#pragma unroll
+        for (int o = NW / 2; o >= 1; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x % NW == 0) part[(size_t)(threadIdx.x / NW) * a.max_blocks + blockIdx.y] = t;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(a.count, 1u) == gridDim.x * gridDim.y - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const int r = nv - 1, nb = gridDim.x;
-    for (int q = threadIdx.x; q < r * nv; q += blockDim.x)
-        if (q % nv < q / nv) sL[q] = a.L[(size_t)(q / nv) * a.K1 + q % nv];
-    for (int v = wid; v < 2 * nv; v += NW) {  // d_i for even v, the new row's <v_i, l> for odd v
-        const double* p = a.partial + (size_t)v * a.max_blocks;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        int b = lane;
-        for (; b + 96 < nb; b += 128) {
-            a0 += __ldcg(p + b);
-            a1 += __ldcg(p + b + 32);
-            a2 += __ldcg(p + b + 64);
-            a3 += __ldcg(p + b + 96);
-        }
-        for (; b < nb; b += 32) a0 += __ldcg(p + b);
-        const double t = warp_sum((a0 + a1) + (a2 + a3));
-        const int i = v >> 1;
-        if (lane == 0) {
-            if ((v & 1) == 0) s_d[i] = t;
-            else if (i < r) {
-                sL[r * nv + i] = t;
-                a.L[(size_t)r * a.K1 + i] = t;
-            }
+    if (!last_arrival(a.count + 1 + grp, gridDim.y, &s_last)) return;
+    const int r = nv - 1, ld = nv | 1;
+    for (int q = threadIdx.x; q < nv * nv; q += blockDim.x) {  // L's older rows, zeros elsewhere
+        const int row = q / nv, col = q % nv;
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(sL + col * ld + row);
+        if (col < row && row < r)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(a.L + (size_t)row * a.K1 + col) : "memory");
+        else
+            sL[col * ld + row] = 0.0;
+    }
+    if (wid < G) {  // <v, w> on lane 0, <v, l> on lane 16
+        const double t = sum_partials<2>(part + (size_t)(2 * wid) * a.max_blocks, a.max_blocks, gridDim.y);
+        const int i = i0 + wid;
+        if (lane == 0) a.hcol[i] = t;
+        if (lane == 16 && i < r) a.L[(size_t)r * a.K1 + i] = t;
+    }
+    if (threadIdx.x == 0) a.count[1 + grp] = 0u;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!last_arrival(a.count, ngr, &s_last) || wid != 0) return;
+    // rows lane and lane + 32 (nv <= 63); the newest row's products straight from memory
+    double t0 = lane < nv ? __ldcg(a.hcol + lane) : 0.0, t1 = 32 + lane < nv ? __ldcg(a.hcol + 32 + lane) : 0.0;
+    for (int j = lane; j < r; j += 32) sL[j * ld + r] = __ldcg(a.L + (size_t)r * a.K1 + j);
+    __syncwarp();
+    if (nv <= 32) {
+#pragma unroll 4
+        for (int j = 0; j < r; ++j) t0 = fma(-(lane < nv ? sL[j * ld + lane] : 0.0), __shfl_sync(0xffffffffu, t0, j), t0);
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < r; ++j) {
+            const double tj = __shfl_sync(0xffffffffu, j < 32 ? t0 : t1, j & 31);
+            t0 = fma(-sL[j * ld + lane], tj, t0);
+            t1 = fma(-(32 + lane < nv ? sL[j * ld + 32 + lane] : 0.0), tj, t1);
         }
     }
-    __syncthreads();
-    if (wid == 0) {  // nv <= 64: each lane owns rows lane and lane + 32
-        for (int j = 0; j < nv; ++j) {
-            const double tj = s_d[j];  // final: every earlier column has been applied
-            for (int i = j + 1 + lane; i < nv; i += 32) s_d[i] -= sL[i * nv + j] * tj;
-            __syncwarp();
-        }
-        for (int i = lane; i < nv; i += 32) a.hcol[i] = s_d[i];
-    }
-    if (threadIdx.x == 0) *a.count = 0u;
+    if (lane < nv) a.hcol[lane] = t0;
+    if (32 + lane < nv) a.hcol[32 + lane] = t1;
+    if (lane == 0) *a.count = 0u;
 }
 
-// w -= sum_i t_i v_i (FP32), then in the last block ||w|| (sqrt of the
-// deterministic sum) and the column's Givens rotation
-__global__ void __launch_bounds__(RED_THREADS, 6) k_lsg_update_f(const LsgArgs a, RedWork rw, int slot) {
+// w -= sum_i t_i v_i (FP32), eight vectors' loads in flight per thread (four,
+// with six blocks per SM: 249 -> 217 us at 40 vectors, 512 x 130 x 128, 35 -> 27
+// at 128 x 66 x 64), then in the last block ||w|| (sqrt of the deterministic
+// sum) and the column's Givens rotation.
+__global__ void __launch_bounds__(RED_THREADS, 4) k_lsg_update_f(const LsgArgs a, RedWork rw, int slot) {
     if (a.skip && *a.skip) return;
     __shared__ double s_red[RED_THREADS / 32];
     __shared__ float s_t[64];
-    __shared__ double s_h[3][64];
+    __shared__ bool s_last;
     const int nv = a.nv;
-    for (int i = threadIdx.x; i < nv && i < 64; i += blockDim.x) s_t[i] = (float)a.hcol[i];
+    if (threadIdx.x < 64) s_t[threadIdx.x] = threadIdx.x < nv ? (float)a.hcol[threadIdx.x] : 0.f;
     __syncthreads();
     double acc = 0.0;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < a.n4;
          q += (long long)gridDim.x * blockDim.x) {
         float4 x = a.w[q];
-#pragma unroll 4
-        for (int i = 0; i < nv; ++i) {
-            const float4 v = __ldcs(a.V + (long long)i * a.n4 + q);  // read once: evict first
-            const float ti = s_t[i];
-            x.x = fmaf(-ti, v.x, x.x);
-            x.y = fmaf(-ti, v.y, x.y);
-            x.z = fmaf(-ti, v.z, x.z);
-            x.w = fmaf(-ti, v.w, x.w);
+        for (int i = 0; i < nv; i += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)  // read once: evict first
+                v[e] = i + e < nv ? __ldcs(a.V + (long long)(i + e) * a.n4 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float ti = s_t[i + e];
+                x.x = fmaf(-ti, v[e].x, x.x);
+                x.y = fmaf(-ti, v[e].y, x.y);
+                x.z = fmaf(-ti, v[e].z, x.z);
+                x.w = fmaf(-ti, v[e].w, x.w);
+            }
         }
         a.w[q] = x;
         acc += (double)dot4f(x, x);
     }
     const double bt = block_sum(acc, s_red);
-    if (!grid_finish(bt, rw, slot, gridDim.x, blockIdx.x, &s_h[0][nv], 1)) return;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-        s_h[0][i] = a.hcol[i];
-        s_h[1][i] = a.gc[i];
-        s_h[2][i] = a.gs[i];
+    if (threadIdx.x == 0) rw.partial[(size_t)slot * rw.max_blocks + blockIdx.x] = bt;
+    if (!last_arrival(rw.count + slot, gridDim.x, &s_last)) return;
+    Givens gv = {nv, a.hcol, a.gg, a.gc, a.gs, a.sc, a.skip != nullptr, a.stop_at};
+    if (threadIdx.x < 32) gv.prefetch();
+    double t = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += __ldcg(rw.partial + (size_t)slot * rw.max_blocks + b);
+    t = block_sum(t, s_red);
+    if (threadIdx.x >= 32) return;
+    const double nrm = sqrt(__shfl_sync(0xffffffffu, t, 0));
+    gv.column(nrm, 1.0);
+    if (threadIdx.x == 0) {
+        a.sc->red[8] = nrm;  // the next step's matvec divides by it
+        rw.count[slot] = 0u;
     }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    a.sc->red[8] = s_h[0][nv];  // the next step's matvec divides by it
-    givens_column(nv, s_h[0], s_h[1], s_h[2], a.hcol, a.gg, a.gc, a.gs, a.sc, a.skip != nullptr, a.stop_at);
 }
 
 // Orthogonalises W against the kit <= 63 vectors of the FP32 basis, then the
@@ -676,24 +782,24 @@ int launch_lsg_f(tbl_handle* h, float* W, int kit, const int* skip, double stop_
     a.V = (const float4*)h->Vf;
     a.nv = kit;
     a.partial = h->lsg_partial;
-    a.count = h->red.count + 15;
+    a.count = h->red.count + 15;  // and one for each of at most 8 groups
     a.max_blocks = h->red.max_blocks;
     a.L = h->lsg_L;
     a.hcol = h->h + (size_t)a.K1 * (kit - 1);
     a.gg = h->gg; a.gc = h->gc; a.gs = h->gs; a.sc = h->sc;
     a.skip = skip;
     a.stop_at = stop_at;
-    // about 16 float4 per thread, fewer where that leaves SMs without 4 blocks
-    // (16 rounds of load latency: 56 us a Gram-Schmidt at 128 x 66 x 64)
+    // one resident wave over all groups: two blocks per SM, one where a block
+    // has at most 8 rounds, which then count less than the partials to be summed
+    // (14.4 -> 11.3 us at 4 vectors, 128 x 66 x 64; 48 -> 59 at 20, 333 x 99 x 85)
     const int ngr = (kit + LSG_G - 1) / LSG_G, sms = h->n_sm > 0 ? h->n_sm : 148;
     const long long one = (a.n4 + RED_THREADS - 1) / RED_THREADS;  // one float4 per thread
-    long long nbd = (one + 15) / 16;
-    if (nbd * ngr < 4 * sms) nbd = (4 * sms + ngr - 1) / ngr;
+    long long nbd = (one * ngr <= 8LL * sms ? 1LL : 2LL) * sms / ngr;
     if (nbd > one) nbd = one;
     if (nbd > h->red.max_blocks) nbd = h->red.max_blocks;
-    k_lsg_dots_f<<<dim3((unsigned)nbd, ngr), RED_THREADS, (size_t)kit * kit * sizeof(double),
-                   h->stream>>>(a);
-    long long nbu = 6LL * sms;  // one resident wave at 6 blocks per SM
+    if (nbd < 1) nbd = 1;
+    k_lsg_dots_f<<<dim3(ngr, (unsigned)nbd), RED_THREADS, (size_t)kit * (kit | 1) * sizeof(double), h->stream>>>(a);
+    long long nbu = 4LL * sms;  // one resident wave at 4 blocks per SM
     if (nbu > one) nbu = one;
     k_lsg_update_f<<<(unsigned)nbu, RED_THREADS, 0, h->stream>>>(a, h->red, 7);
     h->launches += 2;
@@ -716,7 +822,7 @@ int launch_scale_by_inv_f(tbl_handle* h, float* w, const double* denom, const in
 
 int launch_backsub_update_f(tbl_handle* h, int kit) {
     const int K1 = h->cfg.mixed_kmax + 1;
-    k_backsub<<<1, 32, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy, h->gs_d);
+    k_backsub<<<1, 128, 0, h->stream>>>(K1, kit, h->h, h->gg, h->gy, h->gs_d);
     int nb = red_blocks(h);
     k_update_f<<<nb, RED_THREADS, 0, h->stream>>>(h->g.vol / 4, h->PC, (const float4*)h->Vf, h->g.vol / 4, h->gy,
                                                   kit);
@@ -725,7 +831,7 @@ int launch_backsub_update_f(tbl_handle* h, int kit) {
 }
 
 int launch_restart_init_k(tbl_handle* h, int first, int K1) {
-    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, nullptr);
+    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, nullptr, nullptr);
     h->launches++;
     return TBL_OK;
 }
