@@ -20,6 +20,7 @@
 #include "tbl_internal.cuh"
 #include "tbl_reduce.cuh"
 #include "tbl_kernels.cuh"
+#include "tbl_sync.cuh"
 
 namespace tbl {
 
@@ -51,7 +52,7 @@ struct GsFields {
 
 // pc: the handle's table k_gs_coef fills, [p0|p1|p2|p3|d|cT|cB|pb] x nz, p0 = 1/d.
 template <typename T, bool PRE, bool RESID>
-__global__ void __launch_bounds__(32 * GS_ROWS) k_gs_parts(Geom g, T cE, T cN, const double* __restrict__ pc,
+__global__ void __launch_bounds__(32 * GS_ROWS) k_gs_parts(Geom g, T cE, T cN, const double* pc,
                                                            const int* __restrict__ slab_of_k,
                                                            const SlabDesc* __restrict__ slabs, GsFields<T> f, int gx,
                                                            int gy, int gz, int kc, RedWork rw, DevScalars* sc) {
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(32 * GS_ROWS) k_gs_parts(Geom g, T cE, T cN, c
     const int comp = pick(f.comp, blockIdx.y), nz = g.nz;
     const T *U = pick(f.U, comp), *Q = pick(f.Q, comp);
     T* P = pick(f.PRE, comp);
+    dependent_wait(pc);
     double acc = 0.0;
     for (int t = blockIdx.x; t < gx * gy * gz; t += gridDim.x) {
         const int bx = t % gx, by = t / gx % gy, bz = t / (gx * gy);
@@ -207,10 +209,10 @@ static int gs_parts(tbl_handle* h, T* const U[3], T* const Q[3], T* const PRE[3]
         f.U[c] = U[c]; f.Q[c] = Q[c]; f.PRE[c] = PRE[c];
         f.comp[c] = c < ncomp ? comps[c] : 0;
     }
-    (pre ? resid ? k_gs_parts<T, true, true> : k_gs_parts<T, true, false>
-         : k_gs_parts<T, false, true>)<<<dim3((unsigned)nb, ncomp), dim3(32, GS_ROWS), 0, h->stream>>>(
-        g, cE, cN, h->gs_coef, h->slab_of_k, h->slabs, f, gx, gy, gz, kc, h->red, h->sc);
-    TBL_CUDA_TRY(cudaGetLastError());
+    TBL_CUDA_TRY(launch_dependent(pre ? resid ? k_gs_parts<T, true, true> : k_gs_parts<T, true, false>
+                                      : k_gs_parts<T, false, true>,
+                                  dim3((unsigned)nb, ncomp), dim3(32, GS_ROWS), 0, h->stream, g, cE, cN, h->gs_coef,
+                                  h->slab_of_k, h->slabs, f, gx, gy, gz, kc, h->red, h->sc));
     h->launches++;
     return TBL_OK;
 }

@@ -9,6 +9,7 @@
 #include "tbl_internal.cuh"
 #include "tbl_reduce.cuh"
 #include "tbl_kernels.cuh"
+#include "tbl_sync.cuh"
 
 namespace tbl {
 
@@ -221,6 +222,7 @@ struct GsPass {
 // newest vector (its last).
 template <int NP, int NQ, bool GRAM>
 __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
+    dependent_wait();
     if (a.skip && *a.skip) return;  // an Arnoldi step enqueued ahead of a converged one
     constexpr int NW = RED_THREADS / 32;
     constexpr int NV = NQ == 0 ? 1 : GRAM && NQ > 1 ? 16 : 8;  // sums of the pass
@@ -557,7 +559,7 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
                                    : b == nblk - 1 ? (b == 0 ? gs_newest<0>(rest) : gs_newest<GSB>(rest))
                                    : b == 0        ? k_gs_pass<0, GSB, false>
                                                    : k_gs_pass<GSB, GSB, false>;
-        fn<<<(unsigned)nb, RED_THREADS, 0, h->stream>>>(a);
+        TBL_CUDA_TRY(launch_dependent(fn, dim3((unsigned)nb), dim3(RED_THREADS), 0, h->stream, a));
         h->launches++;
     }
     return TBL_OK;
@@ -652,6 +654,7 @@ struct LsgArgs {
 // the Hessenberg column: a forward substitution in one warp's registers, L
 // fetched into shared memory while the sums are formed.
 __global__ void __launch_bounds__(RED_THREADS, 2) k_lsg_dots_f(const LsgArgs a) {
+    dependent_wait();
     if (a.skip && *a.skip) return;
     constexpr int NW = RED_THREADS / 32;
     __shared__ double s_red[16 * NW];
@@ -726,6 +729,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_lsg_dots_f(const LsgArgs a) 
 // at 128 x 66 x 64), then in the last block ||w|| (sqrt of the deterministic
 // sum) and the column's Givens rotation.
 __global__ void __launch_bounds__(RED_THREADS, 4) k_lsg_update_f(const LsgArgs a, RedWork rw, int slot) {
+    dependent_wait();
     if (a.skip && *a.skip) return;
     __shared__ double s_red[RED_THREADS / 32];
     __shared__ float s_t[64];
@@ -798,10 +802,11 @@ int launch_lsg_f(tbl_handle* h, float* W, int kit, const int* skip, double stop_
     if (nbd > one) nbd = one;
     if (nbd > h->red.max_blocks) nbd = h->red.max_blocks;
     if (nbd < 1) nbd = 1;
-    k_lsg_dots_f<<<dim3(ngr, (unsigned)nbd), RED_THREADS, (size_t)kit * (kit | 1) * sizeof(double), h->stream>>>(a);
+    TBL_CUDA_TRY(launch_dependent(k_lsg_dots_f, dim3(ngr, (unsigned)nbd), dim3(RED_THREADS),
+                                  (size_t)kit * (kit | 1) * sizeof(double), h->stream, a));
     long long nbu = 4LL * sms;  // one resident wave at 4 blocks per SM
     if (nbu > one) nbu = one;
-    k_lsg_update_f<<<(unsigned)nbu, RED_THREADS, 0, h->stream>>>(a, h->red, 7);
+    TBL_CUDA_TRY(launch_dependent(k_lsg_update_f, dim3((unsigned)nbu), dim3(RED_THREADS), 0, h->stream, a, h->red, 7));
     h->launches += 2;
     return TBL_OK;
 }

@@ -20,6 +20,7 @@
 
 #include "tbl_internal.cuh"
 #include "tbl_kernels.cuh"
+#include "tbl_sync.cuh"
 
 namespace tbl {
 
@@ -52,10 +53,9 @@ template <typename TI, typename TO, typename TC, bool RESID, bool NORM>
 __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double as, const double* __restrict__ Ab,
                                                        const double* __restrict__ At, const double* __restrict__ Ap,
                                                        const double* __restrict__ scale, int kc,
-                                                       const TI* __restrict__ X, const double* __restrict__ Q8,
-                                                       TO* __restrict__ R, const int* __restrict__ skip,
-                                                       const double* __restrict__ denom, TI* __restrict__ vout) {
-    if (skip && *skip) return;  // an Arnoldi step enqueued ahead of a converged one
+                                                       const TI* X, const double* Q8, TO* __restrict__ R,
+                                                       const int* skip, const double* denom,
+                                                       TI* __restrict__ vout) {
     constexpr int VEC = 16 / sizeof(TI);
     constexpr unsigned ALL = 0xffffffffu;
     __shared__ TC s_c[LAP_KC][6];  // s Ab, s At, s Ap, s aw, s as, s
@@ -65,6 +65,8 @@ __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double
         const double s = scale[k];
         s_c[q / 6][c] = (TC)(s * (c == 0 ? Ab[k] : c == 1 ? At[k] : c == 2 ? Ap[k] : c == 3 ? aw : c == 4 ? as : 1.0));
     }
+    dependent_wait(X);
+    if (skip && *skip) return;  // an Arnoldi step enqueued ahead of a converged one
     __syncthreads();
     const int j = 1 + LAP_ROWS * blockIdx.y + threadIdx.y;
     if (j > g.ny - 2) return;
@@ -155,9 +157,8 @@ static int lap(tbl_handle* h, const TI* X, const double* Q8, TO* R, const double
     if constexpr (sizeof(TI) == 4) fn = denom ? k_lap<TI, TO, TC, false, true> : k_lap<TI, TO, TC, false, false>;
     else if constexpr (sizeof(TO) == 4) fn = k_lap<TI, TO, TC, true, false>;
     else fn = Q8 ? k_lap<TI, TO, TC, true, false> : k_lap<TI, TO, TC, false, false>;
-    fn<<<dim3(gx, gy, (unsigned)((planes + kc - 1) / kc)), dim3(32, LAP_ROWS), 0, h->stream>>>(
-        g, aw, as, h->Ab, h->At, h->Ap, scale, kc, X, Q8, R, skip, denom, vout);
-    TBL_CUDA_TRY(cudaGetLastError());
+    TBL_CUDA_TRY(launch_dependent(fn, dim3(gx, gy, (unsigned)((planes + kc - 1) / kc)), dim3(32, LAP_ROWS), 0, h->stream,
+                                  g, aw, as, h->Ab, h->At, h->Ap, scale, kc, X, Q8, R, skip, denom, vout));
     h->launches++;
     return TBL_OK;
 }

@@ -201,6 +201,7 @@ __host__ __device__ constexpr int line_chunks(int nx) {
 
 template <int MODE, typename V, int E>
 __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 1) k_line(const LineArgs<V> a) {
+    dependent_wait();
     if (a.skip && *a.skip) return;  // every CTA reads the same word, written by an earlier launch
     using B = LineBits<V>;
     constexpr bool GS = MODE == 0, BWD = MODE == 2;
@@ -646,8 +647,8 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
 template <int MODE, typename V>
 static int line_launch(tbl_handle* h, const LineShape& q, LineArgs<V>& a, int nsets) {
     a.nsets = nsets;
-    line_fn<MODE, V>(q.E)<<<q.ncta * nsets, 32 * (q.S * q.KP + q.NC), q.smem, h->stream>>>(a);
-    TBL_CUDA_TRY(cudaGetLastError());
+    TBL_CUDA_TRY(launch_dependent(line_fn<MODE, V>(q.E), dim3(q.ncta * nsets), dim3(32 * (q.S * q.KP + q.NC)), q.smem,
+                                  h->stream, a));
     h->launches++;
     return TBL_OK;
 }

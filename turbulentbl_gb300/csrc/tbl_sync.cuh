@@ -15,6 +15,22 @@ __device__ __forceinline__ void st_release(unsigned long long* p, unsigned long 
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// Programmatic dependent launch: a kernel started with launch_dependent
+// (tbl_internal.cuh) begins when the blocks of the kernel in front of it have
+// left, before its end has been processed and its writes are all visible.  Every
+// thread executes dependent_wait before it touches what other kernels write; the
+// kernel before the one in front has ended by then, because that one has waited
+// for it.  (No kernel lets the next one begin earlier than that: its blocks came
+// to lie two to an SM, beside the last of a sweep, 303 -> 350 ms a mixed step at
+// 768 x 194 x 144, for 1% at 32 x 18 x 24.)
+__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the same, p being read afterwards only (also where the compiler takes what p
+// points to for constant)
+template <typename T>
+__device__ __forceinline__ void dependent_wait(T*& p) {
+    asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+}
+
 constexpr long long SPIN_LIMIT = 1LL << 24;  // ~1 s of polling, then the wait gives up
 
 constexpr long long XLINGER = 1LL << 27;  // bounded wait for the partner at the end
