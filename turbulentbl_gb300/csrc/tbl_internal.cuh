@@ -103,7 +103,7 @@ constexpr int sweep_chunk(size_t value_bytes) { return value_bytes == 4 ? 8 : 4;
 // How the line-scan sweeps (tbl_line.cu) split a grid; S = 0 where they do
 // not take it and the wavefront sweeps run.
 struct LineCta {
-    int slab, blk, kg;  // slab, span block, plane group
+    int bn, K, blk, kg;  // the slab's first plane and planes, span block, plane group
 };
 struct LineShape {
     int S = 0, E = 0;           // warps per line (0: not taken), points per lane

@@ -66,7 +66,6 @@ constexpr int LINE_BARS = LINE_XR + 4;
 template <typename V>
 struct LineArgs {
     Geom g;
-    const SlabDesc* slabs;
     const LineCta* ctas;     // CTAs of one component, lowest planes first
     unsigned* ticket;        // [taken, finished]
     int* err;
@@ -200,7 +199,7 @@ __host__ __device__ constexpr int line_chunks(int nx) {
 }
 
 template <int MODE, typename V, int E>
-__global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 1) k_line(const LineArgs<V> a) {
+__global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 1), 1) k_line(const LineArgs<V> a) {
     dependent_wait();
     if (a.skip && *a.skip) return;  // every CTA reads the same word, written by an earlier launch
     using B = LineBits<V>;
@@ -224,8 +223,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
     __syncthreads();
     const int set = (int)(s_ticket % (unsigned)a.nsets);
     const LineCta cta = a.ctas[s_ticket / (unsigned)a.nsets];
-    const SlabDesc sl = a.slabs[cta.slab];
-    const int J = g.ny - 2, K = sl.K;
+    const int J = g.ny - 2, K = cta.K;
     const int comp = GS ? a.comp[set] : 0;
     const int j0 = cta.blk * a.rows, nrow = min(a.rows, J - j0);  // logical rows [j0, j0 + nrow)
     const int jfirst = BWD ? J - 1 - j0 : j0;                     // logical row 0
@@ -233,7 +231,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
     const int kl = cta.kg * KP + kp;  // logical plane
     const bool sweeps = wid < NW && kl < K;
     const int kidx = BWD ? K - 1 - kl : kl;
-    const int k = sl.bn + (sweeps ? kidx : 0);
+    const int k = cta.bn + (sweeps ? kidx : 0);
     const bool below = kl > 0;  // a plane of the slab comes before this one
     unsigned long long* const full = bars + (sweeps ? wid : 0) * LINE_BARS;
     unsigned long long *const empty = full + XR, *const opfull = full + XR + 2;
@@ -246,12 +244,51 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
     auto xch_plane = [&](int kk) {
         return a.xch + ((((size_t)set * g.nz + kk) * J + j0) * S * 32 + lane) * E;
     };
-    if (wid >= NW) {
+    // The row segments of a warp's operands in global memory: chunks [c0, ..) of
+    // the line, at chunk c0 - clo of the slot.
+    const int C = line_chunks<V, E>(g.nx);
+    if (wid == NW + a.NC) {
+        // Feeder: the rows' operands, half a ring at a time, lane w for warp w (a
+        // bulk copy takes its thread about 100 cycles to issue).
+        const int fl = cta.kg * KP + lane / S, fs = lane % S;
+        const bool feeds = lane < NW && fl < K;
+        unsigned long long* const fb = bars + (feeds ? lane : 0) * LINE_BARS;
+        const int clo = BWD ? C - 32 * (fs + 1) : 32 * fs, c0 = max(clo, 0);
+        const unsigned bytes =
+            min((unsigned)(g.sx - E * c0), 32u * E - (unsigned)(E * (c0 - clo))) * (unsigned)sizeof(V);
+        const long long rstep = BWD ? -(long long)g.sx : (long long)g.sx;
+        const int fk = cta.bn + (feeds ? (BWD ? K - 1 - fl : fl) : 0);
+        const V* src = a.in[comp] + (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * fk) + E * c0;
+        const unsigned dst = smem_u32(rings) + ((unsigned)(feeds ? lane : 0) * XR * 2 * 32 + (unsigned)(c0 - clo)) * E *
+                                                   (unsigned)sizeof(V);
+        const int nh = feeds ? (nrow + H - 1) / H : 0;
+        int m = 0;
+        long long spins = 0;
+        bool fail = false;
+        while (__any_sync(ALL, m < nh && !fail)) {
+            const bool go = m < nh && !fail && (m < 2 || mbar_test(&fb[XR + (m & 1)], (unsigned)(m / 2 - 1) & 1u));
+            if (go) {
+                const int n = min(H, nrow - m * H);
+                mbar_arrive_expect_tx(&fb[XR + 2 + (m & 1)], bytes * n);
+                for (int w = 0; w < n; ++w, src += rstep)
+                    line_fetch(dst + (unsigned)((m & 1) * H + w) * 2 * LBYTES, src, bytes, smem_u32(&fb[XR + 2 + (m & 1)]));
+                ++m;
+                spins = 0;
+            } else if (m < nh && ++spins > SPIN_LIMIT) {
+                fail = true;
+            }
+            if (!__any_sync(ALL, go)) __nanosleep(64);
+        }
+        // every copy has landed before the CTA ends
+        for (int q = max(0, m - 2); q < m; ++q)
+            if (!mbar_wait(&fb[XR + 2 + (q & 1)], (unsigned)(q / 2) & 1u)) fail = true;
+        if (fail) atomicExch(a.err, TBL_ERR_TIMEOUT);
+    } else if (wid >= NW) {
         // Courier: the top plane of the CTA below, row by row, into the rings
         // of this CTA's first plane; its words are emptied for the next launch.
         if (cta.kg > 0 && cta.kg * KP < K) {
             const int kb = BWD ? K - cta.kg * KP : cta.kg * KP - 1;
-            V* src = xch_plane(sl.bn + kb);
+            V* src = xch_plane(cta.bn + kb);
             V none[E];
 #pragma unroll
             for (int e = 0; e < E; ++e) none[e] = B::empty();
@@ -282,27 +319,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
         unsigned long long* const up_full = full + S * LINE_BARS;
         V* xout = to_xch ? xch_plane(k) + (size_t)seg * 32 * E : nullptr;
 
-        // the row's segment in global memory: chunks [c0, ..) of the line, at
-        // chunk c0 - clo of the slot
-        const int C = line_chunks<V, E>(g.nx);
-        const int clo = BWD ? C - 32 * (seg + 1) : 32 * seg, c0 = max(clo, 0);
-        const unsigned lbytes =
-            min((unsigned)(g.sx - E * c0), 32u * E - (unsigned)(E * (c0 - clo))) * (unsigned)sizeof(V);
         const long long rstep = BWD ? -(long long)g.sx : (long long)g.sx;
-        const V* fsrc = a.in[comp] + (long long)g.sx * ((long long)(1 + jfirst) + (long long)g.ny * k) + E * c0;
-        const unsigned fdst = smem_u32(ring) + (unsigned)(c0 - clo) * E * (unsigned)sizeof(V), fbar = smem_u32(opfull);
-        // lane 0: the operands of rows [q, q + H), the next that fsrc points to
-        auto fetch = [&](int q) {
-            const int hh = (q / H) & 1, n = min(H, nrow - q);
-            if (n <= 0) return;
-            mbar_arrive_expect_tx(&opfull[hh], lbytes * n);
-            for (int w = 0; w < n; ++w, fsrc += rstep)
-                line_fetch(fdst + (unsigned)(hh * H + w) * 2 * LBYTES, fsrc, lbytes, fbar + 8u * hh);
-        };
-        if (lane == 0) {
-            fetch(0);
-            fetch(H);
-        }
 
         // this lane's points: chunk ch of the line in sweep order, i = i0 .. i0 + E - 1
         const int ch = seg * 32 + lane;
@@ -365,20 +382,26 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
         // without waiting, get() waits.  An ask that came too early has read a
         // stale slot, and get() follows.  Lanes beyond the line read what is
         // there: no point of the line depends on them.
+        // The first plane of a slab has zeros in the slots of the plane below, and
+        // looks at its operands' barrier in place of theirs.
         const V* const slot0 = ring + (BWD ? 31 - lane : lane) * E;
-        const V* const below0 = ring + (32 + lane) * E;
-        auto take = [&](int s, V(&o)[E]) {
-            line_read<V, E>(o, slot0 + s * 64 * E, BWD);
-            if (below) {
-                V xk[E];
-                line_read<V, E>(xk, below0 + s * 64 * E, false);
+        V* const below0 = ring + (32 + lane) * E;
+        if (!below) {
+            V none[E];
 #pragma unroll
-                for (int e = 0; e < E; ++e) o[e] = fma(ck, xk[e], o[e]);
-            }
+            for (int e = 0; e < E; ++e) none[e] = V(0);
+            for (int s = 0; s < XR; ++s) line_store<V, E>(below0 + s * 64 * E, none, false);
+        }
+        auto take = [&](int s, V(&o)[E]) {
+            V xk[E];
+            line_read<V, E>(o, slot0 + s * 64 * E, BWD);
+            line_read<V, E>(xk, below0 + s * 64 * E, false);
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[e] = fma(ck, xk[e], o[e]);
         };
+        auto there = [&](int s) { return below ? &full[s] : &opfull[s / H]; };
         auto ask = [&](int s, unsigned ph, V(&o)[E]) -> bool {
-            bool rdy = true;
-            if (below) rdy = mbar_test(&full[s], ph);
+            bool rdy = mbar_test(there(s), ph);
             if ((s & (H - 1)) == 0) rdy = mbar_test(&opfull[s / H], ph) && rdy;
             rdy = __all_sync(ALL, rdy);
             take(rdy ? s : (s ^ 1), o);  // the address waits for the test
@@ -386,20 +409,17 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
         };
         bool dead = false;  // a wait gave up: nothing waits any more, and the results mean nothing
         auto get = [&](int s, unsigned ph, V(&o)[E]) {
-            bool got = dead || !below || mbar_wait(&full[s], ph);
+            bool got = dead || mbar_wait(there(s), ph);
             if ((s & (H - 1)) == 0) got = (dead || mbar_wait(&opfull[s / H], ph)) && got;
             if (!__all_sync(ALL, got)) dead = true;
             take(s, o);
         };
         // The H rows up to q have been read: their slots are handed back to the
-        // plane below and fetch the operands of the rows XR later.
+        // plane below and to the feeder.
         auto done = [&](int q, int s) {
             if ((s & (H - 1)) != H - 1) return;
             __syncwarp();
-            if (lane == 0) {
-                if (below && q + H + 1 < nrow) mbar_arrive(&empty[s / H]);
-                fetch(q + H + 1);
-            }
+            if (lane == 0 && q + H + 1 < nrow) mbar_arrive(&empty[s / H]);
         };
 
         // One row: gr holds its right-hand side and the plane below's share.
@@ -433,7 +453,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
             const bool more = r + 1 < nrow;
             const int s1 = (u + 1) % XR;
             const unsigned ph1 = u + 1 == XR ? ph ^ 1u : ph;
-            const bool rdy = !more || ask(s1, ph1, gr);
+            const bool rdy = ask(s1, ph1, gr);  // (after the last row: what a slot holds, and not used)
             // the carry of the segment before
             if (seg > 0) {
                 long long spins = 0;
@@ -481,7 +501,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
 #pragma unroll
                 for (int e = 0; e < E; ++e) x0[GS ? e : 0] = x[e];
             }
-            if (!rdy) get(s1, ph1, gr);
+            if (!rdy && more) get(s1, ph1, gr);
             if (more) done(r + 1, s1);
         };
         get(0, 0u, gr);
@@ -491,7 +511,6 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS), 
             for (int u = 0; u < XR; ++u)
                 if (r0 + u < nrow) row(r0 + u, u, ph);
         }
-        // (a warp that gave up has waited for a second: its own fetches have landed)
         if (dead && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
         __syncwarp();
     }
@@ -574,7 +593,7 @@ static int line_table(const tbl_handle* h, LineShape& q) {
     for (int kg = 0; (int)t.size() < q.ncta; ++kg)
         for (int r = 0; r < h->P; ++r)
             if (kg * q.KP < h->en[r] - h->bn[r] + 1)
-                for (int blk = 0; blk < q.nblk; ++blk) t.push_back({r, blk, kg});
+                for (int blk = 0; blk < q.nblk; ++blk) t.push_back({h->bn[r], h->en[r] - h->bn[r] + 1, blk, kg});
     TBL_CUDA_TRY(cudaMalloc(&q.ctas, t.size() * sizeof(LineCta)));
     TBL_CUDA_TRY(cudaMemcpy(q.ctas, t.data(), t.size() * sizeof(LineCta), cudaMemcpyHostToDevice));
     return TBL_OK;
@@ -631,7 +650,6 @@ template <typename V>
 static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
     LineArgs<V> a = {};
     a.g = h->g;
-    a.slabs = h->slabs;
     a.ctas = q.ctas;
     a.ticket = h->line_ticket;
     a.err = h->err;
@@ -647,7 +665,7 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
 template <int MODE, typename V>
 static int line_launch(tbl_handle* h, const LineShape& q, LineArgs<V>& a, int nsets) {
     a.nsets = nsets;
-    TBL_CUDA_TRY(launch_dependent(line_fn<MODE, V>(q.E), dim3(q.ncta * nsets), dim3(32 * (q.S * q.KP + q.NC)), q.smem,
+    TBL_CUDA_TRY(launch_dependent(line_fn<MODE, V>(q.E), dim3(q.ncta * nsets), dim3(32 * (q.S * q.KP + q.NC + 1)), q.smem,
                                   h->stream, a));
     h->launches++;
     return TBL_OK;
