@@ -149,14 +149,6 @@ __device__ __forceinline__ void xch_put(float* p, const float (&v)[8]) {
     xch_put(p, reinterpret_cast<const float(&)[4]>(v[0]));
     xch_put(p + 4, reinterpret_cast<const float(&)[4]>(v[4]));
 }
-template <int E, typename V>
-__device__ __forceinline__ bool xch_row(V (&w)[E], const V* p) {
-    xch_ld(w, p);
-    bool have = true;
-#pragma unroll
-    for (int e = 0; e < E; ++e) have = have && !line_empty(w[e]);
-    return __all_sync(0xffffffffu, have);
-}
 __device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
@@ -284,33 +276,76 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
             if (!mbar_wait(&fb[XR + 2 + (q & 1)], (unsigned)(q / 2) & 1u)) fail = true;
         if (fail) atomicExch(a.err, TBL_ERR_TIMEOUT);
     } else if (wid >= NW) {
-        // Courier: the top plane of the CTA below, row by row, into the rings
-        // of this CTA's first plane; its words are emptied for the next launch.
-        if (cta.kg > 0 && cta.kg * KP < K) {
-            const int kb = BWD ? K - cta.kg * KP : cta.kg * KP - 1;
-            V* src = xch_plane(cta.bn + kb);
-            V none[E];
+        // Courier: the top plane of the CTA below, row by row, into the rings of
+        // this CTA's first plane; its words are emptied for the next launch.
+        const int sg0 = wid - NW;
+        const bool has = cta.kg > 0 && cta.kg * KP < K;
+        const int kb = BWD ? K - cta.kg * KP : cta.kg * KP - 1;
+        V* const src = xch_plane(has ? cta.bn + kb : cta.bn);
+        V none[E];
 #pragma unroll
-            for (int e = 0; e < E; ++e) none[e] = B::empty();
-            bool good = true;
-            for (int r = 0; r < nrow && good; ++r, src += xrow)
-                for (int sg = wid - NW; sg < S; sg += a.NC) {
-                    V* const from = src + (size_t)sg * 32 * E;
-                    const int u = r & (XR - 1);
-                    unsigned long long* fb = bars + sg * LINE_BARS;
-                    if ((u & (H - 1)) == 0 && r >= XR)
-                        good = __all_sync(ALL, mbar_wait(&fb[XR + u / H], (unsigned)(r / XR - 1) & 1u));
-                    V w[E];
-                    long long spins = 0;
-                    while (good && !xch_row<E>(w, from)) good = ++spins < SPIN_LIMIT / 16;
-                    if (!good) break;
-                    line_store<V, E>(rings + (((size_t)sg * XR + u) * 64 + 32 + lane) * E, w, false);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&fb[u]);
-                    xch_put(from, none);
+        for (int e = 0; e < E; ++e) none[e] = B::empty();
+        auto arrived = [&](const V(&w)[E]) {
+            bool have = true;
+#pragma unroll
+            for (int e = 0; e < E; ++e) have = have && !line_empty(w[e]);
+            return have;
+        };
+        auto hand = [&](int r, int sg, const V(&w)[E]) {
+            const int u = r & (XR - 1);
+            line_store<V, E>(rings + (((size_t)sg * XR + u) * 64 + 32 + lane) * E, w, false);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + sg * LINE_BARS + u);
+            xch_put(src + r * xrow + (size_t)sg * 32 * E, none);
+        };
+        bool good = true;
+        if (has && S <= a.NC) {  // one segment
+            unsigned long long* const fb = bars + sg0 * LINE_BARS + XR;
+            for (int r = 0; r < nrow && good; ++r) {
+                if ((r & (H - 1)) == 0 && r >= XR)
+                    good = __all_sync(ALL, mbar_wait(&fb[(r & (XR - 1)) / H], (unsigned)(r / XR - 1) & 1u));
+                V w[E];
+                for (long long spins = 0; good;) {
+                    xch_ld(w, src + r * xrow + (size_t)sg0 * 32 * E);
+                    if (__all_sync(ALL, arrived(w))) break;
+                    good = ++spins < SPIN_LIMIT / 16;
                 }
-            if (!good && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
+                if (good) hand(r, sg0, w);
+            }
+        } else if (has) {
+            // Several segments: a look at a word takes an L2 round trip, 700 cycles
+            // of a row's 1400, so one at each is in flight and none is waited for
+            // alone (taken in turn, 180 against 174 us a sweep at 512 x 130 x 128
+            // in FP64; a courier for each, whose registers the sweeping warps lack,
+            // 187; this loop for one segment costs a hand-over 0.3 us).
+            constexpr int CS = (line_max_warps(E) + LINE_MAX_COURIERS - 1) / LINE_MAX_COURIERS;
+            int row[CS];  // the next row of segments sg0, sg0 + NC, ..
+#pragma unroll
+            for (int c = 0; c < CS; ++c) row[c] = sg0 + c * a.NC < S ? 0 : nrow;
+            long long spins = 0;
+            for (bool more = true; more && good; good = ++spins < SPIN_LIMIT / 16) {
+                V w[CS][E];
+#pragma unroll
+                for (int c = 0; c < CS; ++c)
+                    if (row[c] < nrow) xch_ld(w[c], src + row[c] * xrow + (size_t)(sg0 + c * a.NC) * 32 * E);
+                more = false;
+#pragma unroll
+                for (int c = 0; c < CS; ++c) {
+                    if (row[c] >= nrow) continue;
+                    const int r = row[c], u = r & (XR - 1), sg = sg0 + c * a.NC;
+                    bool have = arrived(w[c]);
+                    if ((u & (H - 1)) == 0 && r >= XR)
+                        have = mbar_test(bars + sg * LINE_BARS + XR + u / H, (unsigned)(r / XR - 1) & 1u) && have;
+                    if (__all_sync(ALL, have)) {
+                        hand(r, sg, w[c]);
+                        ++row[c];
+                        spins = 0;
+                    }
+                    more = more || row[c] < nrow;
+                }
+            }
         }
+        if (!good && lane == 0) atomicExch(a.err, TBL_ERR_TIMEOUT);
     } else if (sweeps) {
         V* const ring = rings + (size_t)wid * XR * 64 * E;
         const bool has_up = kl + 1 < K;
