@@ -12,10 +12,10 @@
 // division by its norm, which it applies to every value it loads, and it writes
 // the divided vector into the basis.  512 x 130 x 128: 50 -> 25 us (105 MB read
 // and written) with TMA plane tiles in shared memory, whose barriers and
-// scaling pass over each tile were the time, replaced by registers.
+// scaling pass over each tile were the time, replaced by registers; the norm's
+// reciprocal by one warp of a block, 21.5 -> 19.5 us (128 x 66 x 64: 4.7 -> 3.2).
 // FP64: bound by FP64 issue, 7 operations a point (64 cycles a warp each); one
-// thread per point with the scale as an eighth took 137 us, now 118 us (110 us
-// at 600 G FMA/s).
+// thread per point with the scale as an eighth took 137 us, now 105 us.
 #include <algorithm>
 
 #include "tbl_internal.cuh"
@@ -67,6 +67,12 @@ __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double
     }
     dependent_wait(X);
     if (skip && *skip) return;  // an Arnoldi step enqueued ahead of a converged one
+    __shared__ TC s_rs;
+    if (NORM && threadIdx.y == LAP_ROWS - 1) {  // one warp: an FP64 division keeps its pipe for 1000 cycles
+        const double d = *denom;
+        const TC q = d > 0.0 || d < 0.0 ? (TC)(1.0 / d) : TC(1);
+        if (lane == 0) s_rs = q;
+    }
     __syncthreads();
     const int j = 1 + LAP_ROWS * blockIdx.y + threadIdx.y;
     if (j > g.ny - 2) return;
@@ -78,11 +84,7 @@ __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double
     for (int e = 0; e < VEC; ++e)
         if (first + e >= 1 && first + e <= g.nx - 2) okm |= 1u << e;
     const bool whole = okm == (1u << VEC) - 1;
-    TC rs = TC(1);
-    if (NORM) {
-        const double d = *denom;
-        if (d > 0.0 || d < 0.0) rs = (TC)(1.0 / d);
-    }
+    const TC rs = NORM ? s_rs : TC(1);
     auto load = [&](TC(&v)[VEC], const TI* p) {
         lap_load(v, p);
         if (NORM)
