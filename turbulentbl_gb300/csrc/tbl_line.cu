@@ -32,15 +32,18 @@
 // co-residency.  All waits are bounded; a wait that gives up sets the error
 // word and the warps that depend on it give up in turn.
 //
-// What bounds it: the serial chain of J + K rows.  A row of an FP64 warp with 1
-// point per lane takes about 1100 cycles, of which 440 are the scan (114 a
-// level: an FP64 FMA of 64 and two shuffles) and 180 the FMAs before it; the
-// rest, and most of an FP32 row's 950, is the issue of about 190 instructions
-// from one warp per scheduler.  A hand-over to the next CTA takes about 1.2 us.
-// SSOR sweep, wavefront -> line scan: 130 -> 62 us (128 x 66 x 64, FP64, 8
-// slabs), 389 -> 185 us (512 x 130 x 128, FP64), 95 -> 47 us and 251 -> 100 us
-// (FP32); GS sweep of three components with its precomputed terms 620 -> 650 us
-// less the launches it saves at 512, 280 -> 90 us at 128 (FP64).
+// What bounds it: the serial chain of J + K rows.  An FP64 row with 1 point per
+// lane takes about 900 cycles at 128 x 66 x 64, of which 320 are the scan (an
+// FP64 FMA of 64 and two shuffles a level) and 180 the other FMAs; the rest, and
+// most of an FP32 row's 620, is the issue of about 170 instructions from one
+// warp per scheduler, where a branch costs 20 to 30 cycles taken or not.  At
+// 512 x 130 x 128 two FP64 warps share a pipe: 1400.  A hand-over to the next
+// CTA takes about 1 us.  What left the row for that reason: operand copies (100
+// cycles each to issue; a feeder warp does it), selects and tests at its ends.
+// SSOR sweep, wavefront -> line scan: 130 -> 53 us (128 x 66 x 64, FP64, 8
+// slabs), 389 -> 176 us (512 x 130 x 128, FP64), 95 -> 34 us and 251 -> 74 us
+// (FP32); GS sweep of three components without its precomputed terms 280 -> 49 us
+// at 128, 430 -> 301 us at 512 (FP64).
 // A first form with thread-block clusters (st.async into the next CTA's ring)
 // was slower at 512 (243 us): clusters of 15 CTAs doubled up on SMs.  Register
 // prefetch of the operands was slower too (their loads share scoreboards with
@@ -642,16 +645,17 @@ static int line_init(tbl_handle* h) {
     // SSOR: points per lane and planes per CTA.  An FP64 row costs about 65
     // cycles per FMA that a warp issues, so few points per lane spread a line
     // over more of the SM's four FP64 pipes, but every warp pays for the scan.
-    // E = 1 / 2 / 4: 66 / 74 / 94 us at 128 x 66 x 64, 79 / 74 / 94 at
-    // 201 x 77 x 59, 300 / 207 / 214 at 512 x 130 x 128; 244 / 218 (E = 2 / 4)
-    // at 700 x 102 x 100.  FP32 rows are bound by latency: 4 points, and two
-    // planes per CTA save a hand-over (84 / 84 / 88 us with 1 / 2 / 3 at 512);
-    // from five warps a line on, the registers leave one CTA per SM and 8
-    // points are better (4 / 8 points: 198 / 139 at 768 x 194 x 144, 135 / 108
-    // at 600 x 130 x 128, 84 / 89 at 512).
+    // Forward and backward sweep, E = 1 / 2: 100 / 117 us at 128 x 66 x 64,
+    // 116 / 118 at 160 x 66 x 81, 138 / 140 at 201 x 77 x 59, 188 / 173 at
+    // 256 x 98 x 96; 488 / 414 (E = 2 / 4) at 700 x 102 x 100, 352 / 367 at
+    // 512 x 130 x 128.  FP32 rows are bound by latency: 4 points, and two planes
+    // per CTA save a hand-over (one sweep, 84 / 84 / 88 us with 1 / 2 / 3 at
+    // 512 x 130 x 128); from five warps a line on, the registers leave one CTA
+    // per SM and 8 points are better (4 / 8 points: 198 / 139 at 768 x 194 x 144,
+    // 135 / 108 at 600 x 130 x 128, 84 / 89 at 512).
     int E, kp;
     if (sizeof(V) == 8) {
-        E = nx <= 130 ? 1 : nx <= 513 ? 2 : 4;
+        E = nx <= 161 ? 1 : nx <= 513 ? 2 : 4;
         kp = 1;
     } else {
         E = nx <= 513 ? 4 : 8;
