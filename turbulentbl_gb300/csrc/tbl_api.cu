@@ -521,8 +521,7 @@ static int gmres_mixed(tbl_handle* h, std::vector<int32_t>& kits, tbl_step_stats
             }
             {
                 // low-synch MGS: one dot pass over the basis (+1 vector per extra group), one update pass, Givens
-                const int ngr = (k + 7) / 8;
-                ProfScope ps(h, TBL_PROF_MGS, ((k + 2.0 * ngr) + (k + 2.0)) * wN);
+                ProfScope ps(h, TBL_PROF_MGS, (2.0 * k + 4.0) * wN);
                 TRY(launch_lsg_f(h, W, k, skip, thr));
             }
             return TBL_OK;

@@ -79,7 +79,7 @@ struct DevScalars {
     double lamda;
     double lamda03;
     int ksep;
-    int stop;  // set by k_givens when the Arnoldi estimate reaches its target: the kernels
+    int stop;  // set by a Givens rotation when the Arnoldi estimate reaches its target: the kernels
                // of an Arnoldi step enqueued ahead of the host's check then return at once
     // GMRES
     double rho, sumnor, sumav;

@@ -1,7 +1,7 @@
 // tbl_krylov.cu -- GMRES(kmax) building blocks in FP64
-// (dnstbl2/dnstbl.f90:952-1208): modified Gram-Schmidt passes with fused
-// grid reductions, normalisation, Givens rotations and back substitution in
-// one device thread, and the solution update p' += V y.
+// (dnstbl2/dnstbl.f90:952-1208): modified Gram-Schmidt passes over blocks of
+// basis vectors with fused grid reductions, Givens rotations and back
+// substitution in one warp, and the solution update p' += V y.
 //
 // Vector kernels stream the whole padded volume: Krylov vectors are zero
 // outside the interior, so boundary and padding entries add nothing to the dot
@@ -196,9 +196,11 @@ struct Givens {
 // M^-1 A v_k, so c_i = d_i d_k S_i.  The division pass is gone.
 //
 // Bound: two FP64 FMAs per element and basis vector (28.8 us a vector at
-// 512 x 130 x 128 and 600 G FMA/s) and two reads of every basis vector (28 us
-// at 5 TB/s), against 43.6 us a vector with one pass per vector; on small grids
-// the number of launches, a ninth as many.
+// 512 x 130 x 128 and 600 G FMA/s) and two reads of every basis vector (20 us
+// at 6.8 TB/s): 33.4 us a vector at 40 vectors, 43.6 with one pass per vector.
+// On small grids the number of launches, a ninth as many, and what a pass does
+// besides, about 10 us: 145 us at 40 vectors and 128 x 66 x 64, of which 74 are
+// FP64 issue.
 constexpr int GSB = 8;
 struct GsPass {
     long long n2;
@@ -441,7 +443,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_ppe_resid(Geom g, double aw, do
 // ------------------------------------------------ mixed precision (FP32)
 // Inner GMRES vectors are FP32; dot products accumulate in FP64 (the FP32
 // products of 4 consecutive elements are summed in FP32, then added in FP64),
-// and h, g, c, s, y stay FP64 (k_restart_init / k_givens / k_backsub above).
+// and h, g, c, s, y stay FP64 (k_restart_init / Givens / k_backsub above).
 
 __device__ __forceinline__ double dot4(float4 a, float4 b) {
     return (double)fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)));

@@ -576,7 +576,7 @@ static int line_chunks_of(int E, int nx) {
 // Splits the slab columns over CTAs of KP planes for one kernel.  False when
 // the line sweeps do not take the grid: lines of more warps than a CTA may
 // have, or rows that the mailboxes have no room for.
-template <int MODE, typename V>
+template <typename V>
 static bool line_plan(const tbl_handle* h, int rows, int nblk, int E, int kp, LineShape& q) {
     q = LineShape();
     q.E = E;
@@ -591,12 +591,18 @@ static bool line_plan(const tbl_handle* h, int rows, int nblk, int E, int kp, Li
     if (q.KP < 1) return false;
     q.smem = q.KP * plane;
     for (int r = 0; r < h->P; ++r) q.ncta += (h->en[r] - h->bn[r] + 1 + q.KP - 1) / q.KP * nblk;
-    if (cudaFuncSetAttribute((const void*)line_fn<MODE, V>(E), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             LINE_MAX_SMEM) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
     return true;
+}
+
+// Lets the kernel of a plan have its shared memory (and loads it: only the
+// chosen plan's, which tbl_create waits for).
+template <int MODE, typename V>
+static bool line_ready(const LineShape& q) {
+    if (cudaFuncSetAttribute((const void*)line_fn<MODE, V>(q.E), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             LINE_MAX_SMEM) == cudaSuccess)
+        return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 // A Gauss-Seidel launch sweeps three components at once, so its CTAs are
@@ -615,7 +621,7 @@ static bool line_plan_gs(const tbl_handle* h, int rows, int E0, LineShape& q) {
     for (int E = E0; E <= (sizeof(V) == 8 ? 4 : 8); E *= 2)
         for (int kp = sizeof(V) == 8 ? 2 : 3; kp <= 4; ++kp) {
             LineShape t;
-            if (!line_plan<0, V>(h, rows, 1, E, kp, t)) continue;
+            if (!line_plan<V>(h, rows, 1, E, kp, t)) continue;
             const int waves = (3 * t.ncta + h->n_sm - 1) / h->n_sm;
             if (waves < best) {
                 best = waves;
@@ -662,8 +668,9 @@ static int line_init(tbl_handle* h) {
         kp = 2;
     }
     LineShape q[3];
-    const bool ssor = line_plan<1, V>(h, brows, nblk, E, kp, q[1]) && line_plan<2, V>(h, brows, nblk, E, kp, q[2]);
-    const bool gs = line_plan_gs<V>(h, J, E, q[0]);
+    const bool ssor = line_plan<V>(h, brows, nblk, E, kp, q[1]) && line_plan<V>(h, brows, nblk, E, kp, q[2]) &&
+                      line_ready<1, V>(q[1]) && line_ready<2, V>(q[2]);
+    const bool gs = line_plan_gs<V>(h, J, E, q[0]) && line_ready<0, V>(q[0]);
     size_t words = 0;
     for (int m = 0; m < 3; ++m) {
         if (m == 0 ? !gs : !ssor) continue;
