@@ -609,12 +609,14 @@ static bool line_ready(const LineShape& q) {
 // counted in waves of one per SM: a second CTA on an SM shares its FP64 pipes
 // or waits for its registers, and starts its chain late.  The plan takes the
 // fewest waves, and of those the fewest points per lane and then planes per
-// CTA.  FP64, E, KP = 2, 2 / 2, 3 / 4, 2 / 4, 3, us: 124 / 138 / 157 / 160 at
-// 256 x 98 x 96 (one wave each); 195 / 163 / 204 / 191 at 256 x 130 x 128 and
-// 363 / - / 342 / 293 at 512 x 130 x 128 (two, one, two, one).  FP32, 4, 2 /
-// 4, 3 / 8, 3 / 8, 4: 111 / 98 / 101 / 103 at 512 x 130 x 128 (two, one, one,
-// one), 119 / 131 / 116 / 99 at 512 x 102 x 190 (two, two, two, one), and from
-// two planes to three or four the hand-overs saved weigh as much.
+// CTA.  FP64, E, KP = 2, 2 / 2, 3 / 4, 2 / 4, 3, us: 124 / 118 / 139 / 135 at
+// 256 x 98 x 96 (one wave each); 194 / 157 / 203 / 182 at 256 x 130 x 128 and
+// 341 / - / 343 / 300 at 512 x 130 x 128 (two, one, two, one).  FP32, 4, 2 /
+// 4, 3 / 8, 4: 111 / 98 / 103 at 512 x 130 x 128 (two, one, one), 119 / 131 /
+// 99 at 512 x 102 x 190 (two, two, one); from two planes to three or four the
+// hand-overs saved weigh as much.  FP32 lines of four warps or more take 8
+// points (4 / 8: 60 / 64 at 384 x 98 x 96, 95 / 89 at 400 x 130 x 128, 97 / 91 at
+// 512 x 130 x 128).
 template <typename V>
 static bool line_plan_gs(const tbl_handle* h, int rows, int E0, LineShape& q) {
     int best = INT_MAX;
@@ -653,15 +655,16 @@ static int line_init(tbl_handle* h) {
     // over more of the SM's four FP64 pipes, but every warp pays for the scan.
     // Forward and backward sweep, E = 1 / 2: 100 / 117 us at 128 x 66 x 64,
     // 116 / 118 at 160 x 66 x 81, 138 / 140 at 201 x 77 x 59, 188 / 173 at
-    // 256 x 98 x 96; 488 / 414 (E = 2 / 4) at 700 x 102 x 100, 352 / 367 at
-    // 512 x 130 x 128.  FP32 rows are bound by latency: 4 points, and two planes
-    // per CTA save a hand-over (one sweep, 84 / 84 / 88 us with 1 / 2 / 3 at
-    // 512 x 130 x 128); from five warps a line on, the registers leave one CTA
-    // per SM and 8 points are better (4 / 8 points: 198 / 139 at 768 x 194 x 144,
-    // 135 / 108 at 600 x 130 x 128, 84 / 89 at 512).
+    // 256 x 98 x 96; E = 2 / 4: 317 / 356 at 512 x 130 x 128, 341 / 356 at
+    // 700 x 130 x 100, 304 / 276 at 850 x 92 x 90.  FP32 rows are bound by
+    // latency: 4 points, and two planes per CTA save a hand-over (152 / 147 /
+    // 178 with 1 / 2 / 3 at 512 x 130 x 128); from five warps a line on, the
+    // registers leave one CTA per SM and 8 points are better (4 / 8 points:
+    // 316 / 260 at 768 x 194 x 144, 198 / 172 at 600 x 130 x 128, 147 / 153 at
+    // 512).
     int E, kp;
     if (sizeof(V) == 8) {
-        E = nx <= 161 ? 1 : nx <= 513 ? 2 : 4;
+        E = nx <= 161 ? 1 : nx <= 769 ? 2 : 4;
         kp = 1;
     } else {
         E = nx <= 513 ? 4 : 8;
@@ -670,7 +673,7 @@ static int line_init(tbl_handle* h) {
     LineShape q[3];
     const bool ssor = line_plan<V>(h, brows, nblk, E, kp, q[1]) && line_plan<V>(h, brows, nblk, E, kp, q[2]) &&
                       line_ready<1, V>(q[1]) && line_ready<2, V>(q[2]);
-    const bool gs = line_plan_gs<V>(h, J, E, q[0]) && line_ready<0, V>(q[0]);
+    const bool gs = line_plan_gs<V>(h, J, sizeof(V) == 4 && nx > 385 ? 8 : E, q[0]) && line_ready<0, V>(q[0]);
     size_t words = 0;
     for (int m = 0; m < 3; ++m) {
         if (m == 0 ? !gs : !ssor) continue;
