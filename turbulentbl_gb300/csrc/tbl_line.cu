@@ -42,8 +42,8 @@
 // cycles each to issue; a feeder warp does it), selects and tests at its ends.
 // SSOR sweep, wavefront -> line scan: 130 -> 53 us (128 x 66 x 64, FP64, 8
 // slabs), 389 -> 176 us (512 x 130 x 128, FP64), 95 -> 34 us and 251 -> 74 us
-// (FP32); GS sweep of three components without its precomputed terms 280 -> 49 us
-// at 128, 430 -> 301 us at 512 (FP64).
+// (FP32); GS sweep of three components with its precomputed terms 280 -> 64 us
+// at 128, 620 -> 489 us at 512 (FP64).
 // A first form with thread-block clusters (st.async into the next CTA's ring)
 // was slower at 512 (243 us): clusters of 15 CTAs doubled up on SMs.  Register
 // prefetch of the operands was slower too (their loads share scoreboards with

@@ -1,4 +1,4 @@
-// tbl_sync.cuh -- device-side synchronisation primitives of the wavefront
+// tbl_sync.cuh -- device-side synchronisation primitives of the sweep
 // kernels: acquire/release words, bounded mbarrier waits, st.async pushes into
 // another CTA's shared memory and cluster barriers.
 #pragma once
