@@ -132,7 +132,7 @@ static void free_all(tbl_handle* h) {
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
                     h->uold1, h->x3, h->jacinv, h->jac2, h->Ab, h->At, h->Ap, h->rAp, h->gs_coef, h->gs_coef_f, h->lap_scale, h->coef_f, h->ssor_scale, h->line_xch, h->line_ticket, h->line[0].ctas, h->line[1].ctas, h->line[2].ctas, h->usum2, h->vsum2,
                     h->wsum2, h->wt, h->ume1, h->bltkns, h->newk, h->ufl_file, h->ufl_live, h->ufl_full,
-                    h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_nd, h->gs_G, h->gs_hs,
+                    h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_G, h->gs_hs,
                     h->red.partial, h->red.count, h->halo, h->flags, h->ctas, h->slabs, h->err};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -223,7 +223,7 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
         for (int c = 0; c < 3; ++c) { TRY(dalloc(&h->U[c], vol)); TRY(dalloc(&h->Q[c], vol)); }
         TRY(dalloc(&h->Pr, vol)); TRY(dalloc(&h->RH, vol)); TRY(dalloc(&h->PRE, 3 * vol));
         TRY(dalloc(&h->V, vol * (size_t)(cfg->kmax + 1)));
-        TRY(dalloc(&h->gs_d, (size_t)cfg->kmax + 1)); TRY(dalloc(&h->gs_nd, (size_t)cfg->kmax + 1));
+        TRY(dalloc(&h->gs_d, 4 * ((size_t)cfg->kmax + 1)));
         TRY(dalloc(&h->gs_G, 8 * ((size_t)cfg->kmax + 1)));
         TRY(dalloc(&h->gs_hs, (size_t)cfg->kmax + 1));
     }
@@ -601,13 +601,14 @@ int gmres(tbl_handle* h, const int32_t* rec, std::vector<int32_t>& kits, tbl_ste
         int kit = 0;
         const int target = rec ? rec[m] : 0;
         // One Arnoldi step (:1059-1191): preconditioned matvec, MGS, Givens; the
-        // basis vectors are not divided by their norms.  With skip, every kernel returns at once when an
+        // basis vectors are not divided by their norms, but the matvec keeps them in
+        // range by a power of two.  With skip, every kernel returns at once when an
         // earlier step's Givens stopped the cycle.
         auto arnoldi_step = [&](int k, const int* skip) -> int {
             double* W = h->V + (size_t)k * vol;
             {
                 ProfScope ps(h, TBL_PROF_SSOR_FWD, 2.0 * wN);
-                TRY(launch_ssor_fwd(h, h->V + (size_t)(k - 1) * vol, nullptr, skip));
+                TRY(launch_ssor_fwd(h, h->V + (size_t)(k - 1) * vol, nullptr, skip, gs_factor(h, k)));
             }
             {
                 ProfScope ps(h, TBL_PROF_SSOR_BWD, 2.0 * wN);

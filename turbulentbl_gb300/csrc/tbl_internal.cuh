@@ -186,7 +186,8 @@ struct tbl_handle {
     tbl::DevScalars* sc;
     // GMRES small arrays (kmax+1)^2 + 4(kmax+1)
     double *h, *gg, *gc, *gs, *gy;
-    double *gs_d, *gs_nd, *gs_G, *gs_hs;   // FP64 Gram-Schmidt: 1/|v_i|, |v_i|, products inside a block, w's coefficients
+    double *gs_d, *gs_G, *gs_hs;   // FP64 Gram-Schmidt: 4 x (kmax+1) of the norms (GsNorms), products inside a block,
+                                   // w's coefficients
     // reductions
     tbl::RedWork red;
     // wavefront

@@ -30,7 +30,8 @@ int launch_gs_parts(tbl_handle* h, const int* comps, int ncomp, bool pre, bool r
 int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity, bool have_pre);
 int launch_gs_coef(tbl_handle* h);
 int launch_halo_init(tbl_handle* h, int parity);
-int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int* skip = nullptr);
+int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int* skip = nullptr,
+                    const double* factor = nullptr);
 int launch_ssor_bwd(tbl_handle* h, double* out, const int* skip = nullptr);
 int launch_ssor_fwd_f(tbl_handle* h, const float* Xf, const double* PCd, const double* Q8, const int* skip = nullptr,
                       const double* denom = nullptr, float* vout = nullptr);
@@ -44,14 +45,15 @@ int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], const int* com
 template <typename V>
 int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* skip);
 
-// tbl_lap.cu: R = scale(k) L7 X, or scale(k) (Q8 - L7 X) with Q8
-int launch_lap(tbl_handle* h, const double* X, const double* Q8, double* R, const int* skip);
+// tbl_lap.cu: R = factor scale(k) L7 X (no factor: 1), or scale(k) (Q8 - L7 X) with Q8
+int launch_lap(tbl_handle* h, const double* X, const double* Q8, double* R, const int* skip, const double* factor);
 int launch_lap_f(tbl_handle* h, const float* X, float* R, const int* skip, const double* denom, float* vout);
 int launch_lap_resid_f(tbl_handle* h, const double* X, const double* Q8, float* R, const int* skip);
 
 // tbl_krylov.cu
 int launch_dot(tbl_handle* h, const double* a, const double* b, double* out, int op);
 int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at);
+const double* gs_factor(const tbl_handle* h, int k);
 int launch_backsub_update(tbl_handle* h, int kit);
 int launch_restart_init(tbl_handle* h, int first);
 int launch_ppe_resid(tbl_handle* h);

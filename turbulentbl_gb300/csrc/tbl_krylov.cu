@@ -181,10 +181,25 @@ struct Givens {
     }
 };
 
+// What the FP64 Gram-Schmidt keeps of a basis vector's norm: d = 1/|v|, and with
+// p the power of two of 1 <= p |v| < 2 (exact scalings), ds = d / p, ns = p |v|, p.
+struct GsNorms {
+    double *d, *ds, *ns, *p;
+    __device__ __forceinline__ void set(int i, double norm, double rec) const {  // rec = 1 / norm
+        if (!(norm > 0.0)) norm = rec = 1.0;
+        const int e = min(max((__double2hiint(norm) >> 20) & 0x7ff, 1), 2045);  // norm = m 2^(e - 1023)
+        const double up = __hiloint2double((2046 - e) << 20, 0), down = __hiloint2double(e << 20, 0);
+        d[i] = rec;
+        ds[i] = rec * down;
+        ns[i] = norm * up;
+        p[i] = up;
+    }
+};
+
 // ---------------------------------------------------- Gram-Schmidt (FP64)
 // Modified Gram-Schmidt (:1140-1161) over blocks of 8 basis vectors.  One pass
 // takes a block's projections off w and forms the next block's dot products:
-//   w -= sum_i (h_i d_i / d_k) v_i   (i in the previous block)
+//   w -= sum_i (h_i d_i p_k / d_k) v_i   (i in the previous block)
 //   S_i = <v_i, w>                   (i in the next block), or <w, w> at the end
 // Inside a block the dots are all taken against the same w; the modified
 // Gram-Schmidt coefficients follow from h_i = c_i - sum_{j<i} <v_i, v_j> h_j,
@@ -193,7 +208,10 @@ struct Givens {
 // when the basis has lost orthogonality).
 // The basis vectors are kept as they come out of this, not divided by their
 // norms: v_i d_i with d_i = 1 / |v_i| is the reference's unit vector, and w =
-// M^-1 A v_k, so c_i = d_i d_k S_i.  The division pass is gone.
+// p_k M^-1 A v_k with p_k the power of two that brings |v_k| between 1 and 2, so
+// c_i = d_i (d_k / p_k) S_i.  The division pass is gone.  The powers of two change
+// no bit of the result; without them |v_k| is the product of the subdiagonal
+// values, about 0.3 each, and its square is zero after some 300 vectors.
 //
 // Bound: two FP64 FMAs per element and basis vector (28.8 us a vector at
 // 512 x 130 x 128 and 600 G FMA/s) and two reads of every basis vector (20 us
@@ -208,8 +226,9 @@ struct GsPass {
     const double2* V;      // basis, n2 apart
     int p0, q0;            // first vector of the previous and of the next block
     int k;                 // vectors in the basis
-    double *d, *nd, *G;    // 1/|v_i|; |v_i|; <v_i, v_j> / (|v_i| |v_j|), j in i's block, [i][GSB]
-    double *hcol, *hs;     // Hessenberg column; h_i d_i / d_k
+    GsNorms n;
+    double* G;             // <v_i, v_j> / (|v_i| |v_j|), j in i's block, [i][GSB]
+    double *hcol, *hs;     // Hessenberg column; h_i d_i p_k / d_k
     double* partial;       // [16][max_blocks]
     unsigned* count;
     int max_blocks;
@@ -278,12 +297,12 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     double di = 0.0, dk = 0.0, nk = 0.0, grow[GSB];
     Givens gv = {a.k, a.h + (size_t)a.K1 * (a.k - 1), a.gg, a.gc, a.gs, a.sc, a.skip != nullptr, a.stop_at};
     if (wid == 0) {
-        dk = a.d[a.k - 1];
-        nk = a.nd[a.k - 1];
+        dk = a.n.ds[a.k - 1];
+        nk = a.n.ns[a.k - 1];
         if (NQ == 0) {
             gv.prefetch();
         } else {
-            di = lane < NQ ? a.d[i] : 0.0;
+            di = lane < NQ ? a.n.d[i] : 0.0;
 #pragma unroll
             for (int j = 0; j < GSB - 1; ++j)  // this lane's row of the block's products
                 grow[j] = lane < NQ - GRAM && j < lane ? a.G[(size_t)i * GSB + j] : 0.0;
@@ -310,7 +329,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
             for (int j = 0; j < NQ - 1; ++j) {
                 const double dj = __shfl_sync(0xffffffffu, di, j);
                 if (lane == NQ - 1) {
-                    grow[j] = dj * dk * s_val[8 + j];
+                    grow[j] = dj * di * s_val[8 + j];
                     a.G[(size_t)i * GSB + j] = grow[j];
                 }
             }
@@ -324,19 +343,16 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_gs_pass(const GsPass a) {
     } else {
         const double nh = sqrt(s_val[0]);
         const double r = gv.column(dk * nh, nh);
-        if (lane == 0) {
-            a.d[a.k] = nh > 0.0 ? r : 1.0;
-            a.nd[a.k] = nh > 0.0 ? nh : 1.0;
-        }
+        if (lane == 0) a.n.set(a.k, nh, r);
     }
     if (lane == 0) *a.count = 0u;
 }
 
 // Start of a restart (:958-963, :1048-1056): zero h, c, s, g, y; g(1) = rho;
 // sumnor at the first restart; sumav = rho/sumnor.
-// d, nd: 1/|v_i| and |v_i| of the basis vectors, kept as they come (FP64), or null.
+// n: what is kept of the norms of basis vectors kept as they come (FP64), or nulls.
 __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double* gs, double* gy, DevScalars* sc,
-                               int first, double* d, double* nd) {
+                               int first, GsNorms n) {
     for (int q = threadIdx.x; q < K1 * K1; q += blockDim.x) h[q] = 0.0;
     for (int q = threadIdx.x; q < K1; q += blockDim.x) { gg[q] = 0.0; gc[q] = 0.0; gs[q] = 0.0; gy[q] = 0.0; }
     __syncthreads();
@@ -346,10 +362,7 @@ __global__ void k_restart_init(int K1, double* h, double* gg, double* gc, double
         if (first) sc->sumnor = rho;
         sc->sumav = rho / sc->sumnor;
         gg[0] = rho;
-        if (d) {
-            d[0] = rho > 0.0 ? 1.0 / rho : 1.0;
-            nd[0] = rho > 0.0 ? rho : 1.0;
-        }
+        if (n.d) n.set(0, rho, 1.0 / rho);
     }
 }
 
@@ -529,6 +542,14 @@ static void (*gs_last(int n))(const GsPass) {
     }
 }
 
+static GsNorms gs_norms(const tbl_handle* h) {
+    const size_t n = (size_t)h->cfg.kmax + 1;
+    return {h->gs_d, h->gs_d + n, h->gs_d + 2 * n, h->gs_d + 3 * n};
+}
+
+// The factor of step k's matvec (k >= 1).
+const double* gs_factor(const tbl_handle* h, int k) { return gs_norms(h).p + (k - 1); }
+
 // Orthogonalises w against the k vectors of the basis, then the Givens rotation
 // of the column.
 int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) {
@@ -538,8 +559,7 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
     a.V = (const double2*)h->V;
     a.k = k;
     a.K1 = h->cfg.kmax + 1;
-    a.d = h->gs_d;
-    a.nd = h->gs_nd;
+    a.n = gs_norms(h);
     a.G = h->gs_G;
     a.hs = h->gs_hs;
     a.h = h->h;
@@ -569,7 +589,7 @@ int launch_gs(tbl_handle* h, double* w, int k, const int* skip, double stop_at) 
 
 int launch_restart_init(tbl_handle* h, int first) {
     const int K1 = h->cfg.kmax + 1;
-    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, h->gs_d, h->gs_nd);
+    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, gs_norms(h));
     h->launches++;
     return TBL_OK;
 }
@@ -838,7 +858,7 @@ int launch_backsub_update_f(tbl_handle* h, int kit) {
 }
 
 int launch_restart_init_k(tbl_handle* h, int first, int K1) {
-    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, nullptr, nullptr);
+    k_restart_init<<<1, 256, 0, h->stream>>>(K1, h->h, h->gg, h->gc, h->gs, h->gy, h->sc, first, GsNorms());
     h->launches++;
     return TBL_OK;
 }

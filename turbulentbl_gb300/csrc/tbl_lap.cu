@@ -48,14 +48,15 @@ __device__ __forceinline__ void lap_store(float* p, const float (&v)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-// RESID: Q8 - L7 X.  NORM: X is divided by *denom and written to vout.
+// RESID: Q8 - L7 X.  NORM: X is divided by *denom and written to vout.  factor
+// multiplies the coefficients of L7 X.
 template <typename TI, typename TO, typename TC, bool RESID, bool NORM>
 __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double as, const double* __restrict__ Ab,
                                                        const double* __restrict__ At, const double* __restrict__ Ap,
                                                        const double* __restrict__ scale, int kc,
                                                        const TI* X, const double* Q8, TO* __restrict__ R,
                                                        const int* skip, const double* denom,
-                                                       TI* __restrict__ vout) {
+                                                       const double* factor, TI* __restrict__ vout) {
     constexpr int VEC = 16 / sizeof(TI);
     constexpr unsigned ALL = 0xffffffffu;
     __shared__ TC s_c[LAP_KC][6];  // s Ab, s At, s Ap, s aw, s as, s
@@ -66,7 +67,11 @@ __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double
         s_c[q / 6][c] = (TC)(s * (c == 0 ? Ab[k] : c == 1 ? At[k] : c == 2 ? Ap[k] : c == 3 ? aw : c == 4 ? as : 1.0));
     }
     dependent_wait(X);
+    constexpr bool SCALED = sizeof(TI) == 8 && !RESID && !NORM;
+    const double up = SCALED && factor ? *factor : 1.0;  // known by the time the skip word is
     if (skip && *skip) return;  // an Arnoldi step enqueued ahead of a converged one
+    if (SCALED && factor)  // each thread its own entries
+        for (int q = threadIdx.y * 32 + lane; q < 6 * kc; q += 32 * LAP_ROWS) s_c[q / 6][q % 6] *= (TC)up;
     __shared__ TC s_rs;
     if (NORM && threadIdx.y == LAP_ROWS - 1) {  // one warp: an FP64 division keeps its pipe for 1000 cycles
         const double d = *denom;
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double
 
 template <typename TI, typename TO, typename TC>
 static int lap(tbl_handle* h, const TI* X, const double* Q8, TO* R, const double* scale, const int* skip,
-               const double* denom, TI* vout) {
+               const double* denom, const double* factor, TI* vout) {
     const Geom& g = h->g;
     const int vec = 16 / (int)sizeof(TI), planes = g.nz - 2;
     const unsigned gx = (unsigned)((g.nx - 2) / (32 * vec) + 1), gy = (unsigned)((g.ny - 2 + LAP_ROWS - 1) / LAP_ROWS);
@@ -155,25 +160,26 @@ static int lap(tbl_handle* h, const TI* X, const double* Q8, TO* R, const double
     const int kc = (int)std::min((long long)LAP_KC, (planes + want - 1) / want);
     const double aw = 1.0 / (h->cfg.dx * h->cfg.dx), as = 1.0 / (h->cfg.dy * h->cfg.dy);
     void (*fn)(Geom, double, double, const double*, const double*, const double*, const double*, int, const TI*,
-               const double*, TO*, const int*, const double*, TI*);
+               const double*, TO*, const int*, const double*, const double*, TI*);
     if constexpr (sizeof(TI) == 4) fn = denom ? k_lap<TI, TO, TC, false, true> : k_lap<TI, TO, TC, false, false>;
     else if constexpr (sizeof(TO) == 4) fn = k_lap<TI, TO, TC, true, false>;
     else fn = Q8 ? k_lap<TI, TO, TC, true, false> : k_lap<TI, TO, TC, false, false>;
     TBL_CUDA_TRY(launch_dependent(fn, dim3(gx, gy, (unsigned)((planes + kc - 1) / kc)), dim3(32, LAP_ROWS), 0, h->stream,
-                                  g, aw, as, h->Ab, h->At, h->Ap, scale, kc, X, Q8, R, skip, denom, vout));
+                                  g, aw, as, h->Ab, h->At, h->Ap, scale, kc, X, Q8, R, skip, denom, factor, vout));
     h->launches++;
     return TBL_OK;
 }
 
-int launch_lap(tbl_handle* h, const double* X, const double* Q8, double* R, const int* skip) {
-    return lap<double, double, double>(h, X, Q8, R, h->ssor_scale, skip, nullptr, nullptr);
+int launch_lap(tbl_handle* h, const double* X, const double* Q8, double* R, const int* skip, const double* factor) {
+    if (Q8 && factor) return TBL_ERR_BAD_ARG;
+    return lap<double, double, double>(h, X, Q8, R, h->ssor_scale, skip, nullptr, factor, nullptr);
 }
 int launch_lap_f(tbl_handle* h, const float* X, float* R, const int* skip, const double* denom, float* vout) {
     if ((denom == nullptr) != (vout == nullptr) || (vout && vout == X)) return TBL_ERR_BAD_ARG;
-    return lap<float, float, float>(h, X, nullptr, R, h->ssor_scale, skip, denom, vout);
+    return lap<float, float, float>(h, X, nullptr, R, h->ssor_scale, skip, denom, nullptr, vout);
 }
 int launch_lap_resid_f(tbl_handle* h, const double* X, const double* Q8, float* R, const int* skip) {
-    return lap<double, float, double>(h, X, Q8, R, h->ssor_scale, skip, nullptr, nullptr);
+    return lap<double, float, double>(h, X, Q8, R, h->ssor_scale, skip, nullptr, nullptr, nullptr);
 }
 
 }  // namespace tbl

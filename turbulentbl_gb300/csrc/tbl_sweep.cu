@@ -964,8 +964,9 @@ static int launch_gs_sweep_chunk(tbl_handle* h, const int* comps, int ncomp, int
 }
 
 // Forward SSOR sweep of r = L7 X (Q8 == nullptr) or r = Q8 - L7 X.
-int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int* skip) {
-    const int st = launch_lap(h, X, Q8, h->RH, skip);
+// factor: a power of two for r of an Arnoldi step (the sweeps are linear).
+int launch_ssor_fwd(tbl_handle* h, const double* X, const double* Q8, const int* skip, const double* factor) {
+    const int st = launch_lap(h, X, Q8, h->RH, skip, factor);
     if (st != TBL_OK) return st;
     if (h->cfg.flags & TBL_FLAG_RB_PRECOND) return TBL_OK;  // the red-black passes run in launch_ssor_bwd
     if (h->line[SW_FWD].S > 0) return launch_line_ssor<double>(h, false, h->RH, h->RH, skip);
