@@ -42,7 +42,7 @@ extern "C" {
 #define TBL_ERR_NOT_CONVERGED -3  /* GS or GMRES hit mmax (reference continues silently) */
 #define TBL_ERR_NAN           -4  /* NaN/Inf found in the state after a step */
 #define TBL_ERR_BLOWUP        -5  /* u',v' or w' > 25 (reference STOP, dnstbl2/dnstbl.f90:1749-1775) */
-#define TBL_ERR_TIMEOUT       -6  /* a bounded device wait gave up */
+#define TBL_ERR_TIMEOUT       -6  /* a bounded device wait gave up; so does every later step of the handle */
 #define TBL_ERR_NO_DEVICE     -7  /* no CUDA device / library built without it */
 #define TBL_ERR_REPLAY        -8  /* replay counts exhausted or inconsistent */
 #define TBL_ERR_ZERO_RHS      -9  /* zero preconditioned PPE residual at restart 1 (reference divides by zero) */
@@ -366,6 +366,14 @@ int64_t tbl_launch_count(tbl_handle* h);
  * device stays usable.  Returns TBL_OK when the self-test itself ran;
  * *seconds (may be NULL) receives the time the wait took. */
 int tbl_selftest_bounded_wait(int32_t* observed, double* seconds);
+
+/* The same with a handle: one warp waits with the line-scan sweeps' bounded waits,
+ * which = 0 at a shared-memory barrier, 1 for a row of the plane below, 2 for the
+ * carry of the segment before, for what nobody brings, and reports through the
+ * handle's error word, as a stalled sweep does.  The handle reports
+ * TBL_ERR_TIMEOUT from then on: destroy it.  TBL_ERR_BAD_ARG for another `which`
+ * and for handles whose sweeps are not line scans. */
+int tbl_selftest_sweep_wait(tbl_handle* h, int32_t which, int32_t* observed, double* seconds);
 
 /* ------------------------------------------------------------ restart files
  * Host-only readers and writers of the reference's restart files (no device,

@@ -1,6 +1,7 @@
 // tbl_api.cu -- the C ABI (include/tbl_gpu.h): handle lifecycle, state
 // transfer and the per-step driver that sequences the kernels in the order
 // of the reference time loop (dnstbl2/dnstbl.f90:538-2375).
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1079,6 +1080,19 @@ int tbl_selftest_bounded_wait(int32_t* observed, double* seconds) {
     const int st = tbl::selftest_bounded_wait(&v, seconds);
     *observed = v;
     return st;
+}
+
+int tbl_selftest_sweep_wait(tbl_handle* h, int32_t which, int32_t* observed, double* seconds) {
+    if (!h || !observed) return TBL_ERR_BAD_ARG;
+    TBL_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    const auto t0 = std::chrono::steady_clock::now();
+    TRY(line_selftest(h, which));
+    TBL_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (seconds) *seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    int v = 0;
+    TBL_CUDA_TRY(cudaMemcpy(&v, h->err, sizeof(int), cudaMemcpyDeviceToHost));
+    *observed = v;
+    return TBL_OK;
 }
 
 }  // extern "C"

@@ -40,6 +40,7 @@ int selftest_bounded_wait(int* observed, double* seconds);
 
 // tbl_line.cu: line-scan sweeps, where h->line[mode].S > 0
 int line_create(tbl_handle* h);
+int line_selftest(tbl_handle* h, int which);
 template <typename V>
 int launch_line_gs(tbl_handle* h, V* const F[3], V* const PRE[3], const int* comps, int ncomp);
 template <typename V>

@@ -68,10 +68,13 @@ __global__ void __launch_bounds__(32 * LAP_ROWS) k_lap(Geom g, double aw, double
     }
     dependent_wait(X);
     constexpr bool SCALED = sizeof(TI) == 8 && !RESID && !NORM;
-    const double up = SCALED && factor ? *factor : 1.0;  // known by the time the skip word is
+    const int up = SCALED && factor ? __double2hiint(*factor) - 0x3ff00000 : 0;  // known when the skip word is
     if (skip && *skip) return;  // an Arnoldi step enqueued ahead of a converged one
-    if (SCALED && factor)  // each thread its own entries
-        for (int q = threadIdx.y * 32 + lane; q < 6 * kc; q += 32 * LAP_ROWS) s_c[q / 6][q % 6] *= (TC)up;
+    if (SCALED && factor)  // each thread its own entries; in the exponent, an FP64 product a warp costs 64 cycles
+        for (int q = threadIdx.y * 32 + lane; q < 6 * kc; q += 32 * LAP_ROWS) {
+            const double c = s_c[q / 6][q % 6];
+            if (c != 0.0) s_c[q / 6][q % 6] = (TC)__hiloint2double(__double2hiint(c) + up, __double2loint(c));
+        }
     __shared__ TC s_rs;
     if (NORM && threadIdx.y == LAP_ROWS - 1) {  // one warp: an FP64 division keeps its pipe for 1000 cycles
         const double d = *denom;

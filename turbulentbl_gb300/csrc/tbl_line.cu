@@ -29,8 +29,10 @@
 //
 // CTAs take their planes by ticket, the lowest planes of all slabs first, so
 // that a CTA only ever waits for CTAs that have started: the launch needs no
-// co-residency.  All waits are bounded; a wait that gives up sets the error
-// word and the warps that depend on it give up in turn.
+// co-residency.  All waits are bounded (about a second); a wait that gives up
+// sets the error word and the warps that depend on it give up in turn.  Rows it
+// did not take stay in the exchange buffer, so the error word is never cleared:
+// a handle that has timed out reports it from then on.
 //
 // What bounds it: the serial chain of J + K rows.  An FP64 row with 1 point per
 // lane takes about 900 cycles at 128 x 66 x 64, of which 320 are the scan (an
@@ -193,6 +195,34 @@ __host__ __device__ constexpr int line_chunks(int nx) {
     return ((nx - 2) / E + 1 + M - 1) / M * M;
 }
 
+template <typename V, int E>
+__device__ __forceinline__ bool line_arrived(const V (&w)[E]) {
+    bool have = true;
+#pragma unroll
+    for (int e = 0; e < E; ++e) have = have && !line_empty(w[e]);
+    return have;
+}
+// A courier's wait for one segment of a row of the plane below.
+template <typename V, int E>
+__device__ __forceinline__ bool xch_wait(V (&w)[E], const V* p) {
+    bool good = true;
+    for (long long spins = 0; good;) {
+        xch_ld(w, p);
+        if (__all_sync(0xffffffffu, line_arrived(w))) break;
+        good = ++spins < SPIN_LIMIT / 16;
+    }
+    return good;
+}
+// A warp's wait for the carry into its segment.
+template <typename V>
+__device__ __forceinline__ bool carry_wait(V& c, const volatile V* p) {
+    for (long long spins = 0; spins < SPIN_LIMIT; ++spins) {
+        c = *p;
+        if (!__any_sync(0xffffffffu, line_empty(c))) return true;
+    }
+    return false;
+}
+
 template <int MODE, typename V, int E>
 __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 1), 1) k_line(const LineArgs<V> a) {
     dependent_wait();
@@ -288,12 +318,6 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
         V none[E];
 #pragma unroll
         for (int e = 0; e < E; ++e) none[e] = B::empty();
-        auto arrived = [&](const V(&w)[E]) {
-            bool have = true;
-#pragma unroll
-            for (int e = 0; e < E; ++e) have = have && !line_empty(w[e]);
-            return have;
-        };
         auto hand = [&](int r, int sg, const V(&w)[E]) {
             const int u = r & (XR - 1);
             line_store<V, E>(rings + (((size_t)sg * XR + u) * 64 + 32 + lane) * E, w, false);
@@ -308,11 +332,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
                 if ((r & (H - 1)) == 0 && r >= XR)
                     good = __all_sync(ALL, mbar_wait(&fb[(r & (XR - 1)) / H], (unsigned)(r / XR - 1) & 1u));
                 V w[E];
-                for (long long spins = 0; good;) {
-                    xch_ld(w, src + r * xrow + (size_t)sg0 * 32 * E);
-                    if (__all_sync(ALL, arrived(w))) break;
-                    good = ++spins < SPIN_LIMIT / 16;
-                }
+                if (good) good = xch_wait<V, E>(w, src + r * xrow + (size_t)sg0 * 32 * E);
                 if (good) hand(r, sg0, w);
             }
         } else if (has) {
@@ -336,7 +356,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
                 for (int c = 0; c < CS; ++c) {
                     if (row[c] >= nrow) continue;
                     const int r = row[c], u = r & (XR - 1), sg = sg0 + c * a.NC;
-                    bool have = arrived(w[c]);
+                    bool have = line_arrived(w[c]);
                     if ((u & (H - 1)) == 0 && r >= XR)
                         have = mbar_test(bars + sg * LINE_BARS + XR + u / H, (unsigned)(r / XR - 1) & 1u) && have;
                     if (__all_sync(ALL, have)) {
@@ -494,11 +514,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
             const bool rdy = ask(s1, ph1, gr);  // (after the last row: what a slot holds, and not used)
             // the carry of the segment before
             if (seg > 0) {
-                long long spins = 0;
-                while (__any_sync(ALL, line_empty(c)) && !dead) {
-                    if (++spins > SPIN_LIMIT) dead = true;
-                    c = prev_mail[r];
-                }
+                if (__any_sync(ALL, line_empty(c)) && !dead && !carry_wait(c, &prev_mail[r])) dead = true;
                 b = fma(acar, c, b);
             }
             if (seg < S - 1 && lane == 31) my_mail[r] = line_value(b);
@@ -557,6 +573,31 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
         a.ticket[0] = 0u;
         a.ticket[1] = 0u;
     }
+}
+
+// One warp waits as the sweeps do, at a barrier (which = 0), for a row of the plane
+// below (1) or for a carry (2), for what nobody brings.
+template <typename V>
+__global__ void __launch_bounds__(32) k_line_wait(int which, V* word, int* err) {
+    constexpr int E = sizeof(V) == 8 ? 1 : 4;
+    __shared__ unsigned long long s_bar;
+    __shared__ V s_mail;
+    if (threadIdx.x == 0) {
+        mbar_init(&s_bar, 1);
+        s_mail = LineBits<V>::empty();
+    }
+    __syncwarp();
+    bool got;
+    if (which == 0) {
+        got = mbar_wait(&s_bar, 0);
+    } else if (which == 1) {
+        V w[E];
+        got = xch_wait<V, E>(w, word + threadIdx.x * E);
+    } else {
+        V c;
+        got = carry_wait(c, &s_mail);
+    }
+    if (!got && threadIdx.x == 0) atomicExch(err, TBL_ERR_TIMEOUT);
 }
 
 // ------------------------------------------------------------------ host
@@ -745,6 +786,16 @@ int launch_line_ssor(tbl_handle* h, bool bwd, const V* in, V* out, const int* sk
         a.cb = (C + h->ssor_nib - 1) / h->ssor_nib * (ch / q.E);
     }
     return bwd ? line_launch<2, V>(h, q, a, 1) : line_launch<1, V>(h, q, a, 1);
+}
+
+// The exchange buffer holds no row between launches.
+int line_selftest(tbl_handle* h, int which) {
+    if (which < 0 || which > 2 || !h->line_xch) return TBL_ERR_BAD_ARG;
+    if (h->cfg.precision == TBL_PREC_MIXED) k_line_wait<float><<<1, 32, 0, h->stream>>>(which, (float*)h->line_xch, h->err);
+    else k_line_wait<double><<<1, 32, 0, h->stream>>>(which, (double*)h->line_xch, h->err);
+    TBL_CUDA_TRY(cudaGetLastError());
+    h->launches++;
+    return TBL_OK;
 }
 
 template int launch_line_gs<double>(tbl_handle*, double* const[3], double* const[3], const int*, int);
