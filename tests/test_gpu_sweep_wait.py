@@ -43,3 +43,42 @@ def test_a_wait_of_the_sweeps_gives_up(which, mixed):
     g.upload(st)
     assert g.step(1, check=False)[0] == abi.TBL_OK
     g.close()
+
+
+def test_a_timeout_is_reported_by_the_backward_window():
+    """The adjoint's sweeps run after the window's last step: the error word is
+    read with their own residuals."""
+    from turbulentbl_gb300.lib import TblGpu
+    from turbulentbl_gb300.runner import TblError
+    wl = small_workload(nx=24, nz_span=8, ny_wall=14, kmax=20)
+    mesh, rp, st = make_state(wl, nproc=2)
+    rp.cum = 50
+    g = TblGpu(mesh, rp)
+    g.upload(st)
+    x = mesh.dx * mesh.nx
+    g.forward_window(2, 0.25 * x, 0.75 * x, 2)
+    g.backward_window()
+    assert give_up(g, 1)[:2] == (abi.TBL_OK, abi.TBL_ERR_TIMEOUT)
+    with pytest.raises(TblError) as e:
+        g.backward_window()
+    assert e.value.status == abi.TBL_ERR_TIMEOUT
+    g.close()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_a_timeout_is_not_taken_for_a_nan(mixed):
+    from turbulentbl_gb300.lib import TblGpu
+    wl = small_workload(nx=24, nz_span=8, ny_wall=14, kmax=20)
+    mesh, rp, st = make_state(wl, nproc=2)
+    rp.mmax = 20
+    if mixed:
+        rp.precision = abi.TBL_PREC_MIXED
+    st["u"] = st["u"].copy(order="F")
+    st["u"][5, 5, 5] = float("nan")
+    g = TblGpu(mesh, rp)
+    g.upload(st)
+    assert g.step(1, check=False)[0] == abi.TBL_ERR_NAN
+    assert give_up(g, 1)[:2] == (abi.TBL_OK, abi.TBL_ERR_TIMEOUT)
+    g.upload(st)
+    assert g.step(1, check=False)[0] == abi.TBL_ERR_TIMEOUT
+    g.close()

@@ -62,6 +62,13 @@ int readback(tbl_handle* h, const void* dev, size_t bytes) {
     return TBL_OK;
 }
 
+// The device's error word as it came back with other scalars.
+static int wait_status(const double* word) {
+    int err;
+    memcpy(&err, word, sizeof(err));
+    return err;
+}
+
 // 3-D host (nx,ny,nz) <-> device (sx,ny,nz)
 int put3(tbl_handle* h, double* dst, const double* src) {
     const Geom& g = h->g;
@@ -134,7 +141,7 @@ static void free_all(tbl_handle* h) {
                     h->uold1, h->x3, h->jacinv, h->jac2, h->Ab, h->At, h->Ap, h->rAp, h->gs_coef, h->gs_coef_f, h->lap_scale, h->coef_f, h->ssor_scale, h->line_xch, h->line_ticket, h->line[0].ctas, h->line[1].ctas, h->line[2].ctas, h->usum2, h->vsum2,
                     h->wsum2, h->wt, h->ume1, h->bltkns, h->newk, h->ufl_file, h->ufl_live, h->ufl_full,
                     h->usum2_fl, h->sums, h->avg, h->bl_out, h->ubulk, h->sumxz, h->tauw_win, h->slab_of_k, h->sc, h->h, h->gg, h->gc, h->gs, h->gy, h->gs_d, h->gs_G, h->gs_hs,
-                    h->red.partial, h->red.count, h->halo, h->flags, h->ctas, h->slabs, h->err};
+                    h->red.partial, h->red.count, h->halo, h->flags, h->ctas, h->slabs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     adj_free(h);
@@ -252,7 +259,7 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
     TRY(dalloc(&h->red.partial, (size_t)16 * h->red.max_blocks));
     TRY(dalloc(&h->red.count, (size_t)24));
     TRY(dalloc(&h->halo, (size_t)2 * 3 * 2 * h->P * g.ps));
-    TRY(dalloc(&h->err, 1));
+    h->err = &h->sc->err;
     // mesh and per-k coefficients (:487-536); An* == Av*
     std::vector<double> x3(mesh->x3, mesh->x3 + nz), jinv(nz), j2(mesh->jac2, mesh->jac2 + nz);
     std::vector<double> Ab(nz, 0.0), At(nz, 0.0), Ap(nz, 0.0), rAp(nz, 0.0);
@@ -354,8 +361,9 @@ int gs_solve(tbl_handle* h, const int* target, tbl_step_stats& st, bool zero_ok)
                 ProfScope ps(h, TBL_PROF_GS_RESID, (line ? 3.0 : 2.0) * 8.0 * h->npts * n);
                 TRY(launch_gs_parts(h, comps, n, line, true));  // with what the next sweep needs
             }
-            TRY(readback(h, &h->sc->red[0], 3 * sizeof(double)));
-            const double* red = h->hpin;
+            TRY(readback(h, &h->sc->err, 4 * sizeof(double)));
+            TRY(wait_status(h->hpin));
+            const double* red = h->hpin + 1;
             int m = 0;
             bool restarted = false;
             for (int q = 0; q < n; ++q) {
@@ -415,8 +423,8 @@ template <typename Step>
 static int arnoldi_ahead(tbl_handle* h, int kmax, double stop_at, Step& step, int& kit, double& sumav) {
     const int* skip = &h->sc->stop;
     auto post = [&](int k) -> int {
-        TBL_CUDA_TRY(cudaMemcpyAsync(h->hpin + 64 + (k & 1), &h->sc->sumav, sizeof(double), cudaMemcpyDeviceToHost,
-                                     h->stream));
+        TBL_CUDA_TRY(cudaMemcpyAsync(h->hpin + 64 + 2 * (k & 1), &h->sc->sumav, 2 * sizeof(double),
+                                     cudaMemcpyDeviceToHost, h->stream));
         TBL_CUDA_TRY(cudaEventRecord(h->ahead_ev[k & 1], h->stream));
         return TBL_OK;
     };
@@ -430,7 +438,8 @@ static int arnoldi_ahead(tbl_handle* h, int kmax, double stop_at, Step& step, in
             TRY(post(k + 1));
         }
         TBL_CUDA_TRY(cudaEventSynchronize(h->ahead_ev[k & 1]));
-        sumav = h->hpin[64 + (k & 1)];
+        sumav = h->hpin[64 + 2 * (k & 1)];
+        TRY(wait_status(h->hpin + 65 + 2 * (k & 1)));
         if (!(sumav > stop_at) || !more) {
             kit = k;
             if (more)
@@ -483,6 +492,7 @@ static int gmres_mixed(tbl_handle* h, std::vector<int32_t>& kits, tbl_step_stats
         }
         TRY(launch_restart_init_k(h, m == 1, K1));
         TRY(readback(h, &h->sc->rho, 4 * sizeof(double)));
+        TRY(wait_status(h->hpin + 3));
         const double rho_m = h->hpin[0];
         if (m == 1) {
             if (std::isnan(rho_m)) { status = TBL_ERR_NAN; break; }
@@ -531,7 +541,8 @@ static int gmres_mixed(tbl_handle* h, std::vector<int32_t>& kits, tbl_step_stats
             while (kit < kmax && sumav > thr) {
                 kit = kit + 1;
                 TRY(arnoldi_step(kit, nullptr));
-                TRY(readback(h, &h->sc->sumav, sizeof(double)));
+                TRY(readback(h, &h->sc->sumav, 2 * sizeof(double)));
+                TRY(wait_status(h->hpin + 1));
                 sumav = h->hpin[0];
             }
         } else if (kmax > 0 && sumav > thr) {
@@ -594,7 +605,8 @@ int gmres(tbl_handle* h, const int32_t* rec, std::vector<int32_t>& kits, tbl_ste
             TRY(launch_dot(h, V0, V0, &h->sc->rho, 1));
         }
         TRY(launch_restart_init(h, m == 1));
-        TRY(readback(h, &h->sc->rho, 4 * sizeof(double)));  // rho, sumnor, sumav
+        TRY(readback(h, &h->sc->rho, 4 * sizeof(double)));  // rho, sumnor, sumav, err
+        TRY(wait_status(h->hpin + 3));
         double rho = h->hpin[0];
         if (m == 1 && std::isnan(rho)) { status = TBL_ERR_NAN; break; }
         if (m == 1 && !(rho > 0.0)) { status = TBL_ERR_ZERO_RHS; break; }
@@ -626,7 +638,8 @@ int gmres(tbl_handle* h, const int32_t* rec, std::vector<int32_t>& kits, tbl_ste
             while (rec ? (kit < target) : ((sumav > h->cfg.errtol) && (kit < kmax))) {
                 kit = kit + 1;
                 TRY(arnoldi_step(kit, nullptr));
-                TRY(readback(h, &h->sc->sumav, sizeof(double)));
+                TRY(readback(h, &h->sc->sumav, 2 * sizeof(double)));
+                TRY(wait_status(h->hpin + 1));
                 sumav = h->hpin[0];
             }
         } else if (sumav > h->cfg.errtol && kmax > 0) {
@@ -731,13 +744,11 @@ int one_step(tbl_handle* h, tbl_step_stats* out) {
         if (fluc && sete) TRY(fluc_ke());
     }
     h->cnt2 = h->cnt2 + 1;  // end of the step (fnldnstbl.f90:2382, dnstbl.f90:2349)
-    // scalars back: red[3] div, red[4] KE, red[5] max fluct, lamda, err
+    // scalars back: red[3] div, red[4] KE, red[5] max fluct, lamda
     TRY(readback(h, h->sc, sizeof(DevScalars)));
     if (h->prof_on) TRY(prof_drain(h));
     DevScalars sc;
     memcpy(&sc, h->hpin, sizeof(sc));
-    int err = 0;
-    TBL_CUDA_TRY(cudaMemcpy(&err, h->err, sizeof(int), cudaMemcpyDeviceToHost));
     st.div_diag = std::fabs(sc.red[3]) / ((double)(c.ny - 2) * (c.nx - 2) * (c.nz - 2));
     if (c.variant == TBL_VARIANT_ORIGINAL) st.div_diag = std::sqrt(st.div_diag);  // fnldnstbl.f90:1586
     st.ke = fluc ? sc.red[4] / ((double)c.nx * (c.ny - 2) * (c.nz - 2)) : 0.0;
@@ -749,7 +760,7 @@ int one_step(tbl_handle* h, tbl_step_stats* out) {
     for (int q = 0; q < 3; ++q) h->last_counts.push_back(st.gs_sweeps[q]);
     h->last_counts.push_back((int32_t)kits.size());
     for (int q : kits) h->last_counts.push_back(q);
-    if (err != 0) status = err;
+    if (sc.err != 0) status = sc.err;
     else if (!std::isfinite(sc.red[3]) || (fluc && !std::isfinite(sc.red[4]))) status = TBL_ERR_NAN;
     else if (fluc && sc.red[5] > 25.0) status = TBL_ERR_BLOWUP;
     else if (status == TBL_OK && !replay)

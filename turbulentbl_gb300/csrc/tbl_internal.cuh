@@ -83,6 +83,9 @@ struct DevScalars {
                // of an Arnoldi step enqueued ahead of the host's check then return at once
     // GMRES
     double rho, sumnor, sumav;
+    // status of the first bounded device wait that gave up; never cleared.  Between
+    // what the host's solver loops read back, so that each of their copies has it.
+    int err, pad_;
     // reductions (result slots)
     double red[16];
 };
