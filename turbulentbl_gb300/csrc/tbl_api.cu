@@ -83,10 +83,11 @@ int get3(tbl_handle* h, double* dst, const double* src) {
     return TBL_OK;
 }
 
-// FP32 fields travel as doubles and are converted on the device, through a
-// padded FP64 staging field.  Converting on the host took a loop, a zeroed
-// buffer and a pageable copy per field: 25 ms up and 25 ms down for the four
-// fields of 512 x 130 x 128, now 2 ms each way from pinned memory.
+// FP32 fields travel as doubles and are converted on the device, by way of the
+// Poisson right-hand side's field: between steps that holds nothing (every step
+// forms it before reading it, and reads the interior only).  Converting on the host
+// took a loop, a zeroed buffer and a pageable copy per field: 25 ms up and 25 ms
+// down for the four fields of 512 x 130 x 128, now 2 ms each way from pinned memory.
 __global__ void __launch_bounds__(256) k_to_float(long long n4, const double* __restrict__ x, float4* __restrict__ y) {
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
         const double2 a = reinterpret_cast<const double2*>(x)[2 * q], b = reinterpret_cast<const double2*>(x)[2 * q + 1];
@@ -105,18 +106,18 @@ static unsigned cvt_blocks(const tbl_handle* h) {
     return (unsigned)(want < wave ? want : wave);
 }
 static int put3f(tbl_handle* h, float* dst, const double* src) {
-    const int s = put3(h, h->stage, src);
+    const int s = put3(h, h->Q8, src);
     if (s != TBL_OK) return s;
-    k_to_float<<<cvt_blocks(h), 256, 0, h->stream>>>(h->g.vol / 4, h->stage, (float4*)dst);
+    k_to_float<<<cvt_blocks(h), 256, 0, h->stream>>>(h->g.vol / 4, h->Q8, (float4*)dst);
     TBL_CUDA_TRY(cudaGetLastError());
     h->launches++;
     return TBL_OK;
 }
 static int get3f(tbl_handle* h, double* dst, const float* src) {
-    k_to_double<<<cvt_blocks(h), 256, 0, h->stream>>>(h->g.vol / 4, (const float4*)src, h->stage);
+    k_to_double<<<cvt_blocks(h), 256, 0, h->stream>>>(h->g.vol / 4, (const float4*)src, h->Q8);
     TBL_CUDA_TRY(cudaGetLastError());
     h->launches++;
-    return get3(h, dst, h->stage);
+    return get3(h, dst, h->Q8);
 }
 
 template <typename T>
@@ -134,7 +135,7 @@ static int dalloc(T** p, size_t n) {
 
 static void free_all(tbl_handle* h) {
     void* mptrs[] = {h->Uf[0], h->Uf[1], h->Uf[2], h->Pf, h->Qf[0], h->Qf[1], h->Qf[2], h->Df[0], h->Df[1],
-                     h->Df[2], h->Vf, h->RHf, h->R64, h->PREf, h->PRE, h->lsg_partial, h->lsg_L, h->stage};
+                     h->Df[2], h->Vf, h->RHf, h->R64, h->PREf, h->PRE, h->lsg_partial, h->lsg_L};
     for (void* p : mptrs)
         if (p) cudaFree(p);
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
@@ -220,7 +221,6 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
         }
         TRY(dalloc(&h->Pf, vol));
         TRY(dalloc(&h->RHf, vol));
-        TRY(dalloc(&h->stage, vol));
         TRY(dalloc(&h->PREf, 3 * vol));
         // the basis v_0 .. v_kmax, then the Arnoldi vector w before its normalisation
         TRY(dalloc(&h->Vf, vol * (size_t)(cfg->mixed_kmax + 2)));
@@ -258,7 +258,6 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
     h->red.max_blocks = 2048;
     TRY(dalloc(&h->red.partial, (size_t)16 * h->red.max_blocks));
     TRY(dalloc(&h->red.count, (size_t)24));
-    TRY(dalloc(&h->halo, (size_t)2 * 3 * 2 * h->P * g.ps));
     h->err = &h->sc->err;
     // mesh and per-k coefficients (:487-536); An* == Av*
     std::vector<double> x3(mesh->x3, mesh->x3 + nz), jinv(nz), j2(mesh->jac2, mesh->jac2 + nz);
@@ -315,6 +314,8 @@ static int create_impl(const tbl_config* cfg, const tbl_mesh* mesh, tbl_handle* 
     TRY(build_sweep_ctas(h));
     TRY(check_cooperative(h));
     TRY(line_create(h));
+    if (h->line[0].S == 0 && !(cfg->flags & TBL_FLAG_RB_ORDER))  // the wavefront's Gauss-Seidel
+        TRY(dalloc(&h->halo, (size_t)2 * 3 * 2 * h->P * g.ps));
     {   // the matvec's scale in front of the SSOR sweeps: the line-scan sweeps leave the backward sweep's
         // constant factor w (2-w)/w to it (the sweeps are linear)
         const double w = cfg->omega;

@@ -107,12 +107,14 @@ constexpr int sweep_chunk(size_t value_bytes) { return value_bytes == 4 ? 8 : 4;
 // not take it and the wavefront sweeps run.
 struct LineCta {
     int bn, K, blk, kg;  // the slab's first plane and planes, span block, plane group
+    int xp;              // plane of the exchange buffer that its top plane goes to; the one before is the plane below
 };
 struct LineShape {
     int S = 0, E = 0;           // warps per line (0: not taken), points per lane
     int KP = 0, NC = 0;         // planes per CTA, courier warps
     int nblk = 0, rows = 0;     // span blocks per slab, rows per block
     int ncta = 0;               // CTAs of a launch (one component)
+    int nxp = 0;                // planes handed from CTA to CTA (one component)
     size_t smem = 0;
     LineCta* ctas = nullptr;    // [ncta]
 };
@@ -150,7 +152,6 @@ struct tbl_handle {
                         // constant w (2-w)/w where the line-scan sweeps run
     tbl::LineShape line[3];  // line-scan sweeps per mode (GS, forward, backward)
     void* line_xch;          // their exchange between the CTAs of a column
-    size_t line_xdump;       // a row of it that nobody reads
     unsigned* line_ticket;   // their tickets [taken, finished]
     double* V;       // kmax+1 Krylov vectors, vol each
     double* uold1;   // U1 at i=1 before the inflow update, (ny, nz)
@@ -162,7 +163,6 @@ struct tbl_handle {
     float* Vf;       // inner Krylov vectors
     float* RHf;      // inner SSOR work
     double* R64;     // FP64 outer residual
-    double* stage;   // FP64 copy of a field on its way to or from the host
     double* lsg_partial;        // low-synch Gram-Schmidt: per-block partials [2*8*groups][max_blocks]
     double* lsg_L;   // (K1 x K1) strictly lower triangle of the basis' products
     // per-k coefficient arrays and mesh (nz)

@@ -85,7 +85,8 @@ struct LineArgs {
     V* out[3];         // GS: fields; SSOR: out[0]
     const V* in[3];    // GS: precomputed old-value terms; SSOR: in[0]
     int comp[3];
-    V* xch;            // [set][plane][span row][32 E S], empty words all ones
+    V* xch;            // [set][plane handed over][span row][32 E S], empty words all ones
+    int nxp;           // planes handed over (one component)
 };
 
 template <typename V> struct LineBits;
@@ -265,9 +266,9 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
     __syncthreads();
 
     const size_t xrow = (size_t)32 * E * S;
-    // exchange rows of physical plane kk, this lane's values of segment 0
-    auto xch_plane = [&](int kk) {
-        return a.xch + ((((size_t)set * g.nz + kk) * J + j0) * S * 32 + lane) * E;
+    // exchange rows of a plane handed over, this lane's values of segment 0
+    auto xch_plane = [&](int p) {
+        return a.xch + ((((size_t)set * a.nxp + p) * J + j0) * S * 32 + lane) * E;
     };
     // The row segments of a warp's operands in global memory: chunks [c0, ..) of
     // the line, at chunk c0 - clo of the slot.
@@ -313,8 +314,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
         // this CTA's first plane; its words are emptied for the next launch.
         const int sg0 = wid - NW;
         const bool has = cta.kg > 0 && cta.kg * KP < K;
-        const int kb = BWD ? K - cta.kg * KP : cta.kg * KP - 1;
-        V* const src = xch_plane(has ? cta.bn + kb : cta.bn);
+        V* const src = xch_plane(has ? cta.xp - 1 : 0);
         V none[E];
 #pragma unroll
         for (int e = 0; e < E; ++e) none[e] = B::empty();
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
         const bool to_ring = has_up && kp < KP - 1, to_xch = has_up && kp == KP - 1;
         V* const up_ring = ring + (size_t)S * XR * 64 * E + (32 + lane) * E;
         unsigned long long* const up_full = full + S * LINE_BARS;
-        V* xout = to_xch ? xch_plane(k) + (size_t)seg * 32 * E : nullptr;
+        V* xout = to_xch ? xch_plane(cta.xp) + (size_t)seg * 32 * E : nullptr;
 
         const long long rstep = BWD ? -(long long)g.sx : (long long)g.sx;
 
@@ -631,7 +631,11 @@ static bool line_plan(const tbl_handle* h, int rows, int nblk, int E, int kp, Li
     q.KP = std::min(q.KP, (int)(LINE_MAX_SMEM / plane));
     if (q.KP < 1) return false;
     q.smem = q.KP * plane;
-    for (int r = 0; r < h->P; ++r) q.ncta += (h->en[r] - h->bn[r] + 1 + q.KP - 1) / q.KP * nblk;
+    for (int r = 0; r < h->P; ++r) {
+        const int nkg = (h->en[r] - h->bn[r] + 1 + q.KP - 1) / q.KP;
+        q.ncta += nkg * nblk;
+        q.nxp += nkg - 1;
+    }
     return true;
 }
 
@@ -677,10 +681,13 @@ static bool line_plan_gs(const tbl_handle* h, int rows, int E0, LineShape& q) {
 // The CTAs of a launch, the lowest of every column first.
 static int line_table(const tbl_handle* h, LineShape& q) {
     std::vector<LineCta> t;
+    std::vector<int> xp(h->P, 0);  // exchange planes before the column's
+    for (int r = 1; r < h->P; ++r) xp[r] = xp[r - 1] + (h->en[r - 1] - h->bn[r - 1] + 1 + q.KP - 1) / q.KP - 1;
     for (int kg = 0; (int)t.size() < q.ncta; ++kg)
         for (int r = 0; r < h->P; ++r)
             if (kg * q.KP < h->en[r] - h->bn[r] + 1)
-                for (int blk = 0; blk < q.nblk; ++blk) t.push_back({h->bn[r], h->en[r] - h->bn[r] + 1, blk, kg});
+                for (int blk = 0; blk < q.nblk; ++blk)
+                    t.push_back({h->bn[r], h->en[r] - h->bn[r] + 1, blk, kg, xp[r] + kg});
     TBL_CUDA_TRY(cudaMalloc(&q.ctas, t.size() * sizeof(LineCta)));
     TBL_CUDA_TRY(cudaMemcpy(q.ctas, t.data(), t.size() * sizeof(LineCta), cudaMemcpyHostToDevice));
     return TBL_OK;
@@ -712,22 +719,32 @@ static int line_init(tbl_handle* h) {
         kp = 2;
     }
     LineShape q[3];
-    const bool ssor = line_plan<V>(h, brows, nblk, E, kp, q[1]) && line_plan<V>(h, brows, nblk, E, kp, q[2]) &&
-                      line_ready<1, V>(q[1]) && line_ready<2, V>(q[2]);
-    const bool gs = line_plan_gs<V>(h, J, sizeof(V) == 4 && nx > 385 ? 8 : E, q[0]) && line_ready<0, V>(q[0]);
-    size_t words = 0;
+    const bool ssor = !(h->cfg.flags & TBL_FLAG_RB_PRECOND) && line_plan<V>(h, brows, nblk, E, kp, q[1]) &&
+                      line_plan<V>(h, brows, nblk, E, kp, q[2]) && line_ready<1, V>(q[1]) && line_ready<2, V>(q[2]);
+    const bool gs = !(h->cfg.flags & TBL_FLAG_RB_ORDER) &&
+                    line_plan_gs<V>(h, J, sizeof(V) == 4 && nx > 385 ? 8 : E, q[0]) && line_ready<0, V>(q[0]);
+    if (!gs && !ssor) return TBL_OK;
+    size_t words = 32 * 8;  // the self-test's at least
+    for (int m = 0; m < 3; ++m)
+        if (m == 0 ? gs : ssor)
+            words = std::max(words, (size_t)(m == 0 ? 3 : 1) * q[m].nxp * J * 32 * q[m].E * q[m].S);
+    // Up to a few percent of the handle's memory: where only that is missing the
+    // wavefront sweeps do with less.
+    const cudaError_t e = cudaMalloc(&h->line_xch, words * sizeof(V));
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        h->line_xch = nullptr;
+        return TBL_OK;
+    }
+    TBL_CUDA_TRY(e);
+    TBL_CUDA_TRY(cudaMemset(h->line_xch, 0xff, words * sizeof(V)));
+    TBL_CUDA_TRY(cudaMalloc(&h->line_ticket, 2 * sizeof(unsigned)));
+    TBL_CUDA_TRY(cudaMemset(h->line_ticket, 0, 2 * sizeof(unsigned)));
     for (int m = 0; m < 3; ++m) {
         if (m == 0 ? !gs : !ssor) continue;
         h->line[m] = q[m];
         const int st = line_table(h, h->line[m]);
         if (st != TBL_OK) return st;
-        words = std::max(words, (size_t)(m == 0 ? 3 : 1) * h->g.nz * J * 32 * q[m].E * q[m].S);
-    }
-    if (words > 0) {
-        TBL_CUDA_TRY(cudaMalloc(&h->line_xch, words * sizeof(V)));
-        TBL_CUDA_TRY(cudaMemset(h->line_xch, 0xff, words * sizeof(V)));
-        TBL_CUDA_TRY(cudaMalloc(&h->line_ticket, 2 * sizeof(unsigned)));
-        TBL_CUDA_TRY(cudaMemset(h->line_ticket, 0, 2 * sizeof(unsigned)));
     }
     return TBL_OK;
 }
@@ -749,6 +766,7 @@ static LineArgs<V> line_args(tbl_handle* h, const LineShape& q) {
     a.as = 1.0 / (h->cfg.dy * h->cfg.dy);
     a.omega = h->cfg.omega;
     a.xch = (V*)h->line_xch;
+    a.nxp = q.nxp;
     return a;
 }
 
