@@ -205,14 +205,12 @@ __device__ __forceinline__ bool line_arrived(const V (&w)[E]) {
 }
 // A courier's wait for one segment of a row of the plane below.
 template <typename V, int E>
-__device__ __forceinline__ bool xch_wait(V (&w)[E], const V* p) {
-    bool good = true;
+__device__ __forceinline__ void xch_wait(V (&w)[E], const V* p, bool& good) {
     for (long long spins = 0; good;) {
         xch_ld(w, p);
         if (__all_sync(0xffffffffu, line_arrived(w))) break;
         good = ++spins < SPIN_LIMIT / 16;
     }
-    return good;
 }
 // A warp's wait for the carry into its segment.
 template <typename V>
@@ -332,7 +330,7 @@ __global__ void __launch_bounds__(32 * (line_max_warps(E) + LINE_MAX_COURIERS + 
                 if ((r & (H - 1)) == 0 && r >= XR)
                     good = __all_sync(ALL, mbar_wait(&fb[(r & (XR - 1)) / H], (unsigned)(r / XR - 1) & 1u));
                 V w[E];
-                if (good) good = xch_wait<V, E>(w, src + r * xrow + (size_t)sg0 * 32 * E);
+                xch_wait<V, E>(w, src + r * xrow + (size_t)sg0 * 32 * E, good);
                 if (good) hand(r, sg0, w);
             }
         } else if (has) {
@@ -592,7 +590,8 @@ __global__ void __launch_bounds__(32) k_line_wait(int which, V* word, int* err) 
         got = mbar_wait(&s_bar, 0);
     } else if (which == 1) {
         V w[E];
-        got = xch_wait<V, E>(w, word + threadIdx.x * E);
+        got = true;
+        xch_wait<V, E>(w, word + threadIdx.x * E, got);
     } else {
         V c;
         got = carry_wait(c, &s_mail);
