@@ -135,7 +135,7 @@ static int dalloc(T** p, size_t n) {
 
 static void free_all(tbl_handle* h) {
     void* mptrs[] = {h->Uf[0], h->Uf[1], h->Uf[2], h->Pf, h->Qf[0], h->Qf[1], h->Qf[2], h->Df[0], h->Df[1],
-                     h->Df[2], h->Vf, h->RHf, h->R64, h->PREf, h->PRE, h->lsg_partial, h->lsg_L};
+                     h->Df[2], h->Vf, h->RHf, h->PREf, h->PRE, h->lsg_partial, h->lsg_L};
     for (void* p : mptrs)
         if (p) cudaFree(p);
     void* ptrs[] = {h->U[0], h->U[1], h->U[2], h->Pr, h->PC, h->Q[0], h->Q[1], h->Q[2], h->Q8, h->RH, h->V,
@@ -516,8 +516,7 @@ static int gmres_mixed(tbl_handle* h, std::vector<int32_t>& kits, tbl_step_stats
         // inner tolerance relative to the cycle's start (sumav <= thr)
         const double thr = std::fmax(target, inner_tol * rho_m / sumnor);
         // w_k is formed in the slot after the basis; step k+1's matvec divides
-        // it by H(k+1,k) as it reads it and writes v_k into the basis (the
-        // separate scaling pass folded into the TMA matvec, same values)
+        // it by H(k+1,k) as it reads it and writes v_k into the basis
         float* W = h->Vf + (size_t)K1 * vol;
         auto arnoldi_step = [&](int k, const int* skip) -> int {
             {

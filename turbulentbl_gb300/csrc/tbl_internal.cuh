@@ -119,15 +119,6 @@ struct LineShape {
     LineCta* ctas = nullptr;    // [ncta]
 };
 
-template <typename T>
-struct Fields {
-    T* U[3];
-    T* P;
-    T* PC;
-    T* Q[3];
-    T* Q8;
-};
-
 }  // namespace tbl
 
 struct tbl_handle {
@@ -162,7 +153,6 @@ struct tbl_handle {
     float* Df[3];    // GS increments (delta form)
     float* Vf;       // inner Krylov vectors
     float* RHf;      // inner SSOR work
-    double* R64;     // FP64 outer residual
     double* lsg_partial;        // low-synch Gram-Schmidt: per-block partials [2*8*groups][max_blocks]
     double* lsg_L;   // (K1 x K1) strictly lower triangle of the basis' products
     // per-k coefficient arrays and mesh (nz)

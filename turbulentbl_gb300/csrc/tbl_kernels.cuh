@@ -20,13 +20,12 @@ int launch_gs_delta_init(tbl_handle* h, int comp);
 int launch_gs_delta_apply(tbl_handle* h, int comp);
 int launch_gs_delta_restart(tbl_handle* h, int comp);
 
-// tbl_sweep.cu
-int build_sweep_ctas(tbl_handle* h);
-int check_cooperative(tbl_handle* h);
 // tbl_gs.cu
 int launch_gs_parts(tbl_handle* h, const int* comps, int ncomp, bool pre, bool resid);
 
 // tbl_sweep.cu
+int build_sweep_ctas(tbl_handle* h);
+int check_cooperative(tbl_handle* h);
 int launch_gs_sweep(tbl_handle* h, const int* comps, int ncomp, int parity, bool have_pre);
 int launch_gs_coef(tbl_handle* h);
 int launch_halo_init(tbl_handle* h, int parity);

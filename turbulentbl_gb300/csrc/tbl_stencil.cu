@@ -823,8 +823,6 @@ int launch_conv_q(tbl_handle* h) {
     return TBL_OK;
 }
 
-// GS residual of the listed components.  In mixed precision the iteration is
-// on the increment D (delta form) with right-hand side r0 stored in Qf.
 // Mixed precision, delta form of the Gauss-Seidel solve of (I + t L7) U = Q:
 // the FP32 sweeps iterate on an increment D with right-hand side r = Q - A U.
 // In exact arithmetic U + D are the reference's iterates (a sweep is affine),
