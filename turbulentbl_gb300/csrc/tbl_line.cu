@@ -44,8 +44,8 @@
 // cycles each to issue; a feeder warp does it), selects and tests at its ends.
 // SSOR sweep, wavefront -> line scan: 130 -> 53 us (128 x 66 x 64, FP64, 8
 // slabs), 389 -> 176 us (512 x 130 x 128, FP64), 95 -> 34 us and 251 -> 74 us
-// (FP32); GS sweep of three components with its precomputed terms 280 -> 64 us
-// at 128, 620 -> 489 us at 512 (FP64).
+// (FP32); GS sweep of three components 54 us at 128 and 305 at 512 (FP64), with its
+// precomputed terms 280 -> 64 and 620 -> 493 us.
 // A first form with thread-block clusters (st.async into the next CTA's ring)
 // was slower at 512 (243 us): clusters of 15 CTAs doubled up on SMs.  Register
 // prefetch of the operands was slower too (their loads share scoreboards with
@@ -655,7 +655,9 @@ static bool line_ready(const LineShape& q) {
 // fewest waves, and of those the fewest points per lane and then planes per
 // CTA.  FP64, E, KP = 2, 2 / 2, 3 / 4, 2 / 4, 3, us: 124 / 118 / 139 / 135 at
 // 256 x 98 x 96 (one wave each); 194 / 157 / 203 / 182 at 256 x 130 x 128 and
-// 341 / - / 343 / 300 at 512 x 130 x 128 (two, one, two, one).  FP32, 4, 2 /
+// 341 / - / 343 / 300 at 512 x 130 x 128 (two, one, two, one; the last took 284
+// before the couriers kept a look at each segment in flight, 5% that the SSOR
+// sweeps gain: 180 -> 174, twice per Arnoldi step).  FP32, 4, 2 /
 // 4, 3 / 8, 4: 111 / 98 / 103 at 512 x 130 x 128 (two, one, one), 119 / 131 /
 // 99 at 512 x 102 x 190 (two, two, one); from two planes to three or four the
 // hand-overs saved weigh as much.  FP32 lines of four warps or more take 8
@@ -701,8 +703,8 @@ static int line_init(tbl_handle* h) {
     // cycles per FMA that a warp issues, so few points per lane spread a line
     // over more of the SM's four FP64 pipes, but every warp pays for the scan.
     // Forward and backward sweep, E = 1 / 2: 100 / 117 us at 128 x 66 x 64,
-    // 116 / 118 at 160 x 66 x 81, 138 / 140 at 201 x 77 x 59, 188 / 173 at
-    // 256 x 98 x 96; E = 2 / 4: 317 / 356 at 512 x 130 x 128, 341 / 356 at
+    // 116 / 118 at 160 x 66 x 81, 138 / 140 at 201 x 77 x 59, level but for
+    // seven warps a line instead of four, 188 / 173 at 256 x 98 x 96; E = 2 / 4: 317 / 356 at 512 x 130 x 128, 341 / 356 at
     // 700 x 130 x 100, 304 / 276 at 850 x 92 x 90.  FP32 rows are bound by
     // latency: 4 points, and two planes per CTA save a hand-over (152 / 147 /
     // 178 with 1 / 2 / 3 at 512 x 130 x 128); from five warps a line on, the
