@@ -39,9 +39,12 @@ def test_a_box_that_leaves_no_room_for_the_exchange_still_runs():
     """256 x 98 x 97 in one slab, 3 vectors: the line-scan sweeps' exchange is 31 MB
     there.  With half of that left they are not taken, the handle is created all
     the same, and the step is the other sweeps' (1e-12, as in the parity tests)."""
+    import gc
+
     import numpy as np
     import torch
     from turbulentbl_gb300.lib import TblGpu
+    gc.collect()  # no handle of another test is to be freed meanwhile
     wl = small_workload(nx=256, nz_span=96, ny_wall=96, kmax=3)
     mesh, rp, st = make_state(wl, nproc=1)
     rp.flags, counts = abi.TBL_FLAG_REPLAY, [4, 4, 4, 2, 3, 3]
